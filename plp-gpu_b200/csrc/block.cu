@@ -48,6 +48,7 @@ struct BlockArgs {
     SlotHead* heads;
     unsigned long long* places;
     unsigned long long* scratch;
+    int scratch_stride;            // words per decoder's row of scratch
     const uint32_t* __restrict__ mt_init;
     int P, C, N, T, Hz;   // blocks, live points, items, types (tile), top-z index
 };
@@ -368,7 +369,7 @@ __device__ __forceinline__ void block_body(const BlockArgs& a, unsigned char* ba
         const TypeOrs* tors = a.types + I.type_off;
         unsigned long long* best_out = a.places + I.place_off + (long long)restart * I.place_stride;
         unsigned long long* pass_out =
-            I.passes > 1 ? a.scratch + (long long)gdec * I.place_stride : best_out;
+            I.passes > 1 ? a.scratch + (long long)gdec * a.scratch_stride : best_out;
         int mpos = 624;
         {
             const long long sd = I.seed + restart;
@@ -671,6 +672,7 @@ cudaError_t enqueue_block(const DecodeLaunch& L, cudaStream_t st) {
     a.heads = L.heads;
     a.places = L.places;
     a.scratch = L.scratch;
+    a.scratch_stride = L.scratch_stride;
     a.mt_init = L.mt_init;
     a.P = L.P;
     a.C = L.C;

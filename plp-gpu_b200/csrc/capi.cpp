@@ -836,6 +836,7 @@ static DecodeLaunch make_launch(const Batch& b, const TileConfig& t, const int2*
     L.heads = reinterpret_cast<SlotHead*>(b.d_mem + b.o_heads);
     L.places = reinterpret_cast<unsigned long long*>(b.d_mem + b.o_places);
     L.scratch = reinterpret_cast<unsigned long long*>(b.d_mem + b.o_scratch);
+    L.scratch_stride = b.max_stride;
     L.mt_init = b.mt_init;
     L.seed_tab = b.seed_n ? reinterpret_cast<const uint32_t*>(b.d_mem + b.o_seedtab) : nullptr;
     L.seed_lo = b.seed_lo;
@@ -3128,6 +3129,7 @@ int plp_decode_noalloc(const plp_instance* inst, const plp_run_opts* opts, void*
     L.heads = static_cast<SlotHead*>(d_heads);
     L.places = static_cast<unsigned long long*>(d_places);
     L.scratch = reinterpret_cast<unsigned long long*>(d + o_rows);
+    L.scratch_stride = b.max_stride;
     L.mt_init = reinterpret_cast<const uint32_t*>(d + o_mt);
     L.P = t.P;
     L.C = t.C;

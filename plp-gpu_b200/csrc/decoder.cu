@@ -166,6 +166,7 @@ struct DecoderArgs {
     SlotHead* heads;
     unsigned long long* places;
     unsigned long long* scratch;   // per resident warp: passes > 1
+    int scratch_stride;            // words per row of it: at least every instance's place_stride
     const uint32_t* __restrict__ mt_init;
     int P, C, Hz;
     int sync_limit;                // tries per barrier wait (0 = SYNC_WAIT_LIMIT)
@@ -584,7 +585,7 @@ __device__ __forceinline__ void decoder_body(const DecoderArgs& a, unsigned char
         const bool randomized = !(I.first_fit || I.eps == 0.0);
         unsigned long long* best_out = a.places + I.place_off + (long long)restart * I.place_stride;
         unsigned long long* pass_out =
-            I.passes > 1 ? a.scratch + (long long)gdec * I.place_stride : best_out;
+            I.passes > 1 ? a.scratch + (long long)gdec * a.scratch_stride : best_out;
         int mpos = 624;   // RNG position (warp 0)
         if (g == 0) {
             const long long sd = I.seed + restart;
@@ -1426,7 +1427,7 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
         const bool randomized = !(I.first_fit || I.eps == 0.0);
         unsigned long long* best_out = a.places + I.place_off + (long long)restart * I.place_stride;
         unsigned long long* pass_out =
-            I.passes > 1 ? a.scratch + (long long)gdec * I.place_stride : best_out;
+            I.passes > 1 ? a.scratch + (long long)gdec * a.scratch_stride : best_out;
         int mpos = 624;
         {
             const long long sd = I.seed + restart;
@@ -1634,6 +1635,7 @@ static DecoderArgs decoder_args(const DecodeLaunch& L) {
     a.heads = L.heads;
     a.places = L.places;
     a.scratch = L.scratch;
+    a.scratch_stride = L.scratch_stride;
     a.mt_init = L.mt_init;
     a.P = L.P;
     a.C = L.C;

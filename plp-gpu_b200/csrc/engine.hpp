@@ -20,6 +20,7 @@ struct DecodeLaunch {
     SlotHead* heads;
     unsigned long long* places;
     unsigned long long* scratch;
+    int scratch_stride;       // words per resident decoder's row of scratch (the largest place_stride)
     const uint32_t* mt_init;
     int P, C;                 // shared-memory tile: boxes and live points per decoder
     int Hz;                   // entries of the top-z index (max height + 2), 0 = none
