@@ -337,6 +337,20 @@ std::vector<TypeOrs> type_orientations(const Instance& I, int* small) {
     return ot;
 }
 
+// Smallest edge per axis over the types' orientations (1 where there is none).
+void min_edges(const std::vector<TypeOrs>& ors, InstDesc& d) {
+    int m[3] = {INT_MAX, INT_MAX, INT_MAX};
+    for (const TypeOrs& t : ors)
+        for (int k = 0; k < t.n; k++) {
+            m[0] = std::min(m[0], t.w[k]);
+            m[1] = std::min(m[1], t.d[k]);
+            m[2] = std::min(m[2], t.h[k]);
+        }
+    d.mw = m[0] == INT_MAX ? 1 : m[0];
+    d.md = m[1] == INT_MAX ? 1 : m[1];
+    d.mh = m[2] == INT_MAX ? 1 : m[2];
+}
+
 struct Batch {
     std::vector<const Instance*> insts;
     std::vector<plp_run_opts> opts;
@@ -498,6 +512,7 @@ struct Batch {
             }
             if (!small) sup16_ok = 0;
             types.insert(types.end(), ot.begin(), ot.end());
+            min_edges(ot, desc.back());
             desc.back().engine = o.engine;
             desc.back().n_types = (int)I.types.size();
             max_types = std::max(max_types, (int)I.types.size());

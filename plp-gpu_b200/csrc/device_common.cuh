@@ -44,6 +44,10 @@ struct InstDesc {
     int bo_start_off;    // n_types + 1 offsets into that table
     int bo_shape_of_rank;
     int cat_off, n_cat;
+    // smallest edge along x, y, z over every orientation of the instance's
+    // types: a point whose mw x md x mh cuboid leaves the container or meets
+    // a placed box cannot hold any item (the decoders drop it)
+    int mw, md, mh, pad;
 };
 
 // Block shape of the block-building engine (blockproof/plp_block.cpp:29-37):
