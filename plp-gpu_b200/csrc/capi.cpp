@@ -322,7 +322,7 @@ int build_block_tables(const Instance& I, const std::vector<TypeOrs>& ors, const
 
 // Orientation table of every box type of an instance; clears *small when an
 // orientation's footprint area reaches 65536 (its contact areas need 32 bits).
-std::vector<TypeOrs> type_orientations(const Instance& I, int* small) {
+std::vector<TypeOrs> type_orientations(const Instance& I) {
     std::vector<TypeOrs> ot;
     ot.reserve(I.types.size());
     for (const auto& t : I.types) {
@@ -330,8 +330,21 @@ std::vector<TypeOrs> type_orientations(const Instance& I, int* small) {
         const auto v = orientations(t);
         to.n = (int)v.size();
         for (int k = 0; k < to.n; k++) { to.w[k] = v[k][0]; to.d[k] = v[k][1]; to.h[k] = v[k][2]; }
-        for (int k = 0; k < to.n; k++)
-            if (1LL * to.w[k] * to.d[k] >= 65536) *small = 0;
+        // the list is the six slots in order, less those a flag rules out or
+        // an earlier slot equals
+        const int e[3] = {t.l, t.w, t.h};
+        static const int slot[6][3] = {{1, 2, 0}, {2, 1, 0}, {0, 2, 1}, {2, 0, 1}, {0, 1, 2}, {1, 0, 2}};
+        const int flag[3] = {t.lf, t.wf, t.hf};
+        int mask = 0, k = 0;
+        for (int s = 0; s < 6 && k < to.n; s++) {
+            if (!flag[slot[s][2]]) continue;
+            if (e[slot[s][0]] != to.w[k] || e[slot[s][1]] != to.d[k] || e[slot[s][2]] != to.h[k]) continue;
+            mask |= 1 << s;
+            k++;
+        }
+        to.el = std::min(t.l, 0x1ffff) | mask << 20;
+        to.ew = std::min(t.w, 0x1ffff);
+        to.eh = std::min(t.h, 0x1ffff);
         ot.push_back(to);
     }
     return ot;
@@ -365,10 +378,6 @@ struct Batch {
     bool multi_pass = false;
     // block-building engine: shape catalogue and per-instance orderings
     int engine = 0, max_types = 0;
-    // contact areas of the decoder in 16 bits: allowed when every
-    // orientation's footprint area is below 65536, chosen (plan) when the
-    // batch's restarts exceed one wave at 32-bit residency
-    int sup16_ok = 1, sup16 = 0;
     // seeded MT states computed once per distinct restart seed when the
     // batch's restarts share seeds (every instance seeding 0 .. R - 1, say):
     // seeds seed_lo .. seed_lo + seed_n - 1, or seed_n = 0 to seed in place
@@ -417,8 +426,6 @@ struct Batch {
         bcat.clear(); btab.clear();
         engine = op.empty() ? 0 : op[0].engine;
         max_types = 0;
-        sup16_ok = 1;
-        sup16 = 0;
         n_slots = 0; n_places = 0; max_stride = 1; max_steps = 0; multi_pass = false;
         int maxH = 0;
         best_only = true;
@@ -426,11 +433,9 @@ struct Batch {
         // several threads; the rest of the build is appends in instance order
         std::vector<std::vector<int>> seqs;
         std::vector<std::vector<TypeOrs>> ors;
-        std::vector<int> ors_small;
         if (in.size() >= 256) {
             seqs.resize(in.size());
             ors.resize(in.size());
-            ors_small.assign(in.size(), 1);
             const unsigned hw = std::thread::hardware_concurrency();
             const int nt = (int)std::max(1u, std::min(16u, hw ? hw : 1u));
             std::atomic<size_t> next{0};
@@ -438,7 +443,7 @@ struct Batch {
                 for (size_t i0; (i0 = next.fetch_add(64)) < in.size();)
                     for (size_t k = i0; k < std::min(in.size(), i0 + 64); k++) {
                         if (op[k].order == 0 || op[k].order == 1) seqs[k] = item_sequence(*in[k], op[k].order);
-                        ors[k] = type_orientations(*in[k], &ors_small[k]);
+                        ors[k] = type_orientations(*in[k]);
                     }
             };
             std::vector<std::thread> pool;
@@ -502,15 +507,7 @@ struct Batch {
             d.first_fit = o.first_fit ? 1 : 0;
             desc.push_back(d);
             steps.insert(steps.end(), seq.begin(), seq.end());
-            int small = 1;
-            std::vector<TypeOrs> ot;
-            if (ors.empty()) {
-                ot = type_orientations(I, &small);
-            } else {
-                ot = std::move(ors[i]);
-                small = ors_small[i];
-            }
-            if (!small) sup16_ok = 0;
+            std::vector<TypeOrs> ot = ors.empty() ? type_orientations(I) : std::move(ors[i]);
             types.insert(types.end(), ot.begin(), ot.end());
             min_edges(ot, desc.back());
             desc.back().engine = o.engine;
@@ -564,14 +561,6 @@ struct Batch {
 
     void plan(int sms, const TileConfig& t) {
         tile = t;
-        // a latency-bound launch (one wave) gains nothing from the smaller
-        // footprint and the 32-bit areas are a little faster to update
-        sup16 = 0;
-        if (engine == 0 && sup16_ok && t.G == 1) {
-            int occ32 = 1;
-            if (tile_occupancy(*this, t, &occ32) != cudaSuccess || occ32 < 1) occ32 = 1;
-            sup16 = n_slots > (long long)sms * occ32 * t.D ? 1 : 0;
-        }
         int occ = 1;
         if (tile_occupancy(*this, t, &occ) != cudaSuccess || occ < 1) occ = 1;
         const long long need = (n_slots + t.D - 1) / t.D;
@@ -602,7 +591,7 @@ struct Batch {
 
 int tile_smem(const Batch& b, const TileConfig& t) {
     return b.engine == 1 ? block_smem_bytes(t.P, t.C, std::max(1, b.max_steps), std::max(1, b.max_types), b.Hz)
-                         : decoder_smem_bytes(t.P, t.C, b.Hz, t.G, b.sup16);
+                         : decoder_smem_bytes(t.P, t.C, b.Hz, t.G);
 }
 
 bool tile_supported(const Batch& b, const TileConfig& t) {
@@ -612,7 +601,7 @@ bool tile_supported(const Batch& b, const TileConfig& t) {
 cudaError_t tile_occupancy(const Batch& b, const TileConfig& t, int* occ) {
     if (b.engine == 1)
         return block_occupancy(t.P, t.C, std::max(1, b.max_steps), std::max(1, b.max_types), b.Hz, t.D, t.M, occ);
-    return decoder_occupancy(t.P, t.C, b.Hz, t.G, t.D, t.M, occ, b.sup16);
+    return decoder_occupancy(t.P, t.C, b.Hz, t.G, t.D, t.M, occ);
 }
 
 // Fewer decoders per CTA when the tile plus this batch's top-z index (and,
@@ -860,7 +849,6 @@ static DecodeLaunch make_launch(const Batch& b, const TileConfig& t, const int2*
     L.C = t.C;
     L.Hz = b.Hz;
     L.engine = b.engine;
-    L.sup16 = b.sup16;
     L.bcat = reinterpret_cast<const BlkShape*>(b.d_mem + b.o_bcat);
     L.btab = reinterpret_cast<const int*>(b.d_mem + b.o_btab);
     L.N = std::max(1, b.max_steps);
@@ -1607,7 +1595,7 @@ size_t serve_align(size_t x, size_t unit) {    // a multiple of unit and of 128 
 }
 
 struct ServeConfig {
-    int P = 256, C = 512, D = 1, M = 12, Hz = 0, sup16 = 0;
+    int P = 256, C = 512, D = 1, M = 12, Hz = 0;
     int deep_P = 512, deep_C = 2048;   // the overflow decoders' tile (global memory)
     bool valid = false;
 };
@@ -1695,7 +1683,7 @@ struct ServeEngine {
         return o.engine == 0 && o.passes == 1 && o.time_limit_s < 0 && !o.best_only;
     }
 
-    int deep_bytes() const { return decoder_smem_bytes(cfg.deep_P, cfg.deep_C, 4096, 1, 0); }
+    int deep_bytes() const { return decoder_smem_bytes(cfg.deep_P, cfg.deep_C, 4096, 1); }
 
     int init(size_t arena_bytes) {
         device = h->device;
@@ -1719,7 +1707,7 @@ struct ServeEngine {
         if (const char* v = std::getenv("PLP_SERVE_TILE")) {
             int p = 0, c = 0, m = 0;
             if (std::sscanf(v, "%d,%d,%d", &p, &c, &m) == 3 && p >= 16 && p <= P_MAX && c >= 32 && c <= C_MAX &&
-                c % 32 == 0 && serve_config_supported(1, m) && decoder_smem_bytes(p, c, 4096, 1, 0) <= 227 * 1024) {
+                c % 32 == 0 && serve_config_supported(1, m) && decoder_smem_bytes(p, c, 4096, 1) <= 227 * 1024) {
                 cfg.P = p;
                 cfg.C = c;
                 cfg.M = m;
@@ -1839,7 +1827,6 @@ struct ServeEngine {
 
     bool compatible(const Batch& b) const {
         if (!cfg.valid) return true;
-        if (cfg.sup16 && !b.sup16_ok) return false;
         if (cfg.Hz == 0) return true;
         return b.Hz != 0 && b.Hz <= cfg.Hz;
     }
@@ -1847,12 +1834,10 @@ struct ServeEngine {
     void merge_config(const Batch& b) {
         if (!cfg.valid) {
             cfg.Hz = b.Hz;
-            cfg.sup16 = b.sup16_ok;
             cfg.valid = true;
             return;
         }
         cfg.Hz = (cfg.Hz == 0 || b.Hz == 0) ? 0 : std::max(cfg.Hz, b.Hz);
-        cfg.sup16 = cfg.sup16 && b.sup16_ok;
     }
 
     void complete(ServeJob& j, int status, plp_result* res, const std::string& err) {
@@ -1886,18 +1871,17 @@ struct ServeEngine {
         L.P = cfg.P;
         L.C = cfg.C;
         L.Hz = cfg.Hz;
-        L.sup16 = cfg.sup16;
         L.engine = 0;
         L.warps_per_decoder = 1;
         L.decoders_per_cta = cfg.D;
         L.min_blocks = cfg.M;
         int occ = 0;
-        cudaError_t e = serve_occupancy(cfg.P, cfg.C, cfg.Hz, cfg.D, cfg.M, cfg.sup16, &occ);
+        cudaError_t e = serve_occupancy(cfg.P, cfg.C, cfg.Hz, cfg.D, cfg.M, &occ);
         if (e != cudaSuccess) return e;
         if (occ < 1) return cudaErrorInvalidConfiguration;
         L.ctas = std::max(sms * occ, n_deep / cfg.D + 1);
         // the overflow decoders' tile must hold this launch's top-z index
-        args.deep_bytes = decoder_smem_bytes(cfg.deep_P, cfg.deep_C, cfg.Hz, 1, cfg.sup16);
+        args.deep_bytes = decoder_smem_bytes(cfg.deep_P, cfg.deep_C, cfg.Hz, 1);
         if (args.deep_bytes > deep_bytes()) return cudaErrorInvalidConfiguration;
         h_word[2] = L.ctas * cfg.D - n_deep;                      // main decoders
         send_stop(0);
@@ -1913,8 +1897,8 @@ struct ServeEngine {
             n_launches++;
         }
         if (serve_trace())
-            std::fprintf(stderr, "[serve %.6f] launch ctas=%d P=%d C=%d Hz=%d sup16=%d deep=%d tail=%d (%s)\n",
-                         now_seconds(), L.ctas, cfg.P, cfg.C, cfg.Hz, cfg.sup16, n_deep, tail, cudaGetErrorString(e));
+            std::fprintf(stderr, "[serve %.6f] launch ctas=%d P=%d C=%d Hz=%d deep=%d tail=%d (%s)\n",
+                         now_seconds(), L.ctas, cfg.P, cfg.C, cfg.Hz, n_deep, tail, cudaGetErrorString(e));
         return e;
     }
 

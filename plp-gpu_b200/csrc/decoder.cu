@@ -111,16 +111,17 @@ __host__ __device__ inline DecLayout dec_layout(int P, int C, int Hz) {
     return l;
 }
 
-// Layout of one single-warp (incremental) decoder: as above, but every live
-// point also carries its evaluation state and six contact areas.
+// Layout of one single-warp decoder: MT state, top-sorted boxes, and two
+// point buffers of {key, x extent | y extent << 16, z extent} (SoA). A
+// placement writes the updated points from one buffer to the other; between
+// placements the spare buffer holds the step's item list. Eight entries past
+// C take a placement's corners before the capacity check.
 struct Dec1Layout {
-    int off_bx, off_bz, off_z2, off_bi, off_key, off_st, off_sup, off_w, off_wi, off_zt, off_sh, bytes;
+    int off_bx, off_bz, off_z2, off_bi, off_pts, off_zt, bytes;
+    int cap;   // entries per array of a point buffer
 };
 
-// sb: bytes per stored contact area (4, or 2 when every orientation's
-// footprint area is below 65536; an area never exceeds its footprint, since
-// boxes sharing a top cannot overlap below it)
-__host__ __device__ inline Dec1Layout dec1_layout(int P, int C, int Hz, int sb) {
+__host__ __device__ inline Dec1Layout dec1_layout(int P, int C, int Hz) {
     Dec1Layout l;
     int o = 624 * 4;                       // MT state
     o = (o + 15) & ~15;
@@ -129,27 +130,21 @@ __host__ __device__ inline Dec1Layout dec1_layout(int P, int C, int Hz, int sb) 
     l.off_z2 = o;  o += 4 * P;             // top z
     l.off_bi = o;  o += 2 * P;             // placement index
     o = (o + 15) & ~15;
-    // live points: key, state, 6 contact areas; FSR overlays 18 bytes per box
-    l.off_key = o;
-    l.off_st = o + 4 * C;
-    l.off_sup = o + 8 * C;
-    int region = (8 + 6 * sb) * C;
+    l.cap = C + 8;
+    l.off_pts = o;
+    int region = 24 * l.cap;               // two buffers; FSR overlays 18 bytes per box
     if (region < 18 * P + 32) region = 18 * P + 32;
     o += region;
     o = (o + 15) & ~15;
-    l.off_w = o;   o += 8 * C;             // items to evaluate {key, m2 | jlo << 8 | jsup << 20}
-    l.off_wi = o;  o += 2 * C;             // their point index
-    o = (o + 15) & ~15;
     l.off_zt = o;  o += 2 * Hz;            // u16: boxes with top < z
     o = (o + 15) & ~15;
-    l.off_sh = o;  o += (int)sizeof(DecShared);
     l.bytes = o;
     return l;
 }
 
 #ifndef PLP_SERVE_TU
-int decoder_smem_bytes(int P, int C, int Hz, int G, int sup16) {
-    return G == 1 ? dec1_layout(P, C, Hz, sup16 ? 2 : 4).bytes : dec_layout(P, C, Hz).bytes;
+int decoder_smem_bytes(int P, int C, int Hz, int G) {
+    return G == 1 ? dec1_layout(P, C, Hz).bytes : dec_layout(P, C, Hz).bytes;
 }
 #endif
 
@@ -774,23 +769,34 @@ __global__ void __launch_bounds__(32 * G * D, M) decoder_kernel(DecoderArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// incremental single-warp decoder (G = 1)
+// single-warp decoder (G = 1)
 // ---------------------------------------------------------------------------
-// Every live point carries its evaluation for the current item type:
-//   st bits 0-5   C2 mask m2 (orientation inside the container)
-//   st bits 8-13  C1 blocked orientations (exact for the bits of `known`)
-//   st bits 16-21 C3 support-ok orientations (all six at z = 0)
-//   st bits 24-29 known = m2 & support-ok when C1 was evaluated
-//   st bit  31    valid
-//   sup[o]        integer contact area under orientation o (z > 0)
-// Boxes are only ever added during a pass, so a blocked orientation stays
-// blocked and a contact area only grows: a valid point stays exact if each
-// newly placed box is applied to it once (C1 OR, C3 sum), which the next
-// step's filter pass does. Consecutive items of the same type share the
-// evaluation; a type change invalidates every point. A point is evaluated
-// from scratch (all boxes) only while it is invalid: new corners, points the
-// greedy scan has not reached yet, and points whose support grew onto an
-// orientation whose C1 was never evaluated.
+// A live point carries its free extents: ex is the distance from the point
+// along x to the nearest box that reaches the y and z ranges of the cuboid of
+// the instance's smallest edges (mw x md x mh, InstDesc) at the point, or to
+// the container wall; ey and ez likewise. They depend on no item type and only
+// shrink, so each is computed once, when its point appears, and a placed box
+// is applied to it once.
+//  * Dead points: ex < mw, ey < md or ez < mh says that the cuboid itself
+//    leaves the container or meets a box. Every orientation of every type
+//    contains the cuboid, so none fits there now or later in the pass; such
+//    points never hold a feasible pair, and dropping them changes no pick and
+//    no draw. (With unit edges this is the plain "covered by a box" rule.)
+//  * C2 and most of C1: an orientation with an edge longer than the extent
+//    along it leaves the container or meets the box the extent ends at. What
+//    the extents let through (97 % of it passes C1 on the batched workload) is
+//    tested for support (C3), and only then against every box above the
+//    point's z (C1), one point at a time with the lanes over the boxes.
+//  * Same type again: points before the last step's first feasible point v
+//    held no feasible pair for the type, and still hold none: boxes only add
+//    to C1 and C2, and the placed box sits at or after v in (z, y, x) order, so
+//    its top is above every such point's z and supports none of them; its
+//    corners come after it. The scan resumes at v.
+//
+// The work per step is integer tests on data in shared memory, so instructions
+// and their dependent chains bound it; extents replace per-type masks and six
+// contact areas per point that had to be evaluated against every box at each
+// change of type, kept up to date, and moved with the points.
 //
 // The C3 test is the integer form of the reference's FP64 ratio:
 // (double)s / (double)(w*d) < 0.5  <=>  2 s < w d. Both s and w d are
@@ -798,262 +804,98 @@ __global__ void __launch_bounds__(32 * G * D, M) decoder_kernel(DecoderArgs a) {
 // s/(wd) <= 1/2 - 1/(2wd) <= 1/2 - 2^-53, a double below 1/2 that bounds the
 // rounded quotient from above (rounding is monotone); if s/(wd) >= 1/2 the
 // rounded quotient is >= 1/2 as well.
-constexpr uint32_t ST_VALID = 1u << 31;
 
-__device__ __forceinline__ uint32_t st_pack(unsigned m2, unsigned blk, unsigned sok, unsigned known) {
-    return ST_VALID | m2 | (blk << 8) | (sok << 16) | (known << 24);
+// The three edges of a type. Sets of orientations are six-bit masks over the
+// slots of TypeOrs; these give the slots whose edge along an axis is at most v.
+struct Edges {
+    int l, w, h;
+};
+__device__ __forceinline__ unsigned x_within(const Edges& E, int v) {
+    return (E.l <= v ? 0x14u : 0u) | (E.w <= v ? 0x21u : 0u) | (E.h <= v ? 0x0au : 0u);
 }
-__device__ __forceinline__ unsigned st_feasible(uint32_t s) {
-    return (s & ST_VALID) ? (s & (s >> 16) & ~(s >> 8) & 0x3fu) : 0u;
+__device__ __forceinline__ unsigned y_within(const Edges& E, int v) {
+    return (E.l <= v ? 0x28u : 0u) | (E.w <= v ? 0x12u : 0u) | (E.h <= v ? 0x05u : 0u);
 }
-
-// Evaluates items W[w0 .. w1) from scratch and stores their state. A group
-// of 2^lg lanes shares one item (lanes take every 2^lg-th box), 32 >> lg
-// items at a time, lg chosen so that a short item list still spreads over the
-// whole warp. Greedy mode stops after the first group holding a feasible
-// item. Returns {first feasible item or INT_MAX, end of the evaluated range}.
-template <typename SupT>
-__device__ __forceinline__ int2 eval_items(const bool GREEDY, const uint2* W, const unsigned short* wi, int w0, int w1,
-                                           const int4* bx, const int* bzs, int nb, const StepOrs& S,
-                                           uint32_t xmask, uint32_t ymask, int xb, int xyb,
-                                           uint32_t* st, SupT* sup, int C, int lane) {
-    int first = INT_MAX;
-    int w = w0;
-    while (w < w1) {
-        const int K = min(32, w1 - w);
-        const int lg = K > 16 ? 0 : K > 8 ? 1 : K > 4 ? 2 : K > 2 ? 3 : K > 1 ? 4 : 5;
-        const int span = 1 << lg;
-        const int q = lane >> lg, ph = lane & (span - 1);
-        const bool has = q < K;
-        const uint2 e = has ? W[w + q] : make_uint2(0, 0);
-        const unsigned m2 = e.y & 0x3fu;
-        const int jlo = (int)((e.y >> 8) & 0xfffu), jsup = (int)(e.y >> 20);
-        const int x = (int)(e.x & xmask), y = (int)((e.x >> xb) & ymask), z = (int)(e.x >> xyb);
-        const bool supz = has && z > 0;
-        int a0 = 0, a1 = 0, a2 = 0, a3 = 0, a4 = 0, a5 = 0;
-        // C3: boxes whose top is z
-        const int slo = __reduce_min_sync(FULL, supz ? jlo : INT_MAX);
-        const int shi = __reduce_max_sync(FULL, supz ? jsup : 0);
-        for (int j0 = slo; j0 < shi; j0 += 4 << lg) {
-            int4 bb[4];
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const int j = j0 + (u << lg) + ph;
-                bb[u] = j < shi ? bx[j] : make_int4(0, 0, 0, 0);
-            }
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const int j = j0 + (u << lg) + ph;
-                const int4 b = bb[u];
-                if (supz && j >= jlo && j < jsup) {
-#define PLP_ACC(o, av)                                                   \
-    {                                                                    \
-        const int ox = min(x + S.ow[o], b.z) - max(x, b.x);              \
-        const int oy = min(y + S.od[o], b.w) - max(y, b.y);              \
-        if (ox > 0 && oy > 0) av += ox * oy;                             \
-    }
-                    PLP_ACC(0, a0) PLP_ACC(1, a1) PLP_ACC(2, a2) PLP_ACC(3, a3) PLP_ACC(4, a4) PLP_ACC(5, a5)
-#undef PLP_ACC
-                }
-            }
-        }
-        for (int m = 1; m < span; m <<= 1) {
-            a0 += __shfl_xor_sync(FULL, a0, m);
-            a1 += __shfl_xor_sync(FULL, a1, m);
-            a2 += __shfl_xor_sync(FULL, a2, m);
-            a3 += __shfl_xor_sync(FULL, a3, m);
-            a4 += __shfl_xor_sync(FULL, a4, m);
-            a5 += __shfl_xor_sync(FULL, a5, m);
-        }
-        unsigned sok = 0x3fu;
-        if (z > 0) {
-            const int av[6] = {a0, a1, a2, a3, a4, a5};
-            sok = 0;
-#pragma unroll
-            for (int o = 0; o < 6; o++)
-                if (2LL * av[o] >= (long long)S.wd[o]) sok |= 1u << o;
-        }
-        const unsigned known = m2 & sok;
-        unsigned alive = has ? known : 0u;
-        // C1: boxes above z, 4 per lane per round; the "near" test (ahead of
-        // the point, within the largest edge on each axis) gates the
-        // per-orientation test. Lanes of one item AND their alive sets.
-        const int clo = __reduce_min_sync(FULL, alive ? jsup : INT_MAX);
-        for (int j0 = clo; j0 < nb; j0 += 4 << lg) {
-            int4 bb[4];
-            int bz[4];
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const int j = j0 + (u << lg) + ph;
-                const bool in = j < nb;
-                bb[u] = in ? bx[j] : make_int4(0, 0, 0, 0);
-                bz[u] = in ? bzs[j] : 0;
-            }
-            unsigned near = 0;
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const int j = j0 + (u << lg) + ph;
-                const int4 b = bb[u];
-                const bool nu = alive && j >= jsup && x < b.z && y < b.w && b.x < x + S.wmax &&
-                                b.y < y + S.dmax && bz[u] < z + S.hmax;
-                near |= (nu ? 1u : 0u) << u;
-            }
-            const unsigned todo = __reduce_or_sync(FULL, near);
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                if ((todo >> u) & 1u) {
-                    if ((near >> u) & 1u) {
-                        // offsets from the point (coordinates are below 2^16)
-                        const int dx = bb[u].x - x, dy = bb[u].y - y, dz = bz[u] - z;
-#pragma unroll
-                        for (int o = 0; o < 6; o++)
-                            if (dx < S.ow[o] && dy < S.od[o] && dz < S.oh[o]) alive &= ~(1u << o);
-                    }
-                }
-            }
-            for (int m = 1; m < span; m <<= 1) alive &= __shfl_xor_sync(FULL, alive, m);
-            if (!__any_sync(FULL, alive != 0)) break;
-        }
-        if (has && ph == 0) {
-            const int p = wi[w + q];
-            st[p] = st_pack(m2, known & ~alive, sok, known);
-            if (z > 0) {
-                sup[p] = (SupT)a0;
-                sup[C + p] = (SupT)a1;
-                sup[2 * C + p] = (SupT)a2;
-                sup[3 * C + p] = (SupT)a3;
-                sup[4 * C + p] = (SupT)a4;
-                sup[5 * C + p] = (SupT)a5;
-            }
-        }
-        w += K;
-        if (GREEDY) {
-            const unsigned bal = __ballot_sync(FULL, has && ph == 0 && alive != 0);
-            if (bal) {
-                first = w - K + ((__ffs(bal) - 1) >> lg);
-                break;
-            }
-        }
-    }
-    __syncwarp();
-    return make_int2(first, w);
+__device__ __forceinline__ unsigned z_within(const Edges& E, int v) {
+    return (E.l <= v ? 0x03u : 0u) | (E.w <= v ? 0x0cu : 0u) | (E.h <= v ? 0x30u : 0u);
 }
 
-// Applies one newly placed box to a valid point's state (C1 OR, C3 contact
-// areas). Returns the new state, or 0 when the support grew onto an
-// orientation whose C1 was never evaluated (the point is re-evaluated).
-template <typename SupT>
-__device__ __forceinline__ uint32_t st_apply_box(uint32_t s, int x, int y, int z, int4 B, int Bz, int Bz2,
-                                                 const StepOrs& S, SupT* sup, int C, int p) {
-    const bool above = Bz2 > z && x < B.z && y < B.w;
-    const bool level = z > 0 && Bz2 == z;
-    if (!above && !level) return s;   // the box neither blocks nor supports the point
-    const unsigned m2 = s & 0x3fu, known = (s >> 24) & 0x3fu;
-    unsigned blk = (s >> 8) & 0x3fu, sok = (s >> 16) & 0x3fu;
-    if (above) {
-        const int dx = B.x - x, dy = B.y - y, dz = Bz - z;
-#pragma unroll
-        for (int o = 0; o < 6; o++)
-            if (dx < S.ow[o] && dy < S.od[o] && dz < S.oh[o]) blk |= 1u << o;
+// Slots of `cand` whose C3 holds at (x, y, z), z > 0: contact with the boxes
+// [j, je), whose top is z. Areas are at most the container's footprint, below
+// 2^31, so twice an area fits 32 unsigned bits.
+__device__ __forceinline__ unsigned support_slots(unsigned cand, int x, int y, int j, int je, const Edges& E,
+                                                  const int4* bx) {
+    unsigned a0 = 0, a1 = 0, a2 = 0, a3 = 0, a4 = 0, a5 = 0;
+    const int xl = x + E.l, xw = x + E.w, xh = x + E.h, yl = y + E.l, yw = y + E.w, yh = y + E.h;
+    for (; j < je; j++) {
+        const int4 b = bx[j];
+        const int nx = -max(x, b.x), ny = -max(y, b.y);
+        const int tx = b.z + nx, ty = b.w + ny;
+        // overlap along an axis: max(0, min(x + e, b.x2) - max(x, b.x))
+        const unsigned ol = __viaddmin_s32_relu(xl, nx, tx), ow = __viaddmin_s32_relu(xw, nx, tx),
+                       oh = __viaddmin_s32_relu(xh, nx, tx);
+        const unsigned pl = __viaddmin_s32_relu(yl, ny, ty), pw = __viaddmin_s32_relu(yw, ny, ty),
+                       ph = __viaddmin_s32_relu(yh, ny, ty);
+        a0 += ow * ph;
+        a1 += oh * pw;
+        a2 += ol * ph;
+        a3 += oh * pl;
+        a4 += ol * pw;
+        a5 += ow * pl;
     }
-    if (level) {
-#pragma unroll
-        for (int o = 0; o < 6; o++) {
-            if ((m2 >> o) & 1u) {
-                const int ox = min(x + S.ow[o], B.z) - max(x, B.x);
-                const int oy = min(y + S.od[o], B.w) - max(y, B.y);
-                if (ox > 0 && oy > 0) {
-                    const int v = (int)sup[o * C + p] + ox * oy;
-                    sup[o * C + p] = (SupT)v;
-                    if (2LL * v >= (long long)S.wd[o]) sok |= 1u << o;
-                }
-            }
+    // footprints of the slots in `cand` fit the container; others' bits are masked off
+    const unsigned wh = (unsigned)E.w * E.h, lh = (unsigned)E.l * E.h, lw = (unsigned)E.l * E.w;
+    return cand & ((2u * a0 >= wh ? 0x01u : 0u) | (2u * a1 >= wh ? 0x02u : 0u) | (2u * a2 >= lh ? 0x04u : 0u) |
+                   (2u * a3 >= lh ? 0x08u : 0u) | (2u * a4 >= lw ? 0x10u : 0u) | (2u * a5 >= lw ? 0x20u : 0u));
+}
+
+// Warp: slots that some box of [j0, nb) overlaps at (x, y, z) (C1; boxes
+// below j0 end at or under z). Offsets from the point keep each axis to one
+// subtraction and three compares.
+__device__ __forceinline__ unsigned blocked_slots(int x, int y, int z, int j0, int nb, const Edges& E, const int4* bx,
+                                                  const int* bzs, int lane) {
+    unsigned blk = 0;
+    for (int jb = j0; jb < nb; jb += 32) {
+        const int j = jb + lane;
+        if (j < nb) {
+            const int4 b = bx[j];
+            const int bz = bzs[j];
+            if (b.z > x && b.w > y)
+                blk |= ~(x_within(E, b.x - x) | y_within(E, b.y - y) | z_within(E, bz - z));
         }
-        if (sok & m2 & ~known) return 0u;
     }
-    return st_pack(m2, blk, sok, known);
+    return __reduce_or_sync(FULL, blk & 0x3fu);
 }
 
 // Smallest edges over the instance's orientations (InstDesc::mw, md, mh) and
-// the container, for the dead-point rule of place1.
+// the container.
 struct MinEdges {
     int w, d, h;
     int L, W, H;
 };
 
-// Warp: pick the pair, place the box, drop the points it makes dead and
-// insert its live corners (invalid), then update the top-sorted box tables
-// and the top-z index. pp is the first point holding a feasible pair.
-//
-// A point is dead when the cuboid of the instance's smallest edges at it
-// leaves the container or meets a placed box: every orientation of every
-// type contains that cuboid, so none fits there now or later in the pass.
-// (With unit edges this is the plain "covered by a box" rule.) Dead points
-// never hold a feasible pair, so dropping them changes no pick and no draw.
-// Every phase of a step is bound by its integer work per live point; on the
-// batched workload a step meets 41 of them instead of 128 (stress 37 of
-// 137). Measured, decoder alone, 512 batched instances x 128 restarts at tile
-// (128, 384): 24.5 -> 16.8 ms; 64 stress instances x 512: 21.5 -> 12.4 ms; 1024
-// restarts of one instance: 0.554 -> 0.409 ms.
-template <typename SupT>
-__device__ __forceinline__ int place1(int t, int pp, bool full, uint32_t* mt, int& mpos, uint32_t* keys,
-                                      uint32_t* st, SupT* sup, int4* bx, int* bzs, int* z2s,
-                                      unsigned short* bis, unsigned short* zt, int Hz, int& nc, int& nb,
-                                      int P, int C, const StepOrs& S, uint32_t xmask, uint32_t ymask,
-                                      int xb, int xyb, unsigned long long* pass_out, long long& vol,
-                                      int4& Bo, int& Bzo, int& Bz2o, const MinEdges& ME, int lane) {
-    int pick = pp;
-    int pick_oi = __ffs(st_feasible(st[pp])) - 1;
-    if (full) {
-        int count = 0;
-        for (int i = pp + lane; i < nc; i += 32) count += __popc(st_feasible(st[i]));
-        count = __reduce_add_sync(FULL, count);
-        const int idx = mt_randrange(mt, mpos, lane, count);
-        if (idx < 0) return ERR_RNG;
-        // idx-th feasible pair in (point, orientation) order
-        int run = 0;
-        for (int cb = pp; cb < nc; cb += 32) {
-            const int i = cb + lane;
-            const unsigned m = i < nc ? st_feasible(st[i]) : 0u;
-            const int c = __popc(m);
-            // lane prefix of the pair counts (each below 8) from their bits
-            const unsigned b0 = __ballot_sync(FULL, c & 1), b1 = __ballot_sync(FULL, c & 2),
-                           b2 = __ballot_sync(FULL, c & 4);
-            const unsigned lt = lanemask_lt();
-            const int excl = __popc(b0 & lt) + 2 * __popc(b1 & lt) + 4 * __popc(b2 & lt);
-            const int tot = __popc(b0) + 2 * __popc(b1) + 4 * __popc(b2);
-            if (idx < run + tot) {
-                const unsigned hit = __ballot_sync(FULL, idx < run + excl + c);
-                const int l = __ffs(hit) - 1;
-                const int ex = __shfl_sync(FULL, excl, l);
-                const unsigned ml = __shfl_sync(FULL, m, l);
-                pick = cb + l;
-                pick_oi = __fns(ml, 0, idx - run - ex + 1);
-                break;
-            }
-            run += tot;
-        }
-    }
-    const uint32_t pkey = keys[pick];
+// Warp: places a w x d x h box at the point with key pkey: top-sorted box
+// tables, top-z index, then every point from buffer K to buffer K2 (arrays of
+// `cap` entries: key, x | y << 16 extents, z extent) with the box applied to
+// its extents, dead points left out and the box's live corners merged in.
+// resume: in, a point index; out, the survivors before it.
+__device__ __forceinline__ int place1(uint32_t pkey, int pw, int pd, int ph, int& resume, const uint32_t* K,
+                                      uint32_t* K2, int cap, int4* bx, int* bzs, int* z2s, unsigned short* bis,
+                                      unsigned short* zt, int Hz, int& nc, int& nb, int P, int C, uint32_t xmask,
+                                      uint32_t ymask, int xb, int xyb, const MinEdges& ME, int lane) {
     const int px = (int)(pkey & xmask), py = (int)((pkey >> xb) & ymask), pz = (int)(pkey >> xyb);
-    int pw = 0, pd = 0, ph = 0;
-#pragma unroll
-    for (int o = 0; o < 6; o++)
-        if (o == pick_oi) { pw = S.ow[o]; pd = S.od[o]; ph = S.oh[o]; }
     const int px2 = px + pw, py2 = py + pd, pz2 = pz + ph;
     if (nb >= P) return ERR_BOX_CAP;
-    if (lane == 0) pass_out[nb] = pack_place(px, py, pz, pick_oi, t);
-    vol += 1LL * pw * pd * ph;
     // Box tables, one pass from the top: the corners of the new box that a
     // placed box makes dead, and the boxes whose top is above the new box's
     // move up one slot (each round reads before it writes, and writes only
     // slots it or an earlier round has read).
     const int pxm = px + ME.w, px2m = px2 + ME.w, pym = py + ME.d, py2m = py2 + ME.d, pzm = pz + ME.h,
               pz2m = pz2 + ME.h;
-    unsigned cov = 1u;   // corner 0 = (px, py, pz): inside the new box
-    if (px2m > ME.L) cov |= 0xaau;
-    if (py2m > ME.W) cov |= 0xccu;
-    if (pz2m > ME.H) cov |= 0xf0u;
+    unsigned dead = 1u;   // corner 0 = (px, py, pz): inside the new box
+    if (px2m > ME.L) dead |= 0xaau;
+    if (py2m > ME.W) dead |= 0xccu;
+    if (pz2m > ME.H) dead |= 0xf0u;
     int nabove = 0;
     for (int hi = nb; hi > 0; hi -= 32) {
         const int jj = hi - 1 - lane;
@@ -1069,7 +911,7 @@ __device__ __forceinline__ int place1(int t, int pp, bool full, uint32_t* mt, in
             const unsigned xin = (b.x < pxm && px < b.z ? 0x55u : 0u) | (b.x < px2m && px2 < b.z ? 0xaau : 0u);
             const unsigned yin = (b.y < pym && py < b.w ? 0x33u : 0u) | (b.y < py2m && py2 < b.w ? 0xccu : 0u);
             const unsigned zin = (bzb < pzm && pz < bzt ? 0x0fu : 0u) | (bzb < pz2m && pz2 < bzt ? 0xf0u : 0u);
-            cov |= xin & yin & zin;
+            dead |= xin & yin & zin;
         }
         const bool up = in && bzt > pz2;
         nabove += __popc(__ballot_sync(FULL, up));
@@ -1081,7 +923,7 @@ __device__ __forceinline__ int place1(int t, int pp, bool full, uint32_t* mt, in
             bis[jj + 1] = bi;
         }
     }
-    cov = __reduce_or_sync(FULL, cov);
+    unsigned live = ~__reduce_or_sync(FULL, dead) & 0xffu;
     {
         const int ip = nb - nabove;   // after the boxes with equal tops
         __syncwarp();
@@ -1095,104 +937,85 @@ __device__ __forceinline__ int place1(int t, int pp, bool full, uint32_t* mt, in
     if (zt)
         for (int zz = pz2 + 1 + lane; zz < Hz; zz += 32) zt[zz]++;
     nb++;
-    // new corners, in index order c = (cz << 2) | (cy << 1) | cx, which is
-    // their (z, y, x) order
+    // Points: one pass from K to K2. Corners in index order
+    // c = (cz << 2) | (cy << 1) | cx are in key order; lane c counts the
+    // survivors below corner c, and a corner whose key a survivor has is not
+    // new. Keys ascend, so it is found before any point above it is written.
     const uint32_t ck = ((uint32_t)((lane & 4) ? pz2 : pz) << xyb) | ((uint32_t)((lane & 2) ? py2 : py) << xb) |
                         (uint32_t)((lane & 1) ? px2 : px);
-    const unsigned live = ~cov & 0xffu;
-    // Survivors move down in place: every destination is at or below its
-    // source, and each round reads before it writes. The same round counts,
-    // for each live corner, the survivors below it (its rank) and looks for
-    // its key among them (then it is no new point).
-    int ns = 0, rank = 0;
-    bool dup = false;
+    int ns = 0, rank = 0, at = 0;
     for (int cb = 0; cb < nc; cb += 32) {
         const int i = cb + lane;
         bool keep = false;
         uint32_t key = 0;
+        int ex = 0, ey = 0, ez = 0;
         if (i < nc) {
-            key = keys[i];
+            key = K[i];
+            const uint32_t exy = K[cap + i];
+            ex = (int)(exy & 0xffffu);
+            ey = (int)(exy >> 16);
+            ez = (int)K[2 * cap + i];
             const int x = (int)(key & xmask), y = (int)((key >> xb) & ymask), z = (int)(key >> xyb);
-            keep = !(px < x + ME.w && x < px2 && py < y + ME.d && y < py2 && pz < z + ME.h && z < pz2);
+            const bool ix = px < x + ME.w && x < px2, iy = py < y + ME.d && y < py2, iz = pz < z + ME.h && z < pz2;
+            if (iy && iz && x < px2) ex = min(ex, px - x);
+            if (ix && iz && y < py2) ey = min(ey, py - y);
+            if (ix && iy && z < pz2) ez = min(ez, pz - z);
+            keep = ex >= ME.w && ey >= ME.d && ez >= ME.h;
         }
         const unsigned bal = __ballot_sync(FULL, keep);
+        int off = 0;
         for (unsigned m = live; m; m &= m - 1) {
             const int c = __ffs(m) - 1;
             const uint32_t kc = __shfl_sync(FULL, ck, c);
-            const unsigned lt = __ballot_sync(FULL, key < kc) & bal, eq = __ballot_sync(FULL, key == kc) & bal;
-            if (lane == c) {
-                rank += __popc(lt);
-                dup = dup || eq != 0;
+            if (__any_sync(FULL, keep && key == kc)) {
+                live &= ~(1u << c);
+                continue;
             }
+            const unsigned lt = __ballot_sync(FULL, key < kc) & bal;
+            if (lane == c) rank += __popc(lt);
+            off += key > kc;
         }
-        const int kept = __popc(bal);
-        if (ns == cb && kept == min(32, nc - cb)) {   // nothing dropped up to here
-            ns += kept;
-            continue;
-        }
-        uint32_t s = 0;
-        int s0 = 0, s1 = 0, s2 = 0, s3 = 0, s4 = 0, s5 = 0;
+        if (resume >= cb && resume < cb + 32) at = ns + __popc(bal & ((1u << (resume - cb)) - 1u));
         if (keep) {
-            s = st[i];
-            s0 = sup[i]; s1 = sup[C + i]; s2 = sup[2 * C + i];
-            s3 = sup[3 * C + i]; s4 = sup[4 * C + i]; s5 = sup[5 * C + i];
+            const int d = ns + __popc(bal & lanemask_lt()) + off;
+            K2[d] = key;
+            K2[cap + d] = (uint32_t)ex | ((uint32_t)ey << 16);
+            K2[2 * cap + d] = (uint32_t)ez;
         }
-        __syncwarp();
-        if (keep) {
-            const int d = ns + __popc(bal & lanemask_lt());
-            keys[d] = key;
-            st[d] = s;
-            if ((s & ST_VALID) && (key >> xyb) > 0) {
-                sup[d] = (SupT)s0; sup[C + d] = (SupT)s1; sup[2 * C + d] = (SupT)s2;
-                sup[3 * C + d] = (SupT)s3; sup[4 * C + d] = (SupT)s4; sup[5 * C + d] = (SupT)s5;
-            }
-        }
-        ns += kept;
+        ns += __popc(bal);
     }
-    __syncwarp();
-    const bool isnew = ((live >> lane) & 1u) && !dup;   // live has bits 0-7 only
-    const unsigned newm = __ballot_sync(FULL, isnew);
-    const int nnew = ns + __popc(newm);
-    if (nnew > C) return ERR_CAND_CAP;
-    if (newm) {
-        const int first_ins = __reduce_min_sync(FULL, isnew ? rank : INT_MAX);
-        // survivors at or after the first insertion move up by the number of
-        // new corners below them; rounds go from the top, reading first
-        for (int hi = ns; hi > first_ins; hi -= 32) {
-            const int i = hi - 1 - lane;
-            const bool in = i >= first_ins;
-            uint32_t key = 0, s = 0;
-            int s0 = 0, s1 = 0, s2 = 0, s3 = 0, s4 = 0, s5 = 0;
-            if (in) {
-                key = keys[i];
-                s = st[i];
-                s0 = sup[i]; s1 = sup[C + i]; s2 = sup[2 * C + i];
-                s3 = sup[3 * C + i]; s4 = sup[4 * C + i]; s5 = sup[5 * C + i];
+    resume = at;
+    nc = ns + __popc(live);
+    if (nc > C) return ERR_CAND_CAP;
+    __syncwarp();   // box tables and top-z index are final
+    // extents of the new corners: lanes over the boxes above the corner's z
+    int nth = 0;
+    for (unsigned m = live; m; m &= m - 1) {
+        const int c = __ffs(m) - 1;
+        const int x = (c & 1) ? px2 : px, y = (c & 2) ? py2 : py, z = (c & 4) ? pz2 : pz;
+        int ex = ME.L - x, ey = ME.W - y, ez = ME.H - z;
+        for (int jb = box_start(zt, z2s, nb, z + 1); jb < nb; jb += 32) {
+            const int j = jb + lane;
+            if (j < nb) {
+                const int4 b = bx[j];
+                const int bz = bzs[j];
+                const bool ix = b.x < x + ME.w && x < b.z, iy = b.y < y + ME.d && y < b.w, iz = bz < z + ME.h;
+                if (iy && iz && x < b.z) ex = min(ex, b.x - x);
+                if (ix && iz && y < b.w) ey = min(ey, b.y - y);
+                if (ix && iy) ez = min(ez, bz - z);
             }
-            int off = 0;
-            for (unsigned m = newm; m; m &= m - 1) off += __shfl_sync(FULL, ck, __ffs(m) - 1) < key;
-            __syncwarp();
-            if (in && off) {
-                const int d = i + off;
-                keys[d] = key;
-                st[d] = s;
-                if ((s & ST_VALID) && (key >> xyb) > 0) {
-                    sup[d] = (SupT)s0; sup[C + d] = (SupT)s1; sup[2 * C + d] = (SupT)s2;
-                    sup[3 * C + d] = (SupT)s3; sup[4 * C + d] = (SupT)s4; sup[5 * C + d] = (SupT)s5;
-                }
-            }
-            __syncwarp();
         }
-        if (isnew) {
-            const int d = rank + __popc(newm & ((1u << lane) - 1u));
-            keys[d] = ck;
-            st[d] = 0u;
+        ex = __reduce_min_sync(FULL, ex);
+        ey = __reduce_min_sync(FULL, ey);
+        ez = __reduce_min_sync(FULL, ez);
+        if (lane == c) {
+            const int d = rank + nth;
+            K2[d] = ck;
+            K2[cap + d] = (uint32_t)ex | ((uint32_t)ey << 16);
+            K2[2 * cap + d] = (uint32_t)ez;
         }
+        nth++;
     }
-    nc = nnew;
-    Bo = make_int4(px, py, px2, py2);
-    Bzo = pz;
-    Bz2o = pz2;
     __syncwarp();
     return ERR_NONE;
 }
@@ -1367,22 +1190,17 @@ __device__ __forceinline__ void serve_finish(const DecoderArgs& a, const ServeAr
 // MODE 0: batch launch; 1: serving launch, main decoder (pushes restarts
 // that outgrow its tile to the overflow ring); 2: serving launch, overflow
 // decoder (deeper tile in global memory, takes the overflow ring).
-template <typename SupT, int MODE>
+template <int MODE>
 __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned char* base, int gdec,
                                               const ServeArgs& sv) {
     const int lane = threadIdx.x & 31;
-    const Dec1Layout lay = dec1_layout(a.P, a.C, a.Hz, (int)sizeof(SupT));
-    const int C = a.C;
+    const Dec1Layout lay = dec1_layout(a.P, a.C, a.Hz);
     uint32_t* mt = reinterpret_cast<uint32_t*>(base);
     int4* bx = reinterpret_cast<int4*>(base + lay.off_bx);
     int* bzs = reinterpret_cast<int*>(base + lay.off_bz);
     int* z2s = reinterpret_cast<int*>(base + lay.off_z2);
     unsigned short* bis = reinterpret_cast<unsigned short*>(base + lay.off_bi);
-    uint32_t* keys = reinterpret_cast<uint32_t*>(base + lay.off_key);
-    uint32_t* st = reinterpret_cast<uint32_t*>(base + lay.off_st);
-    SupT* sup = reinterpret_cast<SupT*>(base + lay.off_sup);
-    uint2* Wl = reinterpret_cast<uint2*>(base + lay.off_w);
-    unsigned short* wi = reinterpret_cast<unsigned short*>(base + lay.off_wi);
+    uint32_t* pts = reinterpret_cast<uint32_t*>(base + lay.off_pts);
     unsigned short* zt = a.Hz ? reinterpret_cast<unsigned short*>(base + lay.off_zt) : nullptr;
 
     constexpr bool SERVE = MODE != 0;
@@ -1452,131 +1270,146 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
         double best_score = 0.0;
 
         for (int pass = 0; pass < I.passes && err == ERR_NONE; pass++) {
-            int nb = 0, nc = 1;
+            int nb = 0, nc = 1, cur = 0;
             long long vol = 0;
             if (zt)
                 for (int i = lane; i < a.Hz; i += 32) zt[i] = 0;
             if (lane == 0) {
-                keys[0] = 0u;
-                st[0] = 0u;
+                pts[0] = 0u;
+                pts[lay.cap] = (uint32_t)L | ((uint32_t)W << 16);
+                pts[2 * lay.cap] = (uint32_t)H;
             }
             __syncwarp();
             int state_type = -1;
-            bool pending = false;   // a placed box not yet applied to the valid states
+            int resume = 0;         // points before it hold no feasible pair of state_type
             bool stuck = false;     // the last step of state_type found no feasible pair
-            int4 B = make_int4(0, 0, 0, 0);
-            int Bz = 0, Bz2 = 0;
             int t_next = I.n_steps > 0 ? ld_table<SERVE>(a.step_type + I.step_off) : 0;
             for (int sti = 0; sti < I.n_steps; sti++) {
                 const int t = t_next;
                 if (sti + 1 < I.n_steps) t_next = ld_table<SERVE>(a.step_type + I.step_off + sti + 1);
                 // With no box placed since, another item of that type meets the
-                // same states and finds no pair either; it draws no random
+                // same points and finds no pair either; it draws no random
                 // number, so the step is skipped without changing the result.
                 if (stuck && t == state_type) continue;
                 const TypeOrs& T = a.types[I.type_off + t];
-                StepOrs S;
-                S.no = ld_table<SERVE>(&T.n);
-                if (S.no == 0) continue;
-                S.wmax = S.dmax = S.hmax = 0;
-#pragma unroll
-                for (int o = 0; o < 6; o++) {
-                    S.ow[o] = ld_table<SERVE>(&T.w[o]);
-                    S.od[o] = ld_table<SERVE>(&T.d[o]);
-                    S.oh[o] = ld_table<SERVE>(&T.h[o]);
-                    S.wd[o] = S.ow[o] * S.od[o];
-                    S.wmax = max(S.wmax, S.ow[o]);
-                    S.dmax = max(S.dmax, S.od[o]);
-                    S.hmax = max(S.hmax, S.oh[o]);
-                }
-                const bool fresh = t != state_type;
+                const int el = ld_table<SERVE>(&T.el);
+                const Edges E{el & 0x1ffff, ld_table<SERVE>(&T.ew), ld_table<SERVE>(&T.eh)};
+                const unsigned slots = (unsigned)el >> 20;
+                if (slots == 0) continue;
+                const int from = t == state_type ? resume : 0;
                 state_type = t;
-                const bool apply = pending && !fresh;
-                pending = false;
-                // filter: bring valid states up to date with the last box and
-                // read their feasible sets; list the invalid points that have an
-                // orientation inside the container and, above the floor, a box
-                // top at their height. v = first valid point with a feasible pair.
-                int nW = 0, v = INT_MAX, nWg = -1;
-                for (int cb = 0; cb < nc; cb += 32) {
+                const uint32_t* K = pts + cur * 3 * lay.cap;
+                uint32_t* K2 = pts + (cur ^ 1) * 3 * lay.cap;
+                // items: the points whose extents let an orientation through,
+                // {key, slots | point index << 8}
+                uint2* Wl = reinterpret_cast<uint2*>(K2);
+                int nW = 0;
+                for (int cb = from; cb < nc; cb += 32) {
                     const int i = cb + lane;
-                    unsigned f = 0;
-                    bool cand = false;
-                    uint2 it = make_uint2(0, 0);
+                    unsigned m = 0;
+                    uint32_t key = 0;
                     if (i < nc) {
-                        const uint32_t key = keys[i];
-                        const int x = (int)(key & xmask), y = (int)((key >> xb) & ymask), z = (int)(key >> xyb);
-                        uint32_t s = fresh ? 0u : st[i];
-                        const uint32_t s_in = s;
-                        if ((s & ST_VALID) && apply) s = st_apply_box(s, x, y, z, B, Bz, Bz2, S, sup, C, i);
-                        if (s & ST_VALID) {
-                            f = st_feasible(s);
-                        } else {
-                            unsigned m = 0;
-#pragma unroll
-                            for (int o = 0; o < 6; o++)
-                                if (o < S.no && x + S.ow[o] <= L && y + S.od[o] <= W && z + S.oh[o] <= H) m |= 1u << o;
-                            if (!m) {
-                                s = ST_VALID;   // nothing fits: infeasible for the rest of the run
-                            } else {
-                                s = 0u;
-                                const int jlo = box_start(zt, z2s, nb, z);
-                                const int jsup = z > 0 ? box_start(zt, z2s, nb, z + 1) : jlo;
-                                if (z == 0 || jsup > jlo) {
-                                    cand = true;
-                                    it = make_item(key, m, jlo, jsup);
-                                }
-                            }
-                        }
-                        if (s != s_in || fresh) st[i] = s;
+                        key = K[i];
+                        const uint32_t exy = K[lay.cap + i];
+                        m = slots & x_within(E, (int)(exy & 0xffffu)) & y_within(E, (int)(exy >> 16)) &
+                            z_within(E, (int)K[2 * lay.cap + i]);
                     }
-                    const unsigned bal = __ballot_sync(FULL, cand);
-                    if (v == INT_MAX) {
-                        const unsigned bf = __ballot_sync(FULL, f != 0);
-                        if (bf) {
-                            v = cb + __ffs(bf) - 1;
-                            nWg = nW + __popc(bal & ((1u << (v - cb)) - 1u));
-                        }
-                    }
-                    if (cand) {
-                        const int d = nW + __popc(bal & lanemask_lt());
-                        Wl[d] = it;
-                        wi[d] = (unsigned short)i;
-                    }
+                    const unsigned bal = __ballot_sync(FULL, m != 0);
+                    if (m) Wl[nW + __popc(bal & lanemask_lt())] = make_uint2(key, m | ((unsigned)i << 8));
                     nW += __popc(bal);
                 }
-                if (nWg < 0) nWg = nW;
                 __syncwarp();
-                // greedy: the invalid points before v, in order; then, on the
-                // random branch, every item left (one evaluation site)
-                int pp = v, lo = 0, hi = nWg;
-                bool greedy = true, full = false;
-                for (;;) {
-                    if (lo < hi) {
-                        const int2 r = eval_items(greedy, Wl, wi, lo, hi, bx, bzs, nb, S, xmask, ymask, xb, xyb,
-                                                  st, sup, C, lane);
-                        if (greedy) {
-                            if (r.x != INT_MAX) pp = wi[r.x];
-                            lo = r.y;
+                // C3 for 32 items at a time, then C1 item by item in order. The
+                // first item with a feasible pair decides the branch; the random
+                // branch goes on to the end and keeps every item's feasible set.
+                int first = -1, pick_p = 0;      // item and point of the first feasible pair
+                unsigned pick_m = 0;             // its feasible set
+                uint32_t pick_key = 0;
+                int count = 0;
+                bool full = false;
+                for (int w0 = 0; w0 < nW; w0 += 32) {
+                    const uint2 e = w0 + lane < nW ? Wl[w0 + lane] : make_uint2(0, 0);
+                    unsigned cand = e.y & 0x3fu;
+                    const int z = (int)(e.x >> xyb);
+                    if (z > 0 && cand) {
+                        const int j = box_start(zt, z2s, nb, z), je = box_start(zt, z2s, nb, z + 1);
+                        cand = support_slots(cand, (int)(e.x & xmask), (int)((e.x >> xb) & ymask), j, je, E, bx);
+                    }
+                    __syncwarp();
+                    unsigned mine = 0;
+                    for (unsigned bal = __ballot_sync(FULL, cand != 0); bal; bal &= bal - 1) {
+                        const int q = __ffs(bal) - 1;
+                        const uint32_t kq = __shfl_sync(FULL, e.x, q);
+                        const int zq = (int)(kq >> xyb);
+                        const unsigned ok = __shfl_sync(FULL, cand, q) &
+                                            ~blocked_slots((int)(kq & xmask), (int)((kq >> xb) & ymask), zq,
+                                                           box_start(zt, z2s, nb, zq + 1), nb, E, bx, bzs, lane);
+                        if (lane == q) mine = ok;
+                        if (ok && first < 0) {
+                            first = w0 + q;
+                            pick_key = kq;
+                            pick_m = ok;
+                            pick_p = (int)(__shfl_sync(FULL, e.y, q) >> 8);
+                            // random() only once a feasible pair exists
+                            full = randomized && mt_random(mt, mpos, lane) >= 1.0 - I.eps;
+                            if (!full) break;
                         }
                     }
-                    if (!greedy || pp == INT_MAX) break;
-                    full = randomized && mt_random(mt, mpos, lane) >= 1.0 - I.eps;
-                    if (!full || lo >= nW) break;
-                    greedy = false;   // every feasible pair is needed
-                    hi = nW;
+                    if (first >= 0) {
+                        if (!full) break;
+                        count += __popc(mine);
+                        if (w0 + lane < nW) Wl[w0 + lane].y = mine;
+                    }
                 }
-                stuck = pp == INT_MAX;
+                stuck = first < 0;
                 if (stuck) continue;                     // no feasible pair: no draw
-                err = place1(t, pp, full, mt, mpos, keys, st, sup, bx, bzs, z2s, bis, zt, a.Hz, nc, nb, a.P,
-                             C, S, xmask, ymask, xb, xyb, pass_out, vol, B, Bz, Bz2,
-                             MinEdges{I.mw, I.md, I.mh, L, W, H}, lane);
+                int slot = __ffs(pick_m) - 1;
+                if (full) {
+                    const int idx = mt_randrange(mt, mpos, lane, __reduce_add_sync(FULL, count));
+                    if (idx < 0) {
+                        err = ERR_RNG;
+                        break;
+                    }
+                    __syncwarp();
+                    // idx-th feasible pair in (point, orientation) order
+                    int run = 0;
+                    for (int w0 = first & ~31; w0 < nW; w0 += 32) {
+                        const uint2 e = w0 + lane < nW ? Wl[w0 + lane] : make_uint2(0, 0);
+                        const int c = __popc(e.y);
+                        // lane prefix of the pair counts (each below 8) from their bits
+                        const unsigned b0 = __ballot_sync(FULL, c & 1), b1 = __ballot_sync(FULL, c & 2),
+                                       b2 = __ballot_sync(FULL, c & 4);
+                        const unsigned lt = lanemask_lt();
+                        const int excl = __popc(b0 & lt) + 2 * __popc(b1 & lt) + 4 * __popc(b2 & lt);
+                        const int tot = __popc(b0) + 2 * __popc(b1) + 4 * __popc(b2);
+                        if (idx < run + tot) {
+                            const int q = __ffs(__ballot_sync(FULL, idx < run + excl + c)) - 1;
+                            unsigned m = __shfl_sync(FULL, e.y, q);
+                            for (int k = idx - run - __shfl_sync(FULL, excl, q); k > 0; k--) m &= m - 1;
+                            pick_key = __shfl_sync(FULL, e.x, q);
+                            slot = __ffs(m) - 1;
+                            break;
+                        }
+                        run += tot;
+                    }
+                }
+                const int pw = (0x14 >> slot) & 1 ? E.l : (0x21 >> slot) & 1 ? E.w : E.h;
+                const int pd = (0x28 >> slot) & 1 ? E.l : (0x12 >> slot) & 1 ? E.w : E.h;
+                const int ph = slot < 2 ? E.l : slot < 4 ? E.w : E.h;
+                resume = pick_p;
+                if (lane == 0 && nb < a.P)
+                    pass_out[nb] = pack_place((int)(pick_key & xmask), (int)((pick_key >> xb) & ymask),
+                                              (int)(pick_key >> xyb), __popc(slots & ((1u << slot) - 1u)), t);
+                vol += 1LL * pw * pd * ph;
+                __syncwarp();   // every lane has read the item list before K2 is written
+                err = place1(pick_key, pw, pd, ph, resume, K, K2, lay.cap, bx, bzs, z2s, bis, zt, a.Hz, nc, nb, a.P,
+                             a.C, xmask, ymask, xb, xyb, MinEdges{I.mw, I.md, I.mh, L, W, H}, lane);
                 if (err != ERR_NONE) break;
-                pending = true;
+                cur ^= 1;
             }
             if (err != ERR_NONE) break;
             const double score =
-                fsr_score_warp(bx, bzs, z2s, bis, nb, I.mu, reinterpret_cast<char*>(keys), lane, nullptr, zt);
+                fsr_score_warp(bx, bzs, z2s, bis, nb, I.mu, reinterpret_cast<char*>(pts), lane, nullptr, zt);
             const bool acc = !I.has_theta || score >= I.theta;
             bool take;
             if (acc) take = !have_acc || vol > best_vol || (vol == best_vol && nb > best_n);
@@ -1652,14 +1485,12 @@ static DecoderArgs decoder_args(const DecodeLaunch& L) {
 }
 
 #ifndef PLP_SERVE_TU
-// S16: contact areas stored as 16-bit (every footprint area < 65536)
-template <int D, int M, int S16>
+template <int D, int M>
 __global__ void __launch_bounds__(32 * D, M) decoder1_kernel(DecoderArgs a) {
-    using SupT = typename std::conditional<S16 != 0, unsigned short, int>::type;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int dec = threadIdx.x >> 5;
-    const Dec1Layout lay = dec1_layout(a.P, a.C, a.Hz, (int)sizeof(SupT));
-    decoder1_body<SupT, 0>(a, smem_raw + (size_t)dec * lay.bytes, blockIdx.x * D + dec, ServeArgs{});
+    const Dec1Layout lay = dec1_layout(a.P, a.C, a.Hz);
+    decoder1_body<0>(a, smem_raw + (size_t)dec * lay.bytes, blockIdx.x * D + dec, ServeArgs{});
 }
 
 
@@ -1840,17 +1671,16 @@ __global__ void gather_best_kernel(const InstDesc* __restrict__ inst, int n_inst
 
 using DecoderFn = void (*)(DecoderArgs);
 
-// G = 1: the incremental single-warp decoder (16- or 32-bit contact areas);
-// G > 1: the multi-warp decoder
+// G = 1: the single-warp decoder; G > 1: the multi-warp decoder
 template <int G, int D, int M>
-static DecoderFn pick_kernel(int sup16) {
-    if constexpr (G == 1) return sup16 ? decoder1_kernel<D, M, 1> : decoder1_kernel<D, M, 0>;
+static DecoderFn pick_kernel() {
+    if constexpr (G == 1) return decoder1_kernel<D, M>;
     else return decoder_kernel<G, D, M>;
 }
 
-static DecoderFn decoder_fn(int G, int D, int M, int sup16 = 0) {
+static DecoderFn decoder_fn(int G, int D, int M) {
 #define PLP_PICK(g, d, m) \
-    if (G == g && D == d && M == m) return pick_kernel<g, d, m>(sup16);
+    if (G == g && D == d && M == m) return pick_kernel<g, d, m>();
     PLP_DECODER_CONFIGS(PLP_PICK)
 #undef PLP_PICK
     return nullptr;
@@ -1899,14 +1729,14 @@ cudaError_t cached_occupancy(const void* fn, int threads, int smem, int* ctas_pe
 
 
 static int decoder_launch_smem(const DecodeLaunch& L) {
-    return decoder_smem_bytes(L.P, L.C, L.Hz, L.warps_per_decoder, L.sup16) * L.decoders_per_cta;
+    return decoder_smem_bytes(L.P, L.C, L.Hz, L.warps_per_decoder) * L.decoders_per_cta;
 }
 
 // Function attributes (dynamic shared memory) for a launch; not a stream
 // operation, so it is done before any capture.
 cudaError_t configure_decoder(const DecodeLaunch& L) {
     if (L.engine == 1) return configure_block(L);
-    DecoderFn fn = decoder_fn(L.warps_per_decoder, L.decoders_per_cta, L.min_blocks, L.sup16);
+    DecoderFn fn = decoder_fn(L.warps_per_decoder, L.decoders_per_cta, L.min_blocks);
     if (!fn) return cudaErrorInvalidConfiguration;
     return ensure_dyn_smem(reinterpret_cast<const void*>(fn), decoder_launch_smem(L));
 }
@@ -1914,7 +1744,7 @@ cudaError_t configure_decoder(const DecodeLaunch& L) {
 // Stream operations only (counter resets and the launch): capturable.
 cudaError_t enqueue_decoder(const DecodeLaunch& L, cudaStream_t st) {
     if (L.engine == 1) return enqueue_block(L, st);
-    DecoderFn fn = decoder_fn(L.warps_per_decoder, L.decoders_per_cta, L.min_blocks, L.sup16);
+    DecoderFn fn = decoder_fn(L.warps_per_decoder, L.decoders_per_cta, L.min_blocks);
     if (!fn) return cudaErrorInvalidConfiguration;
     cudaError_t e = cudaMemsetAsync(L.work_next, 0, sizeof(int), st);
     if (e != cudaSuccess) return e;
@@ -1936,10 +1766,10 @@ cudaError_t launch_seed_table(long long lo, int n, const uint32_t* mt_init, uint
     return cudaGetLastError();
 }
 
-cudaError_t decoder_occupancy(int P, int C, int Hz, int G, int D, int M, int* ctas_per_sm, int sup16) {
-    DecoderFn fn = decoder_fn(G, D, M, sup16);
+cudaError_t decoder_occupancy(int P, int C, int Hz, int G, int D, int M, int* ctas_per_sm) {
+    DecoderFn fn = decoder_fn(G, D, M);
     if (!fn) return cudaErrorInvalidConfiguration;
-    const int smem = decoder_smem_bytes(P, C, Hz, G, sup16) * D;
+    const int smem = decoder_smem_bytes(P, C, Hz, G) * D;
     return cached_occupancy(reinterpret_cast<const void*>(fn), 32 * G * D, smem, ctas_per_sm);
 }
 
@@ -2018,9 +1848,8 @@ cudaError_t launch_gather_best(const InstDesc* inst, int n_inst, const int2* bes
 
 #ifdef PLP_SERVE_TU
 // The serving launch: the single-warp decoder over the host-published ring.
-template <int D, int M, int S16>
+template <int D, int M>
 __global__ void __launch_bounds__(32 * D, M) serve_kernel(DecoderArgs a, ServeArgs s) {
-    using SupT = typename std::conditional<S16 != 0, unsigned short, int>::type;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int dec = threadIdx.x >> 5;
     const int gdec = blockIdx.x * D + dec;
@@ -2028,10 +1857,10 @@ __global__ void __launch_bounds__(32 * D, M) serve_kernel(DecoderArgs a, ServeAr
         DecoderArgs ad = a;
         ad.P = s.deep_P;
         ad.C = s.deep_C;
-        decoder1_body<SupT, 2>(ad, s.deep_scratch + (size_t)gdec * s.deep_bytes, gdec, s);
+        decoder1_body<2>(ad, s.deep_scratch + (size_t)gdec * s.deep_bytes, gdec, s);
     } else {
-        const Dec1Layout lay = dec1_layout(a.P, a.C, a.Hz, (int)sizeof(SupT));
-        decoder1_body<SupT, 1>(a, smem_raw + (size_t)dec * lay.bytes, gdec, s);
+        const Dec1Layout lay = dec1_layout(a.P, a.C, a.Hz);
+        decoder1_body<1>(a, smem_raw + (size_t)dec * lay.bytes, gdec, s);
     }
 }
 
@@ -2039,29 +1868,29 @@ __global__ void __launch_bounds__(32 * D, M) serve_kernel(DecoderArgs a, ServeAr
 using ServeFn = void (*)(DecoderArgs, ServeArgs);
 #define PLP_SERVE_CONFIGS(X) X(1, 1) X(1, 12)
 
-static ServeFn serve_fn(int D, int M, int sup16) {
+static ServeFn serve_fn(int D, int M) {
 #define PLP_PICK_SERVE(d, m) \
-    if (D == d && M == m) return sup16 ? serve_kernel<d, m, 1> : serve_kernel<d, m, 0>;
+    if (D == d && M == m) return serve_kernel<d, m>;
     PLP_SERVE_CONFIGS(PLP_PICK_SERVE)
 #undef PLP_PICK_SERVE
     return nullptr;
 }
 
-bool serve_config_supported(int D, int M) { return serve_fn(D, M, 0) != nullptr; }
+bool serve_config_supported(int D, int M) { return serve_fn(D, M) != nullptr; }
 
-cudaError_t serve_occupancy(int P, int C, int Hz, int D, int M, int sup16, int* ctas_per_sm) {
-    ServeFn fn = serve_fn(D, M, sup16);
+cudaError_t serve_occupancy(int P, int C, int Hz, int D, int M, int* ctas_per_sm) {
+    ServeFn fn = serve_fn(D, M);
     if (!fn) return cudaErrorInvalidConfiguration;
-    const int smem = decoder_smem_bytes(P, C, Hz, 1, sup16) * D;
+    const int smem = decoder_smem_bytes(P, C, Hz, 1) * D;
     cudaError_t e = ensure_dyn_smem(reinterpret_cast<const void*>(fn), smem);
     if (e != cudaSuccess) return e;
     return cached_occupancy(reinterpret_cast<const void*>(fn), 32 * D, smem, ctas_per_sm);
 }
 
 cudaError_t launch_serve(const DecodeLaunch& L, const ServeArgs& s, cudaStream_t st) {
-    ServeFn fn = serve_fn(L.decoders_per_cta, L.min_blocks, L.sup16);
+    ServeFn fn = serve_fn(L.decoders_per_cta, L.min_blocks);
     if (!fn || L.warps_per_decoder != 1 || L.engine != 0) return cudaErrorInvalidConfiguration;
-    const int smem = decoder_smem_bytes(L.P, L.C, L.Hz, 1, L.sup16) * L.decoders_per_cta;
+    const int smem = decoder_smem_bytes(L.P, L.C, L.Hz, 1) * L.decoders_per_cta;
     cudaError_t e = ensure_dyn_smem(reinterpret_cast<const void*>(fn), smem);
     if (e != cudaSuccess) return e;
     e = cudaMemsetAsync(L.abort, 0, sizeof(int), st);

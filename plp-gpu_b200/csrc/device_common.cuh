@@ -67,10 +67,14 @@ __device__ __forceinline__ long long global_ns() {
 
 // Orientation table entry of one box type: up to 6 (w, d, h), dedup'd in the
 // reference's parser order (gpu/plp_common.hpp:269-280); unused slots are 0.
+// el, ew, eh are the type's three edges (held below 2^17: an edge of 65536 or
+// more fits no container) and el's bits 20-25 say which of the six slots
+//   0 (w, h, l)  1 (h, w, l)  2 (l, h, w)  3 (h, l, w)  4 (l, w, h)  5 (w, l, h)
+// are in the list: slot s is entry popc(slots below s).
 struct TypeOrs {
     int n;
     int w[6], d[6], h[6];
-    int pad[3];
+    int el, ew, eh;
 };
 static_assert(sizeof(TypeOrs) == 88, "TypeOrs layout");
 

@@ -25,7 +25,6 @@ struct DecodeLaunch {
     int P, C;                 // shared-memory tile: boxes and live points per decoder
     int Hz;                   // entries of the top-z index (max height + 2), 0 = none
     int engine;               // 0 extreme-point decoder, 1 block-building engine
-    int sup16;                // decoder: contact areas stored as 16-bit
     const BlkShape* bcat;     // block engine: shape catalogue of the batch
     const int* btab;          // block engine: per-instance orderings (ints)
     int N, T;                 // block engine tile: items, types per decoder
@@ -42,9 +41,9 @@ struct DecodeLaunch {
 // seeded MT states of seeds lo .. lo + n - 1, 624 words each
 cudaError_t launch_seed_table(long long lo, int n, const uint32_t* mt_init, uint32_t* out, cudaStream_t st);
 
-int decoder_smem_bytes(int P, int C, int Hz, int G, int sup16 = 0);   // sup16: 16-bit contact areas
+int decoder_smem_bytes(int P, int C, int Hz, int G);
 bool decoder_config_supported(int G, int D, int M);
-cudaError_t decoder_occupancy(int P, int C, int Hz, int G, int D, int M, int* ctas_per_sm, int sup16 = 0);
+cudaError_t decoder_occupancy(int P, int C, int Hz, int G, int D, int M, int* ctas_per_sm);
 cudaError_t launch_decoder(const DecodeLaunch& L, cudaStream_t st);     // configure + enqueue
 cudaError_t configure_decoder(const DecodeLaunch& L);                    // function attributes
 cudaError_t enqueue_decoder(const DecodeLaunch& L, cudaStream_t st);     // stream operations only
@@ -98,7 +97,7 @@ struct ServeArgs {
     int deep_idle_polls;            // empty polls before an overflow decoder exits
 };
 bool serve_config_supported(int D, int M);
-cudaError_t serve_occupancy(int P, int C, int Hz, int D, int M, int sup16, int* ctas_per_sm);
+cudaError_t serve_occupancy(int P, int C, int Hz, int D, int M, int* ctas_per_sm);
 cudaError_t launch_serve(const DecodeLaunch& L, const ServeArgs& s, cudaStream_t st);
 
 cudaError_t launch_redo_collect(const int2* work, int n_work, const InstDesc* inst, const SlotHead* heads,
