@@ -350,18 +350,21 @@ std::vector<TypeOrs> type_orientations(const Instance& I) {
     return ot;
 }
 
-// Smallest edge per axis over the types' orientations (1 where there is none).
-void min_edges(const std::vector<TypeOrs>& ors, InstDesc& d) {
-    int m[3] = {INT_MAX, INT_MAX, INT_MAX};
+// Smallest and largest edge per axis over the types' orientations (1 where
+// there is none).
+void edge_range(const std::vector<TypeOrs>& ors, InstDesc& d) {
+    bool any = false;
+    d.mw = d.md = d.mh = d.xw = d.xd = d.xh = 1;
     for (const TypeOrs& t : ors)
         for (int k = 0; k < t.n; k++) {
-            m[0] = std::min(m[0], t.w[k]);
-            m[1] = std::min(m[1], t.d[k]);
-            m[2] = std::min(m[2], t.h[k]);
+            d.mw = any ? std::min(d.mw, t.w[k]) : t.w[k];
+            d.md = any ? std::min(d.md, t.d[k]) : t.d[k];
+            d.mh = any ? std::min(d.mh, t.h[k]) : t.h[k];
+            d.xw = std::max(d.xw, t.w[k]);
+            d.xd = std::max(d.xd, t.d[k]);
+            d.xh = std::max(d.xh, t.h[k]);
+            any = true;
         }
-    d.mw = m[0] == INT_MAX ? 1 : m[0];
-    d.md = m[1] == INT_MAX ? 1 : m[1];
-    d.mh = m[2] == INT_MAX ? 1 : m[2];
 }
 
 struct Batch {
@@ -509,7 +512,7 @@ struct Batch {
             steps.insert(steps.end(), seq.begin(), seq.end());
             std::vector<TypeOrs> ot = ors.empty() ? type_orientations(I) : std::move(ors[i]);
             types.insert(types.end(), ot.begin(), ot.end());
-            min_edges(ot, desc.back());
+            edge_range(ot, desc.back());
             desc.back().engine = o.engine;
             desc.back().n_types = (int)I.types.size();
             max_types = std::max(max_types, (int)I.types.size());

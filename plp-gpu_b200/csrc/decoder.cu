@@ -783,10 +783,14 @@ __global__ void __launch_bounds__(32 * G * D, M) decoder_kernel(DecoderArgs a) {
 //    points never hold a feasible pair, and dropping them changes no pick and
 //    no draw. (With unit edges this is the plain "covered by a box" rule.)
 //  * C2 and most of C1: an orientation with an edge longer than the extent
-//    along it leaves the container or meets the box the extent ends at. What
-//    the extents let through (97 % of it passes C1 on the batched workload) is
-//    tested for support (C3), and only then against every box above the
-//    point's z (C1), one point at a time with the lanes over the boxes.
+//    along it leaves the container or meets the box the extent ends at.
+//    Extents are cut at the instance's largest edges (InstDesc), which no
+//    orientation exceeds. A point whose ex x ey x ez cuboid meets no box is
+//    clear: whatever its extents let through passes C1. 97 % of the points are
+//    clear when they appear, and a placed box that meets the cuboid of a clear
+//    point marks it (bit 16 of the z extent). Only marked points are tested
+//    against the boxes above their z (C1), after the support test (C3), one
+//    point at a time with the lanes over the boxes.
 //  * Same type again: points before the last step's first feasible point v
 //    held no feasible pair for the type, and still hold none: boxes only add
 //    to C1 and C2, and the placed box sits at or after v in (z, y, x) order, so
@@ -827,6 +831,7 @@ __device__ __forceinline__ unsigned support_slots(unsigned cand, int x, int y, i
                                                   const int4* bx) {
     unsigned a0 = 0, a1 = 0, a2 = 0, a3 = 0, a4 = 0, a5 = 0;
     const int xl = x + E.l, xw = x + E.w, xh = x + E.h, yl = y + E.l, yw = y + E.w, yh = y + E.h;
+#pragma unroll 1
     for (; j < je; j++) {
         const int4 b = bx[j];
         const int nx = -max(x, b.x), ny = -max(y, b.y);
@@ -855,6 +860,7 @@ __device__ __forceinline__ unsigned support_slots(unsigned cand, int x, int y, i
 __device__ __forceinline__ unsigned blocked_slots(int x, int y, int z, int j0, int nb, const Edges& E, const int4* bx,
                                                   const int* bzs, int lane) {
     unsigned blk = 0;
+#pragma unroll 1
     for (int jb = j0; jb < nb; jb += 32) {
         const int j = jb + lane;
         if (j < nb) {
@@ -867,11 +873,36 @@ __device__ __forceinline__ unsigned blocked_slots(int x, int y, int z, int j0, i
     return __reduce_or_sync(FULL, blk & 0x3fu);
 }
 
-// Smallest edges over the instance's orientations (InstDesc::mw, md, mh) and
+// Smallest and largest edges over the instance's orientations (InstDesc) and
 // the container.
-struct MinEdges {
-    int w, d, h;
+struct EdgeRange {
+    int w, d, h;      // smallest along x, y, z
+    int Mw, Md, Mh;   // largest
     int L, W, H;
+};
+
+constexpr uint32_t PT_MARKED = 1u << 16;   // z extent word: a box meets the extents' cuboid
+
+// A new box's corner coordinates (px .. px2 and so on) and the far ends of the
+// smallest-edge cuboid at them. Sets of corners are eight-bit masks over
+// c = (z2 << 2) | (y2 << 1) | x2.
+struct CornerFrame {
+    int x, y, z, x2, y2, z2;
+    int xm, ym, zm, x2m, y2m, z2m;
+    // How a placed box lies to the corners, a byte each from the low end: the
+    // corners whose x extent it ends, whose y extent, whose z extent, and
+    // those it reaches past on every axis. Corners whose cuboid it meets are
+    // added to dead.
+    __device__ __forceinline__ uint32_t relate(const int4& b, int bz, int bt, unsigned& dead) const {
+        const bool ax = x < b.z, ax2 = x2 < b.z, ay = y < b.w, ay2 = y2 < b.w, az = z < bt, az2 = z2 < bt;
+        const unsigned xa = (ax ? 0x55u : 0u) | (ax2 ? 0xaau : 0u), ya = (ay ? 0x33u : 0u) | (ay2 ? 0xccu : 0u),
+                       za = (az ? 0x0fu : 0u) | (az2 ? 0xf0u : 0u);
+        const unsigned xi = xa & ((b.x < xm ? 0x55u : 0u) | (b.x < x2m ? 0xaau : 0u)),
+                       yi = ya & ((b.y < ym ? 0x33u : 0u) | (b.y < y2m ? 0xccu : 0u)),
+                       zi = za & ((bz < zm ? 0x0fu : 0u) | (bz < z2m ? 0xf0u : 0u));
+        dead |= xi & yi & zi;
+        return (xa & yi & zi) | (xi & ya & zi) << 8 | (xi & yi & za) << 16 | (xa & ya & za) << 24;
+    }
 };
 
 // Warp: places a w x d x h box at the point with key pkey: top-sorted box
@@ -882,45 +913,57 @@ struct MinEdges {
 __device__ __forceinline__ int place1(uint32_t pkey, int pw, int pd, int ph, int& resume, const uint32_t* K,
                                       uint32_t* K2, int cap, int4* bx, int* bzs, int* z2s, unsigned short* bis,
                                       unsigned short* zt, int Hz, int& nc, int& nb, int P, int C, uint32_t xmask,
-                                      uint32_t ymask, int xb, int xyb, const MinEdges& ME, int lane) {
+                                      uint32_t ymask, int xb, int xyb, const EdgeRange& ME, int lane) {
     const int px = (int)(pkey & xmask), py = (int)((pkey >> xb) & ymask), pz = (int)(pkey >> xyb);
     const int px2 = px + pw, py2 = py + pd, pz2 = pz + ph;
     if (nb >= P) return ERR_BOX_CAP;
-    // Box tables, one pass from the top: the corners of the new box that a
-    // placed box makes dead, and the boxes whose top is above the new box's
-    // move up one slot (each round reads before it writes, and writes only
-    // slots it or an earlier round has read).
-    const int pxm = px + ME.w, px2m = px2 + ME.w, pym = py + ME.d, py2m = py2 + ME.d, pzm = pz + ME.h,
-              pz2m = pz2 + ME.h;
+    // Box tables, one pass from the top: how each placed box lies to the new
+    // box's corners, and the boxes whose top is above the new box's move up
+    // one slot (each round reads before it writes, and writes only slots it or
+    // an earlier round has read). The two top rounds stay in registers for the
+    // corners' extents.
+    const CornerFrame F{px, py, pz, px2, py2, pz2, px + ME.w, py + ME.d, pz + ME.h, px2 + ME.w, py2 + ME.d, pz2 + ME.h};
     unsigned dead = 1u;   // corner 0 = (px, py, pz): inside the new box
-    if (px2m > ME.L) dead |= 0xaau;
-    if (py2m > ME.W) dead |= 0xccu;
-    if (pz2m > ME.H) dead |= 0xf0u;
+    if (F.x2m > ME.L) dead |= 0xaau;
+    if (F.y2m > ME.W) dead |= 0xccu;
+    if (F.z2m > ME.H) dead |= 0xf0u;
     int nabove = 0;
-    for (int hi = nb; hi > 0; hi -= 32) {
-        const int jj = hi - 1 - lane;
-        const bool in = jj >= 0;
-        int4 b = make_int4(0, 0, 0, 0);
-        int bzb = 0, bzt = 0;
-        unsigned short bi = 0;
-        if (in) {
-            b = bx[jj];
-            bzb = bzs[jj];
-            bzt = z2s[jj];
-            bi = bis[jj];
-            const unsigned xin = (b.x < pxm && px < b.z ? 0x55u : 0u) | (b.x < px2m && px2 < b.z ? 0xaau : 0u);
-            const unsigned yin = (b.y < pym && py < b.w ? 0x33u : 0u) | (b.y < py2m && py2 < b.w ? 0xccu : 0u);
-            const unsigned zin = (bzb < pzm && pz < bzt ? 0x0fu : 0u) | (bzb < pz2m && pz2 < bzt ? 0xf0u : 0u);
-            dead |= xin & yin & zin;
-        }
-        const bool up = in && bzt > pz2;
-        nabove += __popc(__ballot_sync(FULL, up));
-        __syncwarp();
-        if (up) {
-            bx[jj + 1] = b;
-            bzs[jj + 1] = bzb;
-            z2s[jj + 1] = bzt;
-            bis[jj + 1] = bi;
+    const int nb0 = nb;
+    int4 wb[2];
+    int wz[2];
+    uint32_t wm[2] = {0u, 0u};
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+        // rounds 0 and 1 keep their box; round 2 stands for all below them
+#pragma unroll 1
+        for (int hi = nb0 - 32 * r; hi > 0; hi -= 32) {
+            const int jj = hi - 1 - lane;
+            const bool in = jj >= 0;
+            int4 b = make_int4(0, 0, 0, 0);
+            int bzb = 0, bzt = 0;
+            unsigned short bi = 0;
+            if (in) {
+                b = bx[jj];
+                bzb = bzs[jj];
+                bzt = z2s[jj];
+                bi = bis[jj];
+            }
+            const uint32_t m = F.relate(b, bzb, bzt, dead);
+            const bool up = in && bzt > pz2;
+            nabove += __popc(__ballot_sync(FULL, up));
+            __syncwarp();
+            if (up) {
+                bx[jj + 1] = b;
+                bzs[jj + 1] = bzb;
+                z2s[jj + 1] = bzt;
+                bis[jj + 1] = bi;
+            }
+            if (r < 2) {
+                wb[r] = b;
+                wz[r] = bzb;
+                wm[r] = m;
+                break;
+            }
         }
     }
     unsigned live = ~__reduce_or_sync(FULL, dead) & 0xffu;
@@ -934,8 +977,21 @@ __device__ __forceinline__ int place1(uint32_t pkey, int pw, int pd, int ph, int
             bis[ip] = (unsigned short)nb;
         }
     }
-    if (zt)
-        for (int zz = pz2 + 1 + lane; zz < Hz; zz += 32) zt[zz]++;
+    if (zt) {
+        // entries above the new top, two to a word (counts stay below 2^16), four words a lane in flight
+        const int z0 = pz2 + 1;
+        if ((z0 & 1) && lane == 0) zt[z0]++;
+        uint32_t* zw = reinterpret_cast<uint32_t*>(zt);
+#pragma unroll 1
+        for (int w = ((z0 + 1) >> 1) + lane; w < Hz >> 1; w += 128) {
+            uint32_t v[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) v[u] = w + 32 * u < Hz >> 1 ? zw[w + 32 * u] : 0u;
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (w + 32 * u < Hz >> 1) zw[w + 32 * u] = v[u] + 0x10001u;
+        }
+    }
     nb++;
     // Points: one pass from K to K2. Corners in index order
     // c = (cz << 2) | (cy << 1) | cx are in key order; lane c counts the
@@ -944,26 +1000,31 @@ __device__ __forceinline__ int place1(uint32_t pkey, int pw, int pd, int ph, int
     const uint32_t ck = ((uint32_t)((lane & 4) ? pz2 : pz) << xyb) | ((uint32_t)((lane & 2) ? py2 : py) << xb) |
                         (uint32_t)((lane & 1) ? px2 : px);
     int ns = 0, rank = 0, at = 0;
+#pragma unroll 1
     for (int cb = 0; cb < nc; cb += 32) {
         const int i = cb + lane;
         bool keep = false;
         uint32_t key = 0;
         int ex = 0, ey = 0, ez = 0;
+        uint32_t mark = 0;
         if (i < nc) {
             key = K[i];
-            const uint32_t exy = K[cap + i];
+            const uint32_t exy = K[cap + i], ezm = K[2 * cap + i];
             ex = (int)(exy & 0xffffu);
             ey = (int)(exy >> 16);
-            ez = (int)K[2 * cap + i];
+            ez = (int)(ezm & 0xffffu);
+            mark = ezm & PT_MARKED;
             const int x = (int)(key & xmask), y = (int)((key >> xb) & ymask), z = (int)(key >> xyb);
             const bool ix = px < x + ME.w && x < px2, iy = py < y + ME.d && y < py2, iz = pz < z + ME.h && z < pz2;
             if (iy && iz && x < px2) ex = min(ex, px - x);
             if (ix && iz && y < py2) ey = min(ey, py - y);
             if (ix && iy && z < pz2) ez = min(ez, pz - z);
             keep = ex >= ME.w && ey >= ME.d && ez >= ME.h;
+            if (px < x + ex && x < px2 && py < y + ey && y < py2 && pz < z + ez && z < pz2) mark = PT_MARKED;
         }
         const unsigned bal = __ballot_sync(FULL, keep);
         int off = 0;
+#pragma unroll 1
         for (unsigned m = live; m; m &= m - 1) {
             const int c = __ffs(m) - 1;
             const uint32_t kc = __shfl_sync(FULL, ck, c);
@@ -980,7 +1041,7 @@ __device__ __forceinline__ int place1(uint32_t pkey, int pw, int pd, int ph, int
             const int d = ns + __popc(bal & lanemask_lt()) + off;
             K2[d] = key;
             K2[cap + d] = (uint32_t)ex | ((uint32_t)ey << 16);
-            K2[2 * cap + d] = (uint32_t)ez;
+            K2[2 * cap + d] = (uint32_t)ez | mark;
         }
         ns += __popc(bal);
     }
@@ -988,31 +1049,53 @@ __device__ __forceinline__ int place1(uint32_t pkey, int pw, int pd, int ph, int
     nc = ns + __popc(live);
     if (nc > C) return ERR_CAND_CAP;
     __syncwarp();   // box tables and top-z index are final
-    // extents of the new corners: lanes over the boxes above the corner's z
+    // Extents of the new corners: the boxes in registers, then any below them
+    // from the tables (their old slots [0, nb0 - 64) now lie within
+    // [0, nb0 - 64]; a box met twice, or the new one, changes nothing).
     int nth = 0;
-    for (unsigned m = live; m; m &= m - 1) {
-        const int c = __ffs(m) - 1;
+#pragma unroll 1
+    for (unsigned mc = live; mc; mc &= mc - 1) {
+        const int c = __ffs(mc) - 1;
         const int x = (c & 1) ? px2 : px, y = (c & 2) ? py2 : py, z = (c & 4) ? pz2 : pz;
-        int ex = ME.L - x, ey = ME.W - y, ez = ME.H - z;
-        for (int jb = box_start(zt, z2s, nb, z + 1); jb < nb; jb += 32) {
-            const int j = jb + lane;
-            if (j < nb) {
-                const int4 b = bx[j];
-                const int bz = bzs[j];
-                const bool ix = b.x < x + ME.w && x < b.z, iy = b.y < y + ME.d && y < b.w, iz = bz < z + ME.h;
-                if (iy && iz && x < b.z) ex = min(ex, b.x - x);
-                if (ix && iz && y < b.w) ey = min(ey, b.y - y);
-                if (ix && iy) ez = min(ez, bz - z);
+        int ex = min(ME.L - x, ME.Mw), ey = min(ME.W - y, ME.Md), ez = min(ME.H - z, ME.Mh);
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            if (32 * r < nb0) {
+                const uint32_t m = wm[r] >> c;
+                if (m & 1u) ex = min(ex, wb[r].x - x);
+                if (m & 0x100u) ey = min(ey, wb[r].y - y);
+                if (m & 0x10000u) ez = min(ez, wz[r] - z);
             }
+        }
+        const int j0 = nb0 > 64 ? box_start(zt, z2s, nb, z + 1) : nb;
+#pragma unroll 1
+        for (int j = j0 + lane; j <= nb0 - 64; j += 32) {
+            const int4 b = bx[j];
+            const int bz = bzs[j];
+            const bool ix = b.x < x + ME.w && x < b.z, iy = b.y < y + ME.d && y < b.w, iz = bz < z + ME.h;
+            if (iy && iz && x < b.z) ex = min(ex, b.x - x);
+            if (ix && iz && y < b.w) ey = min(ey, b.y - y);
+            if (ix && iy) ez = min(ez, bz - z);
         }
         ex = __reduce_min_sync(FULL, ex);
         ey = __reduce_min_sync(FULL, ey);
         ez = __reduce_min_sync(FULL, ez);
+        bool meets = false;
+#pragma unroll
+        for (int r = 0; r < 2; r++)
+            if (32 * r < nb0)
+                meets = meets || (((wm[r] >> c) & 0x1000000u) && wb[r].x < x + ex && wb[r].y < y + ey && wz[r] < z + ez);
+#pragma unroll 1
+        for (int j = j0 + lane; j <= nb0 - 64; j += 32) {
+            const int4 b = bx[j];
+            meets = meets || (b.x < x + ex && x < b.z && b.y < y + ey && y < b.w && bzs[j] < z + ez);
+        }
+        const uint32_t mark = __any_sync(FULL, meets) ? PT_MARKED : 0u;
         if (lane == c) {
             const int d = rank + nth;
             K2[d] = ck;
             K2[cap + d] = (uint32_t)ex | ((uint32_t)ey << 16);
-            K2[2 * cap + d] = (uint32_t)ez;
+            K2[2 * cap + d] = (uint32_t)ez | mark;
         }
         nth++;
     }
@@ -1205,6 +1288,7 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
 
     constexpr bool SERVE = MODE != 0;
     const int n_work = SERVE ? 0 : (a.n_work_dev ? *a.n_work_dev : a.n_work);
+#pragma unroll 1
     for (;;) {
         if (*reinterpret_cast<volatile int*>(a.abort)) break;
         int2 wk;
@@ -1255,6 +1339,7 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
                 // the seeded state, computed once for every restart of the batch with this seed
                 const uint4* src = reinterpret_cast<const uint4*>(a.seed_tab + (sd - a.seed_lo) * 624);
                 uint4* dst = reinterpret_cast<uint4*>(mt);
+#pragma unroll 1
                 for (int i = lane; i < 156; i += 32) dst[i] = __ldg(src + i);
                 __syncwarp();
             } else {
@@ -1269,64 +1354,87 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
         int best_n = 0;
         double best_score = 0.0;
 
+#pragma unroll 1
         for (int pass = 0; pass < I.passes && err == ERR_NONE; pass++) {
             int nb = 0, nc = 1, cur = 0;
             long long vol = 0;
             if (zt)
+#pragma unroll 1
                 for (int i = lane; i < a.Hz; i += 32) zt[i] = 0;
             if (lane == 0) {
                 pts[0] = 0u;
-                pts[lay.cap] = (uint32_t)L | ((uint32_t)W << 16);
-                pts[2 * lay.cap] = (uint32_t)H;
+                pts[lay.cap] = (uint32_t)min(L, I.xw) | ((uint32_t)min(W, I.xd) << 16);
+                pts[2 * lay.cap] = (uint32_t)min(H, I.xh);
             }
             __syncwarp();
             int state_type = -1;
             int resume = 0;         // points before it hold no feasible pair of state_type
             bool stuck = false;     // the last step of state_type found no feasible pair
-            int t_next = I.n_steps > 0 ? ld_table<SERVE>(a.step_type + I.step_off) : 0;
-            for (int sti = 0; sti < I.n_steps; sti++) {
+            const EdgeRange ER{I.mw, I.md, I.mh, I.xw, I.xd, I.xh, L, W, H};
+            // a step's type and its edges are fetched one step ahead
+            const int* steps = a.step_type + I.step_off;
+            const TypeOrs* tors = a.types + I.type_off;
+            int t_next = -1, el_next = 0, ew_next = 0, eh_next = 0;
+            Edges E{0, 0, 0};
+            unsigned slots = 0;
+#pragma unroll 1
+            for (int sti = -1; sti < I.n_steps; sti++) {
                 const int t = t_next;
-                if (sti + 1 < I.n_steps) t_next = ld_table<SERVE>(a.step_type + I.step_off + sti + 1);
+                const bool fresh = t != state_type;
+                if (fresh) {
+                    E = Edges{el_next & 0x1ffff, ew_next, eh_next};
+                    slots = (unsigned)el_next >> 20;
+                }
+                if (sti + 1 < I.n_steps) {
+                    t_next = ld_table<SERVE>(steps + sti + 1);
+                    if (t_next != t) {
+                        el_next = ld_table<SERVE>(&tors[t_next].el);
+                        ew_next = ld_table<SERVE>(&tors[t_next].ew);
+                        eh_next = ld_table<SERVE>(&tors[t_next].eh);
+                    }
+                }
                 // With no box placed since, another item of that type meets the
                 // same points and finds no pair either; it draws no random
                 // number, so the step is skipped without changing the result.
-                if (stuck && t == state_type) continue;
-                const TypeOrs& T = a.types[I.type_off + t];
-                const int el = ld_table<SERVE>(&T.el);
-                const Edges E{el & 0x1ffff, ld_table<SERVE>(&T.ew), ld_table<SERVE>(&T.eh)};
-                const unsigned slots = (unsigned)el >> 20;
-                if (slots == 0) continue;
-                const int from = t == state_type ? resume : 0;
+                if (stuck && !fresh) continue;
+                const int from = fresh ? 0 : resume;
                 state_type = t;
+                if (slots == 0) {   // no orientation at all (or the fetch of the first step)
+                    stuck = true;
+                    continue;
+                }
                 const uint32_t* K = pts + cur * 3 * lay.cap;
                 uint32_t* K2 = pts + (cur ^ 1) * 3 * lay.cap;
                 // items: the points whose extents let an orientation through,
-                // {key, slots | point index << 8}
+                // {key, slots | marked << 7 | point index << 8}
                 uint2* Wl = reinterpret_cast<uint2*>(K2);
                 int nW = 0;
+#pragma unroll 1
                 for (int cb = from; cb < nc; cb += 32) {
                     const int i = cb + lane;
                     unsigned m = 0;
                     uint32_t key = 0;
                     if (i < nc) {
                         key = K[i];
-                        const uint32_t exy = K[lay.cap + i];
+                        const uint32_t exy = K[lay.cap + i], ezm = K[2 * lay.cap + i];
                         m = slots & x_within(E, (int)(exy & 0xffffu)) & y_within(E, (int)(exy >> 16)) &
-                            z_within(E, (int)K[2 * lay.cap + i]);
+                            z_within(E, (int)(ezm & 0xffffu));
+                        if (m) m |= (ezm & PT_MARKED) >> 9 | (unsigned)i << 8;
                     }
                     const unsigned bal = __ballot_sync(FULL, m != 0);
-                    if (m) Wl[nW + __popc(bal & lanemask_lt())] = make_uint2(key, m | ((unsigned)i << 8));
+                    if (m) Wl[nW + __popc(bal & lanemask_lt())] = make_uint2(key, m);
                     nW += __popc(bal);
                 }
                 __syncwarp();
-                // C3 for 32 items at a time, then C1 item by item in order. The
-                // first item with a feasible pair decides the branch; the random
-                // branch goes on to the end and keeps every item's feasible set.
+                // C3 for 32 items at a time, then C1 of the marked ones. The first
+                // item with a feasible pair decides the branch; the random branch
+                // goes on to the end and keeps every item's feasible set.
                 int first = -1, pick_p = 0;      // item and point of the first feasible pair
                 unsigned pick_m = 0;             // its feasible set
                 uint32_t pick_key = 0;
                 int count = 0;
                 bool full = false;
+#pragma unroll 1
                 for (int w0 = 0; w0 < nW; w0 += 32) {
                     const uint2 e = w0 + lane < nW ? Wl[w0 + lane] : make_uint2(0, 0);
                     unsigned cand = e.y & 0x3fu;
@@ -1336,15 +1444,19 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
                         cand = support_slots(cand, (int)(e.x & xmask), (int)((e.x >> xb) & ymask), j, je, E, bx);
                     }
                     __syncwarp();
-                    unsigned mine = 0;
-                    for (unsigned bal = __ballot_sync(FULL, cand != 0); bal; bal &= bal - 1) {
+                    const unsigned marked = __ballot_sync(FULL, cand && (e.y & 0x80u));
+                    // items in order up to the first feasible one, then the marked ones
+#pragma unroll 1
+                    for (unsigned bal = first < 0 ? __ballot_sync(FULL, cand != 0) : marked; bal; bal &= bal - 1) {
                         const int q = __ffs(bal) - 1;
                         const uint32_t kq = __shfl_sync(FULL, e.x, q);
-                        const int zq = (int)(kq >> xyb);
-                        const unsigned ok = __shfl_sync(FULL, cand, q) &
-                                            ~blocked_slots((int)(kq & xmask), (int)((kq >> xb) & ymask), zq,
-                                                           box_start(zt, z2s, nb, zq + 1), nb, E, bx, bzs, lane);
-                        if (lane == q) mine = ok;
+                        unsigned ok = __shfl_sync(FULL, cand, q);
+                        if ((marked >> q) & 1u) {
+                            const int zq = (int)(kq >> xyb);
+                            ok &= ~blocked_slots((int)(kq & xmask), (int)((kq >> xb) & ymask), zq,
+                                                 box_start(zt, z2s, nb, zq + 1), nb, E, bx, bzs, lane);
+                            if (lane == q) cand = ok;
+                        }
                         if (ok && first < 0) {
                             first = w0 + q;
                             pick_key = kq;
@@ -1353,12 +1465,13 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
                             // random() only once a feasible pair exists
                             full = randomized && mt_random(mt, mpos, lane) >= 1.0 - I.eps;
                             if (!full) break;
+                            bal &= marked | (1u << q);
                         }
                     }
                     if (first >= 0) {
                         if (!full) break;
-                        count += __popc(mine);
-                        if (w0 + lane < nW) Wl[w0 + lane].y = mine;
+                        count += __popc(cand);
+                        if (w0 + lane < nW) Wl[w0 + lane].y = cand;
                     }
                 }
                 stuck = first < 0;
@@ -1373,6 +1486,7 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
                     __syncwarp();
                     // idx-th feasible pair in (point, orientation) order
                     int run = 0;
+#pragma unroll 1
                     for (int w0 = first & ~31; w0 < nW; w0 += 32) {
                         const uint2 e = w0 + lane < nW ? Wl[w0 + lane] : make_uint2(0, 0);
                         const int c = __popc(e.y);
@@ -1385,6 +1499,7 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
                         if (idx < run + tot) {
                             const int q = __ffs(__ballot_sync(FULL, idx < run + excl + c)) - 1;
                             unsigned m = __shfl_sync(FULL, e.y, q);
+#pragma unroll 1
                             for (int k = idx - run - __shfl_sync(FULL, excl, q); k > 0; k--) m &= m - 1;
                             pick_key = __shfl_sync(FULL, e.x, q);
                             slot = __ffs(m) - 1;
@@ -1403,7 +1518,7 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
                 vol += 1LL * pw * pd * ph;
                 __syncwarp();   // every lane has read the item list before K2 is written
                 err = place1(pick_key, pw, pd, ph, resume, K, K2, lay.cap, bx, bzs, z2s, bis, zt, a.Hz, nc, nb, a.P,
-                             a.C, xmask, ymask, xb, xyb, MinEdges{I.mw, I.md, I.mh, L, W, H}, lane);
+                             a.C, xmask, ymask, xb, xyb, ER, lane);
                 if (err != ERR_NONE) break;
                 cur ^= 1;
             }
@@ -1419,6 +1534,7 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
                 best_n = nb;
                 best_score = score;
                 if (pass_out != best_out)
+#pragma unroll 1
                     for (int i = lane; i < nb; i += 32) best_out[i] = pass_out[i];
             }
             have_any = true;
@@ -1485,8 +1601,15 @@ static DecoderArgs decoder_args(const DecodeLaunch& L) {
 }
 
 #ifndef PLP_SERVE_TU
+// The M = 16 configuration is built for 18 resident decoders: the compiler
+// settles at 90 registers (112 for a bound of 16), and 18 decoders of 112
+// registers or fewer fit the register file as well as 16 do. 512 batched
+// instances x 128 restarts: 7.9 ms built for 16, 7.25 for 18, 8.3 for 20 (4 KB
+// more code, see below). Straight-line code is kept short throughout
+// (unroll 1): with the twist and the FSR unrolled, 68 KB instead of 44, the
+// same build took 8.0 ms and one 4 KB larger 12 ms, waiting for instructions.
 template <int D, int M>
-__global__ void __launch_bounds__(32 * D, M) decoder1_kernel(DecoderArgs a) {
+__global__ void __launch_bounds__(32 * D, M == 16 ? 18 : M) decoder1_kernel(DecoderArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int dec = threadIdx.x >> 5;
     const Dec1Layout lay = dec1_layout(a.P, a.C, a.Hz);

@@ -47,7 +47,8 @@ struct InstDesc {
     // smallest edge along x, y, z over every orientation of the instance's
     // types: a point whose mw x md x mh cuboid leaves the container or meets
     // a placed box cannot hold any item (the decoders drop it)
-    int mw, md, mh, pad;
+    int mw, md, mh;
+    int xw, xd, xh;      // largest edge along x, y, z
 };
 
 // Block shape of the block-building engine (blockproof/plp_block.cpp:29-37):
@@ -189,6 +190,7 @@ static __device__ __noinline__ void mt_seed_warp(uint32_t* mt, unsigned long lon
 // i >= 227. Chunks of 32 in increasing i therefore only read finished or
 // untouched words; inside a chunk all lanes read before any lane writes.
 static __device__ __noinline__ void mt_twist_warp(uint32_t* mt, int lane) {
+#pragma unroll 1
     for (int base = 0; base < 623; base += 32) {
         const int i = base + lane;
         uint32_t nv = 0;

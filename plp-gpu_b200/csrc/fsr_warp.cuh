@@ -31,14 +31,18 @@ static __device__ __noinline__ double fsr_score_warp(const int4* bx, const int* 
     while (npad < n) npad <<= 1;
     // sort keys: (0xffff - z) << 16 | idx  ->  ascending = z desc, idx asc.
     // npad may exceed n; the tail lives in the tot[] area, which is filled after.
+#pragma unroll 1
     for (int p = lane; p < npad; p += 32) {
         key[p] = p < n ? ((uint32_t)(0xffff - bz[p]) << 16) | bi[p] : 0xffffffffu;
         if (p < n) pos[bi[p]] = (unsigned short)p;
     }
     __syncwarp();
     // bitonic sort in shared memory (ascending)
+#pragma unroll 1
     for (int k = 2; k <= npad; k <<= 1) {
+#pragma unroll 1
         for (int j = k >> 1; j > 0; j >>= 1) {
+#pragma unroll 1
             for (int i = lane; i < npad; i += 32) {
                 const int l = i ^ j;
                 if (l > i) {
@@ -54,6 +58,7 @@ static __device__ __noinline__ double fsr_score_warp(const int4* bx, const int* 
         }
     }
     // masses and contact totals
+#pragma unroll 1
     for (int p = lane; p < n; p += 32) {
         const int4 b = bx[p];
         const int h = z2[p] - bz[p];
@@ -61,12 +66,14 @@ static __device__ __noinline__ double fsr_score_warp(const int4* bx, const int* 
         load[p] = 50.0 * (double)vol / 1e6;
     }
     __syncwarp();
+#pragma unroll 1
     for (int p = lane; p < n; p += 32) {
         const int4 b = bx[p];
         const int zb = bz[p];
         int t = 0;
         if (zb > 0) {
             const int j0 = zt ? (int)zt[zb] : lower_bound_top(z2, n, zb);
+#pragma unroll 1
             for (int j = j0; j < n && z2[j] == zb; j++) {
                 const int4 c = bx[j];
                 const int ox = min(b.z, c.z) - max(b.x, c.x);
@@ -80,10 +87,12 @@ static __device__ __noinline__ double fsr_score_warp(const int4* bx, const int* 
     __syncwarp();
     // propagate, level by level in (z desc, index asc) order
     int q = 0;
+#pragma unroll 1
     while (q < n) {
         const int k0 = pos[key[q] & 0xffff];
         const int zl = bz[k0];
         int qe = q;
+#pragma unroll 1
         while (qe < n && (int)(0xffff - (key[qe] >> 16)) == zl) qe++;
         if (zl > 0) {
             int jlo, jhi;
@@ -93,13 +102,16 @@ static __device__ __noinline__ double fsr_score_warp(const int4* bx, const int* 
             } else {
                 jlo = lower_bound_top(z2, n, zl);
                 jhi = jlo;
+#pragma unroll 1
                 while (jhi < n && z2[jhi] == zl) jhi++;
             }
+#pragma unroll 1
             for (int jb = jlo; jb < jhi; jb += 32) {
                 const int j = jb + lane;
                 if (j < jhi) {
                     const int4 c = bx[j];
                     double lj = load[j];
+#pragma unroll 1
                     for (int qq = q; qq < qe; qq++) {
                         const int k = pos[key[qq] & 0xffff];
                         const int total = tot[k];
@@ -119,6 +131,7 @@ static __device__ __noinline__ double fsr_score_warp(const int4* bx, const int* 
         q = qe;
     }
     int cnt = 0;
+#pragma unroll 1
     for (int p = lane; p < n; p += 32) {
         const int4 b = bx[p];
         const long long vol = 1LL * (b.z - b.x) * (b.w - b.y) * (z2[p] - bz[p]);
