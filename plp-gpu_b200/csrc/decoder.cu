@@ -111,14 +111,13 @@ __host__ __device__ inline DecLayout dec_layout(int P, int C, int Hz) {
     return l;
 }
 
-// Layout of one single-warp decoder: MT state, top-sorted boxes, and two
-// point buffers of {key, x extent | y extent << 16, z extent} (SoA). A
-// placement writes the updated points from one buffer to the other; between
-// placements the spare buffer holds the step's item list. Eight entries past
-// C take a placement's corners before the capacity check.
+// Layout of one single-warp decoder: MT state, top-sorted boxes, the points
+// {key, x extent | y extent << 16, z extent | mark} (SoA, in no order) and
+// the step's items. Eight slots past C take
+// a placement's corners before the capacity check.
 struct Dec1Layout {
-    int off_bx, off_bz, off_z2, off_bi, off_pts, off_zt, bytes;
-    int cap;   // entries per array of a point buffer
+    int off_bx, off_bz, off_z2, off_bi, off_pts, off_w, off_free, off_zt, bytes;
+    int cap;   // entries per array of the points
 };
 
 __host__ __device__ inline Dec1Layout dec1_layout(int P, int C, int Hz) {
@@ -132,10 +131,12 @@ __host__ __device__ inline Dec1Layout dec1_layout(int P, int C, int Hz) {
     o = (o + 15) & ~15;
     l.cap = C + 8;
     l.off_pts = o;
-    int region = 24 * l.cap;               // two buffers; FSR overlays 18 bytes per box
+    l.off_w = o + 12 * l.cap;
+    int region = 12 * l.cap + 8 * (C + 2);       // FSR overlays 18 bytes per box
     if (region < 18 * P + 32) region = 18 * P + 32;
     o += region;
     o = (o + 15) & ~15;
+    l.off_free = o;  o += 64;              // u16: slots a placement frees (the first 32)
     l.off_zt = o;  o += 2 * Hz;            // u16: boxes with top < z
     o = (o + 15) & ~15;
     l.bytes = o;
@@ -791,16 +792,26 @@ __global__ void __launch_bounds__(32 * G * D, M) decoder_kernel(DecoderArgs a) {
 //    point marks it (bit 16 of the z extent). Only marked points are tested
 //    against the boxes above their z (C1), after the support test (C3), one
 //    point at a time with the lanes over the boxes.
-//  * Same type again: points before the last step's first feasible point v
-//    held no feasible pair for the type, and still hold none: boxes only add
-//    to C1 and C2, and the placed box sits at or after v in (z, y, x) order, so
-//    its top is above every such point's z and supports none of them; its
-//    corners come after it. The scan resumes at v.
+//  * Same type again: points before (in key order) the last step's first
+//    feasible point v held no feasible pair for the type, and still hold none:
+//    boxes only add to C1 and C2, and the placed box sits at or after v in
+//    (z, y, x) order, so its top is above every such point's z and supports
+//    none of them; its corners come after it. They are left out by key.
+//
+// Points lie in no order: a new point takes a dead one's slot, and the last
+// point fills a slot left over, so at most a few points move. The order the reference's list has
+// enters only where a pair is picked: the first feasible point is a minimum
+// over the keys, and the idx-th pair counts the pairs at smaller keys.
 //
 // The work per step is integer tests on data in shared memory, so instructions
 // and their dependent chains bound it; extents replace per-type masks and six
 // contact areas per point that had to be evaluated against every box at each
-// change of type, kept up to date, and moved with the points.
+// change of type, kept up to date, and moved with the points. Measured, decoder
+// alone at 128 boxes, 160 points, M = 16: 512 batched instances x 128 restarts
+// 7.0 ms, 64 stress instances x 512 3.7 ms, 1024 restarts of one instance 0.306
+// ms, one greedy decode 0.148 ms (16.3, 11.3, 0.409 and 0.192 ms with masks and
+// areas; 24.5, 21.5, 0.554 and 0.226 ms with those and without the dead-point
+// rule; 7.25, 4.0, 0.325 and 0.169 ms with extents on points kept in order).
 //
 // The C3 test is the integer form of the reference's FP64 ratio:
 // (double)s / (double)(w*d) < 0.5  <=>  2 s < w d. Both s and w d are
@@ -831,22 +842,27 @@ __device__ __forceinline__ unsigned support_slots(unsigned cand, int x, int y, i
                                                   const int4* bx) {
     unsigned a0 = 0, a1 = 0, a2 = 0, a3 = 0, a4 = 0, a5 = 0;
     const int xl = x + E.l, xw = x + E.w, xh = x + E.h, yl = y + E.l, yw = y + E.w, yh = y + E.h;
+    // two boxes at a time; past the end an empty box, which adds nothing
 #pragma unroll 1
-    for (; j < je; j++) {
-        const int4 b = bx[j];
-        const int nx = -max(x, b.x), ny = -max(y, b.y);
-        const int tx = b.z + nx, ty = b.w + ny;
-        // overlap along an axis: max(0, min(x + e, b.x2) - max(x, b.x))
-        const unsigned ol = __viaddmin_s32_relu(xl, nx, tx), ow = __viaddmin_s32_relu(xw, nx, tx),
-                       oh = __viaddmin_s32_relu(xh, nx, tx);
-        const unsigned pl = __viaddmin_s32_relu(yl, ny, ty), pw = __viaddmin_s32_relu(yw, ny, ty),
-                       ph = __viaddmin_s32_relu(yh, ny, ty);
-        a0 += ow * ph;
-        a1 += oh * pw;
-        a2 += ol * ph;
-        a3 += oh * pl;
-        a4 += ol * pw;
-        a5 += ow * pl;
+    for (; j < je; j += 2) {
+        const int4 b0 = bx[j], b1 = j + 1 < je ? bx[j + 1] : make_int4(0, 0, 0, 0);
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int4 b = u ? b1 : b0;
+            const int nx = -max(x, b.x), ny = -max(y, b.y);
+            const int tx = b.z + nx, ty = b.w + ny;
+            // overlap along an axis: max(0, min(x + e, b.x2) - max(x, b.x))
+            const unsigned ol = __viaddmin_s32_relu(xl, nx, tx), ow = __viaddmin_s32_relu(xw, nx, tx),
+                           oh = __viaddmin_s32_relu(xh, nx, tx);
+            const unsigned pl = __viaddmin_s32_relu(yl, ny, ty), pw = __viaddmin_s32_relu(yw, ny, ty),
+                           ph = __viaddmin_s32_relu(yh, ny, ty);
+            a0 += ow * ph;
+            a1 += oh * pw;
+            a2 += ol * ph;
+            a3 += oh * pl;
+            a4 += ol * pw;
+            a5 += ow * pl;
+        }
     }
     // footprints of the slots in `cand` fit the container; others' bits are masked off
     const unsigned wh = (unsigned)E.w * E.h, lh = (unsigned)E.l * E.h, lw = (unsigned)E.l * E.w;
@@ -906,12 +922,11 @@ struct CornerFrame {
 };
 
 // Warp: places a w x d x h box at the point with key pkey: top-sorted box
-// tables, top-z index, then every point from buffer K to buffer K2 (arrays of
-// `cap` entries: key, x | y << 16 extents, z extent) with the box applied to
-// its extents, dead points left out and the box's live corners merged in.
-// resume: in, a point index; out, the survivors before it.
-__device__ __forceinline__ int place1(uint32_t pkey, int pw, int pd, int ph, int& resume, const uint32_t* K,
-                                      uint32_t* K2, int cap, int4* bx, int* bzs, int* z2s, unsigned short* bis,
+// tables, top-z index, and the points K (arrays of `cap` entries: key,
+// x | y << 16 extents, z extent | mark): the box is applied to every point,
+// dead ones give up their slots, and the box's live corners come in.
+__device__ __forceinline__ int place1(uint32_t pkey, int pw, int pd, int ph, uint32_t* K, int cap,
+                                      unsigned short* free_slots, int4* bx, int* bzs, int* z2s, unsigned short* bis,
                                       unsigned short* zt, int Hz, int& nc, int& nb, int P, int C, uint32_t xmask,
                                       uint32_t ymask, int xb, int xyb, const EdgeRange& ME, int lane) {
     const int px = (int)(pkey & xmask), py = (int)((pkey >> xb) & ymask), pz = (int)(pkey >> xyb);
@@ -993,66 +1008,61 @@ __device__ __forceinline__ int place1(uint32_t pkey, int pw, int pd, int ph, int
         }
     }
     nb++;
-    // Points: one pass from K to K2. Corners in index order
-    // c = (cz << 2) | (cy << 1) | cx are in key order; lane c counts the
-    // survivors below corner c, and a corner whose key a survivor has is not
-    // new. Keys ascend, so it is found before any point above it is written.
+    // Points in place. A corner whose key a point already has is not new.
     const uint32_t ck = ((uint32_t)((lane & 4) ? pz2 : pz) << xyb) | ((uint32_t)((lane & 2) ? py2 : py) << xb) |
                         (uint32_t)((lane & 1) ? px2 : px);
-    int ns = 0, rank = 0, at = 0;
+    int nf = 0;            // slots freed
+    unsigned dup = 0;      // corners this lane has met
 #pragma unroll 1
     for (int cb = 0; cb < nc; cb += 32) {
         const int i = cb + lane;
-        bool keep = false;
-        uint32_t key = 0;
-        int ex = 0, ey = 0, ez = 0;
-        uint32_t mark = 0;
-        if (i < nc) {
-            key = K[i];
-            const uint32_t exy = K[cap + i], ezm = K[2 * cap + i];
-            ex = (int)(exy & 0xffffu);
-            ey = (int)(exy >> 16);
-            ez = (int)(ezm & 0xffffu);
-            mark = ezm & PT_MARKED;
-            const int x = (int)(key & xmask), y = (int)((key >> xb) & ymask), z = (int)(key >> xyb);
-            const bool ix = px < x + ME.w && x < px2, iy = py < y + ME.d && y < py2, iz = pz < z + ME.h && z < pz2;
-            if (iy && iz && x < px2) ex = min(ex, px - x);
-            if (ix && iz && y < py2) ey = min(ey, py - y);
-            if (ix && iy && z < pz2) ez = min(ez, pz - z);
-            keep = ex >= ME.w && ey >= ME.d && ez >= ME.h;
-            if (px < x + ex && x < px2 && py < y + ey && y < py2 && pz < z + ez && z < pz2) mark = PT_MARKED;
+        const bool in = i < nc;
+        const uint32_t key = in ? K[i] : 0u, exy = in ? K[cap + i] : 0u, ezm = in ? K[2 * cap + i] : 0u;
+        int ex = (int)(exy & 0xffffu), ey = (int)(exy >> 16), ez = (int)(ezm & 0xffffu);
+        uint32_t mark = ezm & PT_MARKED;
+        const int x = (int)(key & xmask), y = (int)((key >> xb) & ymask), z = (int)(key >> xyb);
+        const bool ax = x < px2, ay = y < py2, az = z < pz2;
+        const bool ix = ax && px < x + ME.w, iy = ay && py < y + ME.d, iz = az && pz < z + ME.h;
+        if (iy && iz && ax) ex = min(ex, px - x);
+        if (ix && iz && ay) ey = min(ey, py - y);
+        if (ix && iy && az) ez = min(ez, pz - z);
+        if (ax && ay && az && px < x + ex && py < y + ey && pz < z + ez) mark = PT_MARKED;
+        const bool gone = in && (ex < ME.w || ey < ME.d || ez < ME.h);
+        if (in) {
+            K[cap + i] = gone ? 0u : (uint32_t)ex | ((uint32_t)ey << 16);
+            K[2 * cap + i] = (uint32_t)ez | mark;
         }
-        const unsigned bal = __ballot_sync(FULL, keep);
-        int off = 0;
-#pragma unroll 1
-        for (unsigned m = live; m; m &= m - 1) {
-            const int c = __ffs(m) - 1;
-            const uint32_t kc = __shfl_sync(FULL, ck, c);
-            if (__any_sync(FULL, keep && key == kc)) {
-                live &= ~(1u << c);
-                continue;
-            }
-            const unsigned lt = __ballot_sync(FULL, key < kc) & bal;
-            if (lane == c) rank += __popc(lt);
-            off += key > kc;
+        if ((x == px || x == px2) && (y == py || y == py2) && (z == pz || z == pz2))
+            dup |= 1u << ((x == px2 ? 1 : 0) | (y == py2 ? 2 : 0) | (z == pz2 ? 4 : 0));
+        const unsigned fr = __ballot_sync(FULL, gone);
+        if (fr) {
+            const int q = nf + __popc(fr & lanemask_lt());
+            if (gone && q < 32) free_slots[q] = (unsigned short)i;
+            nf += __popc(fr);
         }
-        if (resume >= cb && resume < cb + 32) at = ns + __popc(bal & ((1u << (resume - cb)) - 1u));
-        if (keep) {
-            const int d = ns + __popc(bal & lanemask_lt()) + off;
-            K2[d] = key;
-            K2[cap + d] = (uint32_t)ex | ((uint32_t)ey << 16);
-            K2[2 * cap + d] = (uint32_t)ez | mark;
-        }
-        ns += __popc(bal);
     }
-    resume = at;
-    nc = ns + __popc(live);
+    // (Lanes past the end read key 0, the container's corner: never a live corner.)
+    live &= ~__reduce_or_sync(FULL, dup);
+    __syncwarp();   // box tables, top-z index, points and freed slots are final
+    // The n-th live corner takes the n-th freed slot, or one past the end; the
+    // last point fills a slot left over. Slots past the 32nd freed in one
+    // placement keep their dead point, which the next placement frees again.
+    nf = min(nf, 32);
+    const int nl = __popc(live);
+    const int nth = __popc(live & ((1u << (lane & 7)) - 1u));
+    const int slot = nth < nf ? (int)free_slots[nth] : nc + nth - nf;
+#pragma unroll 1
+    for (int q = nf - 1; q >= nl; q--) {   // from the highest slot: the last point is alive or in it
+        const int h = free_slots[q];
+        nc--;
+        if (h != nc && lane < 3) K[lane * cap + h] = K[lane * cap + nc];
+        __syncwarp();
+    }
+    nc += max(nl - nf, 0);
     if (nc > C) return ERR_CAND_CAP;
-    __syncwarp();   // box tables and top-z index are final
     // Extents of the new corners: the boxes in registers, then any below them
     // from the tables (their old slots [0, nb0 - 64) now lie within
     // [0, nb0 - 64]; a box met twice, or the new one, changes nothing).
-    int nth = 0;
 #pragma unroll 1
     for (unsigned mc = live; mc; mc &= mc - 1) {
         const int c = __ffs(mc) - 1;
@@ -1092,12 +1102,10 @@ __device__ __forceinline__ int place1(uint32_t pkey, int pw, int pd, int ph, int
         }
         const uint32_t mark = __any_sync(FULL, meets) ? PT_MARKED : 0u;
         if (lane == c) {
-            const int d = rank + nth;
-            K2[d] = ck;
-            K2[cap + d] = (uint32_t)ex | ((uint32_t)ey << 16);
-            K2[2 * cap + d] = (uint32_t)ez | mark;
+            K[slot] = ck;
+            K[cap + slot] = (uint32_t)ex | ((uint32_t)ey << 16);
+            K[2 * cap + slot] = (uint32_t)ez | mark;
         }
-        nth++;
     }
     __syncwarp();
     return ERR_NONE;
@@ -1284,6 +1292,8 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
     int* z2s = reinterpret_cast<int*>(base + lay.off_z2);
     unsigned short* bis = reinterpret_cast<unsigned short*>(base + lay.off_bi);
     uint32_t* pts = reinterpret_cast<uint32_t*>(base + lay.off_pts);
+    uint2* Wl = reinterpret_cast<uint2*>(base + lay.off_w);
+    unsigned short* free_slots = reinterpret_cast<unsigned short*>(base + lay.off_free);
     unsigned short* zt = a.Hz ? reinterpret_cast<unsigned short*>(base + lay.off_zt) : nullptr;
 
     constexpr bool SERVE = MODE != 0;
@@ -1356,7 +1366,7 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
 
 #pragma unroll 1
         for (int pass = 0; pass < I.passes && err == ERR_NONE; pass++) {
-            int nb = 0, nc = 1, cur = 0;
+            int nb = 0, nc = 1;
             long long vol = 0;
             if (zt)
 #pragma unroll 1
@@ -1368,13 +1378,15 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
             }
             __syncwarp();
             int state_type = -1;
-            int resume = 0;         // points before it hold no feasible pair of state_type
+            uint32_t from_key = 0;  // points at smaller keys hold no feasible pair of state_type
             bool stuck = false;     // the last step of state_type found no feasible pair
             const EdgeRange ER{I.mw, I.md, I.mh, I.xw, I.xd, I.xh, L, W, H};
-            // a step's type and its edges are fetched one step ahead
+            // a step's type is fetched two steps ahead, its edges one, so that no
+            // step waits for the tables
             const int* steps = a.step_type + I.step_off;
             const TypeOrs* tors = a.types + I.type_off;
-            int t_next = -1, el_next = 0, ew_next = 0, eh_next = 0;
+            int t_next = -1, t_next2 = I.n_steps > 0 ? ld_table<SERVE>(steps) : -1;
+            int el_next = 0, ew_next = 0, eh_next = 0;
             Edges E{0, 0, 0};
             unsigned slots = 0;
 #pragma unroll 1
@@ -1385,55 +1397,49 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
                     E = Edges{el_next & 0x1ffff, ew_next, eh_next};
                     slots = (unsigned)el_next >> 20;
                 }
-                if (sti + 1 < I.n_steps) {
-                    t_next = ld_table<SERVE>(steps + sti + 1);
-                    if (t_next != t) {
-                        el_next = ld_table<SERVE>(&tors[t_next].el);
-                        ew_next = ld_table<SERVE>(&tors[t_next].ew);
-                        eh_next = ld_table<SERVE>(&tors[t_next].eh);
-                    }
+                t_next = t_next2;
+                if (sti + 2 < I.n_steps) t_next2 = ld_table<SERVE>(steps + sti + 2);
+                if (t_next != t && t_next >= 0) {
+                    el_next = ld_table<SERVE>(&tors[t_next].el);
+                    ew_next = ld_table<SERVE>(&tors[t_next].ew);
+                    eh_next = ld_table<SERVE>(&tors[t_next].eh);
                 }
                 // With no box placed since, another item of that type meets the
                 // same points and finds no pair either; it draws no random
                 // number, so the step is skipped without changing the result.
                 if (stuck && !fresh) continue;
-                const int from = fresh ? 0 : resume;
+                if (fresh) from_key = 0;
                 state_type = t;
                 if (slots == 0) {   // no orientation at all (or the fetch of the first step)
                     stuck = true;
                     continue;
                 }
-                const uint32_t* K = pts + cur * 3 * lay.cap;
-                uint32_t* K2 = pts + (cur ^ 1) * 3 * lay.cap;
                 // items: the points whose extents let an orientation through,
-                // {key, slots | marked << 7 | point index << 8}
-                uint2* Wl = reinterpret_cast<uint2*>(K2);
+                // {key, slots | marked << 7}
                 int nW = 0;
 #pragma unroll 1
-                for (int cb = from; cb < nc; cb += 32) {
+                for (int cb = 0; cb < nc; cb += 32) {
                     const int i = cb + lane;
                     unsigned m = 0;
                     uint32_t key = 0;
                     if (i < nc) {
-                        key = K[i];
-                        const uint32_t exy = K[lay.cap + i], ezm = K[2 * lay.cap + i];
+                        key = pts[i];
+                        const uint32_t exy = pts[lay.cap + i], ezm = pts[2 * lay.cap + i];
                         m = slots & x_within(E, (int)(exy & 0xffffu)) & y_within(E, (int)(exy >> 16)) &
                             z_within(E, (int)(ezm & 0xffffu));
-                        if (m) m |= (ezm & PT_MARKED) >> 9 | (unsigned)i << 8;
+                        if (key < from_key) m = 0;
+                        if (m) m |= (ezm & PT_MARKED) >> 9;
                     }
                     const unsigned bal = __ballot_sync(FULL, m != 0);
                     if (m) Wl[nW + __popc(bal & lanemask_lt())] = make_uint2(key, m);
                     nW += __popc(bal);
                 }
                 __syncwarp();
-                // C3 for 32 items at a time, then C1 of the marked ones. The first
-                // item with a feasible pair decides the branch; the random branch
-                // goes on to the end and keeps every item's feasible set.
-                int first = -1, pick_p = 0;      // item and point of the first feasible pair
-                unsigned pick_m = 0;             // its feasible set
-                uint32_t pick_key = 0;
+                // feasible set of every item: C3, then C1 of the marked ones. The
+                // first feasible point is the one with the smallest key.
+                uint32_t best_key = 0xffffffffu;   // of this lane's items
+                unsigned best_set = 0;
                 int count = 0;
-                bool full = false;
 #pragma unroll 1
                 for (int w0 = 0; w0 < nW; w0 += 32) {
                     const uint2 e = w0 + lane < nW ? Wl[w0 + lane] : make_uint2(0, 0);
@@ -1444,83 +1450,75 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
                         cand = support_slots(cand, (int)(e.x & xmask), (int)((e.x >> xb) & ymask), j, je, E, bx);
                     }
                     __syncwarp();
-                    const unsigned marked = __ballot_sync(FULL, cand && (e.y & 0x80u));
-                    // items in order up to the first feasible one, then the marked ones
 #pragma unroll 1
-                    for (unsigned bal = first < 0 ? __ballot_sync(FULL, cand != 0) : marked; bal; bal &= bal - 1) {
+                    for (unsigned bal = __ballot_sync(FULL, cand && (e.y & 0x80u)); bal; bal &= bal - 1) {
                         const int q = __ffs(bal) - 1;
                         const uint32_t kq = __shfl_sync(FULL, e.x, q);
-                        unsigned ok = __shfl_sync(FULL, cand, q);
-                        if ((marked >> q) & 1u) {
-                            const int zq = (int)(kq >> xyb);
-                            ok &= ~blocked_slots((int)(kq & xmask), (int)((kq >> xb) & ymask), zq,
-                                                 box_start(zt, z2s, nb, zq + 1), nb, E, bx, bzs, lane);
-                            if (lane == q) cand = ok;
-                        }
-                        if (ok && first < 0) {
-                            first = w0 + q;
-                            pick_key = kq;
-                            pick_m = ok;
-                            pick_p = (int)(__shfl_sync(FULL, e.y, q) >> 8);
-                            // random() only once a feasible pair exists
-                            full = randomized && mt_random(mt, mpos, lane) >= 1.0 - I.eps;
-                            if (!full) break;
-                            bal &= marked | (1u << q);
-                        }
+                        const int zq = (int)(kq >> xyb);
+                        const unsigned blk = blocked_slots((int)(kq & xmask), (int)((kq >> xb) & ymask), zq,
+                                                           box_start(zt, z2s, nb, zq + 1), nb, E, bx, bzs, lane);
+                        if (lane == q) cand &= ~blk;
                     }
-                    if (first >= 0) {
-                        if (!full) break;
-                        count += __popc(cand);
-                        if (w0 + lane < nW) Wl[w0 + lane].y = cand;
+                    const int c = __popc(cand);
+                    count += c;
+                    if (cand && e.x < best_key) {
+                        best_key = e.x;
+                        best_set = cand;
                     }
+                    if (w0 + lane < nW) Wl[w0 + lane].y = cand | (unsigned)c << 8;
                 }
-                stuck = first < 0;
+                uint32_t pick_key = __reduce_min_sync(FULL, best_key);
+                stuck = pick_key == 0xffffffffu;
                 if (stuck) continue;                     // no feasible pair: no draw
-                int slot = __ffs(pick_m) - 1;
-                if (full) {
+                from_key = pick_key;
+                unsigned pick_set = __shfl_sync(FULL, best_set, __ffs(__ballot_sync(FULL, best_key == pick_key)) - 1);
+                // random() only once a feasible pair exists
+                if (randomized && mt_random(mt, mpos, lane) >= 1.0 - I.eps) {
                     const int idx = mt_randrange(mt, mpos, lane, __reduce_add_sync(FULL, count));
                     if (idx < 0) {
                         err = ERR_RNG;
                         break;
                     }
                     __syncwarp();
-                    // idx-th feasible pair in (point, orientation) order
-                    int run = 0;
+                    // idx-th feasible pair in (point, orientation) order: the item
+                    // with at most idx pairs at smaller keys and more with its own
 #pragma unroll 1
-                    for (int w0 = first & ~31; w0 < nW; w0 += 32) {
+                    for (int w0 = 0; w0 < nW; w0 += 32) {
                         const uint2 e = w0 + lane < nW ? Wl[w0 + lane] : make_uint2(0, 0);
-                        const int c = __popc(e.y);
-                        // lane prefix of the pair counts (each below 8) from their bits
-                        const unsigned b0 = __ballot_sync(FULL, c & 1), b1 = __ballot_sync(FULL, c & 2),
-                                       b2 = __ballot_sync(FULL, c & 4);
-                        const unsigned lt = lanemask_lt();
-                        const int excl = __popc(b0 & lt) + 2 * __popc(b1 & lt) + 4 * __popc(b2 & lt);
-                        const int tot = __popc(b0) + 2 * __popc(b1) + 4 * __popc(b2);
-                        if (idx < run + tot) {
-                            const int q = __ffs(__ballot_sync(FULL, idx < run + excl + c)) - 1;
-                            unsigned m = __shfl_sync(FULL, e.y, q);
-#pragma unroll 1
-                            for (int k = idx - run - __shfl_sync(FULL, excl, q); k > 0; k--) m &= m - 1;
+                        int k = idx;
+                        // two items to a load; an odd last one reads a word that
+                        // is not below any key
+                        if (lane == 0 && (nW & 1)) Wl[nW] = make_uint2(0xffffffffu, 0u);
+                        __syncwarp();
+                        const uint4* W2 = reinterpret_cast<const uint4*>(Wl);
+#pragma unroll 2
+                        for (int w = 0; w < (nW + 1) >> 1; w++) {
+                            const uint4 o = W2[w];
+                            if (o.x < e.x) k -= (int)(o.y >> 8);
+                            if (o.z < e.x) k -= (int)(o.w >> 8);
+                        }
+                        const unsigned hit = __ballot_sync(FULL, k >= 0 && k < (int)(e.y >> 8));
+                        if (hit) {
+                            const int q = __ffs(hit) - 1;
                             pick_key = __shfl_sync(FULL, e.x, q);
-                            slot = __ffs(m) - 1;
+                            pick_set = __shfl_sync(FULL, e.y, q) & 0x3fu;
+#pragma unroll 1
+                            for (k = __shfl_sync(FULL, k, q); k > 0; k--) pick_set &= pick_set - 1;
                             break;
                         }
-                        run += tot;
                     }
                 }
+                const int slot = __ffs(pick_set) - 1;
                 const int pw = (0x14 >> slot) & 1 ? E.l : (0x21 >> slot) & 1 ? E.w : E.h;
                 const int pd = (0x28 >> slot) & 1 ? E.l : (0x12 >> slot) & 1 ? E.w : E.h;
                 const int ph = slot < 2 ? E.l : slot < 4 ? E.w : E.h;
-                resume = pick_p;
                 if (lane == 0 && nb < a.P)
                     pass_out[nb] = pack_place((int)(pick_key & xmask), (int)((pick_key >> xb) & ymask),
                                               (int)(pick_key >> xyb), __popc(slots & ((1u << slot) - 1u)), t);
                 vol += 1LL * pw * pd * ph;
-                __syncwarp();   // every lane has read the item list before K2 is written
-                err = place1(pick_key, pw, pd, ph, resume, K, K2, lay.cap, bx, bzs, z2s, bis, zt, a.Hz, nc, nb, a.P,
+                err = place1(pick_key, pw, pd, ph, pts, lay.cap, free_slots, bx, bzs, z2s, bis, zt, a.Hz, nc, nb, a.P,
                              a.C, xmask, ymask, xb, xyb, ER, lane);
                 if (err != ERR_NONE) break;
-                cur ^= 1;
             }
             if (err != ERR_NONE) break;
             const double score =

@@ -140,22 +140,32 @@ static __device__ __noinline__ void mt_seed_warp(uint32_t* mt, unsigned long lon
         const uint32_t k0 = (uint32_t)seed_abs;
         const uint32_t k1 = (uint32_t)(seed_abs >> 32);
         const uint32_t add0 = k0, add1 = k1 ? k1 + 1u : k0;
-        // First loop: 624 steps over i = 1 .. 623, then i = 1 again. Blocks
-        // of 8 with their old words loaded up front keep the load latency
-        // off the serial chain.
+        // First loop: 624 steps over i = 1 .. 623, then i = 1 again. Blocks of
+        // 8 whose old words were loaded during the block before, so the chain
+        // is the five dependent operations of each step.
         uint32_t prev = mt[0];
-        for (int i = 1; i < 624; i += 8) {
-            uint32_t o[8];
+        uint32_t o[8];
 #pragma unroll
-            for (int u = 0; u < 8; u++) o[u] = i + u < 624 ? mt[i + u] : 0u;
+        for (int u = 0; u < 8; u++) o[u] = mt[1 + u];
+#pragma unroll 1
+        for (int i = 1; i < 617; i += 8) {       // 77 blocks: i = 1 .. 616
+            uint32_t nx[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) nx[u] = mt[min(i + 8 + u, 623)];
 #pragma unroll
             for (int u = 0; u < 8; u++) {
-                if (i + u < 624) {
-                    const uint32_t t = prev ^ (prev >> 30);
-                    prev = (o[u] ^ (t * 1664525u)) + (((i + u - 1) & 1) ? add1 : add0);
-                    mt[i + u] = prev;
-                }
+                const uint32_t t = prev ^ (prev >> 30);
+                prev = (o[u] ^ (t * 1664525u)) + ((u & 1) ? add1 : add0);   // step i + u - 1
+                mt[i + u] = prev;
             }
+#pragma unroll
+            for (int u = 0; u < 8; u++) o[u] = nx[u];
+        }
+#pragma unroll
+        for (int u = 0; u < 7; u++) {            // i = 617 .. 623
+            const uint32_t t = prev ^ (prev >> 30);
+            prev = (o[u] ^ (t * 1664525u)) + ((u & 1) ? add1 : add0);
+            mt[617 + u] = prev;
         }
         {
             const uint32_t t = prev ^ (prev >> 30);
@@ -163,18 +173,27 @@ static __device__ __noinline__ void mt_seed_warp(uint32_t* mt, unsigned long lon
             mt[1] = prev;
         }
         // Second loop: 623 steps over i = 2 .. 623, then i = 1.
-        for (int i = 2; i < 624; i += 8) {
-            uint32_t o[8];
 #pragma unroll
-            for (int u = 0; u < 8; u++) o[u] = i + u < 624 ? mt[i + u] : 0u;
+        for (int u = 0; u < 8; u++) o[u] = mt[2 + u];
+#pragma unroll 1
+        for (int i = 2; i < 618; i += 8) {       // 77 blocks: i = 2 .. 617
+            uint32_t nx[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) nx[u] = mt[min(i + 8 + u, 623)];
 #pragma unroll
             for (int u = 0; u < 8; u++) {
-                if (i + u < 624) {
-                    const uint32_t t = prev ^ (prev >> 30);
-                    prev = (o[u] ^ (t * 1566083941u)) - (uint32_t)(i + u);
-                    mt[i + u] = prev;
-                }
+                const uint32_t t = prev ^ (prev >> 30);
+                prev = (o[u] ^ (t * 1566083941u)) - (uint32_t)(i + u);
+                mt[i + u] = prev;
             }
+#pragma unroll
+            for (int u = 0; u < 8; u++) o[u] = nx[u];
+        }
+#pragma unroll
+        for (int u = 0; u < 6; u++) {            // i = 618 .. 623
+            const uint32_t t = prev ^ (prev >> 30);
+            prev = (o[u] ^ (t * 1566083941u)) - (uint32_t)(618 + u);
+            mt[618 + u] = prev;
         }
         {
             const uint32_t t = prev ^ (prev >> 30);
