@@ -574,7 +574,7 @@ __device__ __forceinline__ void block_body(const BlockArgs& a, unsigned char* ba
                     fbi[p] = (unsigned short)q;
                 }
                 __syncwarp();
-                const double score = fsr_score_warp(fbx, fbz, fz2, fbi, n_items, I.mu,
+                const double score = fsr_score_warp(WideBoxes{fbx, fbz, fz2, fbi}, n_items, I.mu,
                                                     reinterpret_cast<char*>(fsr_base + lay.f_scr), lane, nullptr);
                 const bool acc = !I.has_theta || score >= I.theta;
                 bool take;

@@ -116,7 +116,7 @@ __host__ __device__ inline DecLayout dec_layout(int P, int C, int Hz) {
 // the step's items. Eight slots past C take
 // a placement's corners before the capacity check.
 struct Dec1Layout {
-    int off_bx, off_bz, off_z2, off_bi, off_pts, off_w, off_free, off_zt, bytes;
+    int off_box, off_pts, off_w, off_free, off_zt, bytes;
     int cap;   // entries per array of the points
 };
 
@@ -124,16 +124,12 @@ __host__ __device__ inline Dec1Layout dec1_layout(int P, int C, int Hz) {
     Dec1Layout l;
     int o = 624 * 4;                       // MT state
     o = (o + 15) & ~15;
-    l.off_bx = o;  o += 16 * P;            // int4 {x, y, x2, y2}
-    l.off_bz = o;  o += 4 * P;             // bottom z
-    l.off_z2 = o;  o += 4 * P;             // top z
-    l.off_bi = o;  o += 2 * P;             // placement index
-    o = (o + 15) & ~15;
+    l.off_box = o;  o += 16 * P;           // PackedBoxes
     l.cap = C + 8;
     l.off_pts = o;
     l.off_w = o + 12 * l.cap;
-    int region = 12 * l.cap + 8 * (C + 2);       // FSR overlays 18 bytes per box
-    if (region < 18 * P + 32) region = 18 * P + 32;
+    int region = 12 * l.cap + 8 * (C + 2);       // FSR overlays 14 bytes per box
+    if (region < 14 * P + 16) region = 14 * P + 16;
     o += region;
     o = (o + 15) & ~15;
     l.off_free = o;  o += 64;              // u16: slots a placement frees (the first 32)
@@ -717,7 +713,7 @@ __device__ __forceinline__ void decoder_body(const DecoderArgs& a, unsigned char
             if (err != ERR_NONE) break;
             // score the pass and keep the selected one (warp 0)
             if (g == 0) {
-                const double score = fsr_score_warp(bx, bzs, z2s, bis, nb, I.mu,
+                const double score = fsr_score_warp(WideBoxes{bx, bzs, z2s, bis}, nb, I.mu,
                                                     reinterpret_cast<char*>(candA), lane, nullptr);
                 const bool acc = !I.has_theta || score >= I.theta;
                 bool take;
@@ -835,22 +831,28 @@ __device__ __forceinline__ unsigned z_within(const Edges& E, int v) {
     return (E.l <= v ? 0x03u : 0u) | (E.w <= v ? 0x0cu : 0u) | (E.h <= v ? 0x30u : 0u);
 }
 
+// First box with top >= z: from the top-z index, or by search without one.
+__device__ __forceinline__ int top_start(const unsigned short* zt, const uint4* bx, int nb, int z) {
+    return zt ? (int)zt[z] : first_top(PackedBoxes{bx}, nb, z);
+}
+
 // Slots of `cand` whose C3 holds at (x, y, z), z > 0: contact with the boxes
 // [j, je), whose top is z. Areas are at most the container's footprint, below
 // 2^31, so twice an area fits 32 unsigned bits.
 __device__ __forceinline__ unsigned support_slots(unsigned cand, int x, int y, int j, int je, const Edges& E,
-                                                  const int4* bx) {
+                                                  const uint4* bx) {
     unsigned a0 = 0, a1 = 0, a2 = 0, a3 = 0, a4 = 0, a5 = 0;
     const int xl = x + E.l, xw = x + E.w, xh = x + E.h, yl = y + E.l, yw = y + E.w, yh = y + E.h;
     // two boxes at a time; past the end an empty box, which adds nothing
 #pragma unroll 1
     for (; j < je; j += 2) {
-        const int4 b0 = bx[j], b1 = j + 1 < je ? bx[j + 1] : make_int4(0, 0, 0, 0);
+        const uint2 b0 = *reinterpret_cast<const uint2*>(bx + j);
+        const uint2 b1 = j + 1 < je ? *reinterpret_cast<const uint2*>(bx + j + 1) : make_uint2(0, 0);
 #pragma unroll
         for (int u = 0; u < 2; u++) {
-            const int4 b = u ? b1 : b0;
-            const int nx = -max(x, b.x), ny = -max(y, b.y);
-            const int tx = b.z + nx, ty = b.w + ny;
+            const uint2 b = u ? b1 : b0;
+            const int nx = -max(x, (int)(b.x & 0xffffu)), ny = -max(y, (int)(b.y & 0xffffu));
+            const int tx = (int)(b.x >> 16) + nx, ty = (int)(b.y >> 16) + ny;
             // overlap along an axis: max(0, min(x + e, b.x2) - max(x, b.x))
             const unsigned ol = __viaddmin_s32_relu(xl, nx, tx), ow = __viaddmin_s32_relu(xw, nx, tx),
                            oh = __viaddmin_s32_relu(xh, nx, tx);
@@ -873,17 +875,17 @@ __device__ __forceinline__ unsigned support_slots(unsigned cand, int x, int y, i
 // Warp: slots that some box of [j0, nb) overlaps at (x, y, z) (C1; boxes
 // below j0 end at or under z). Offsets from the point keep each axis to one
 // subtraction and three compares.
-__device__ __forceinline__ unsigned blocked_slots(int x, int y, int z, int j0, int nb, const Edges& E, const int4* bx,
-                                                  const int* bzs, int lane) {
+__device__ __forceinline__ unsigned blocked_slots(int x, int y, int z, int j0, int nb, const Edges& E, const uint4* bx,
+                                                  int lane) {
     unsigned blk = 0;
 #pragma unroll 1
     for (int jb = j0; jb < nb; jb += 32) {
         const int j = jb + lane;
         if (j < nb) {
-            const int4 b = bx[j];
-            const int bz = bzs[j];
-            if (b.z > x && b.w > y)
-                blk |= ~(x_within(E, b.x - x) | y_within(E, b.y - y) | z_within(E, bz - z));
+            const uint4 b = bx[j];
+            if ((int)(b.x >> 16) > x && (int)(b.y >> 16) > y)
+                blk |= ~(x_within(E, (int)(b.x & 0xffffu) - x) | y_within(E, (int)(b.y & 0xffffu) - y) |
+                         z_within(E, (int)(b.z & 0xffffu) - z));
         }
     }
     return __reduce_or_sync(FULL, blk & 0x3fu);
@@ -909,12 +911,14 @@ struct CornerFrame {
     // corners whose x extent it ends, whose y extent, whose z extent, and
     // those it reaches past on every axis. Corners whose cuboid it meets are
     // added to dead.
-    __device__ __forceinline__ uint32_t relate(const int4& b, int bz, int bt, unsigned& dead) const {
-        const bool ax = x < b.z, ax2 = x2 < b.z, ay = y < b.w, ay2 = y2 < b.w, az = z < bt, az2 = z2 < bt;
+    __device__ __forceinline__ uint32_t relate(const uint4& v, unsigned& dead) const {
+        const int bx2 = (int)(v.x >> 16), by2 = (int)(v.y >> 16), bt = (int)(v.z >> 16);
+        const int bx = (int)(v.x & 0xffffu), by = (int)(v.y & 0xffffu), bz = (int)(v.z & 0xffffu);
+        const bool ax = x < bx2, ax2 = x2 < bx2, ay = y < by2, ay2 = y2 < by2, az = z < bt, az2 = z2 < bt;
         const unsigned xa = (ax ? 0x55u : 0u) | (ax2 ? 0xaau : 0u), ya = (ay ? 0x33u : 0u) | (ay2 ? 0xccu : 0u),
                        za = (az ? 0x0fu : 0u) | (az2 ? 0xf0u : 0u);
-        const unsigned xi = xa & ((b.x < xm ? 0x55u : 0u) | (b.x < x2m ? 0xaau : 0u)),
-                       yi = ya & ((b.y < ym ? 0x33u : 0u) | (b.y < y2m ? 0xccu : 0u)),
+        const unsigned xi = xa & ((bx < xm ? 0x55u : 0u) | (bx < x2m ? 0xaau : 0u)),
+                       yi = ya & ((by < ym ? 0x33u : 0u) | (by < y2m ? 0xccu : 0u)),
                        zi = za & ((bz < zm ? 0x0fu : 0u) | (bz < z2m ? 0xf0u : 0u));
         dead |= xi & yi & zi;
         return (xa & yi & zi) | (xi & ya & zi) << 8 | (xi & yi & za) << 16 | (xa & ya & za) << 24;
@@ -926,7 +930,7 @@ struct CornerFrame {
 // x | y << 16 extents, z extent | mark): the box is applied to every point,
 // dead ones give up their slots, and the box's live corners come in.
 __device__ __forceinline__ int place1(uint32_t pkey, int pw, int pd, int ph, uint32_t* K, int cap,
-                                      unsigned short* free_slots, int4* bx, int* bzs, int* z2s, unsigned short* bis,
+                                      unsigned short* free_slots, uint4* bx,
                                       unsigned short* zt, int Hz, int& nc, int& nb, int P, int C, uint32_t xmask,
                                       uint32_t ymask, int xb, int xyb, const EdgeRange& ME, int lane) {
     const int px = (int)(pkey & xmask), py = (int)((pkey >> xb) & ymask), pz = (int)(pkey >> xyb);
@@ -944,8 +948,7 @@ __device__ __forceinline__ int place1(uint32_t pkey, int pw, int pd, int ph, uin
     if (F.z2m > ME.H) dead |= 0xf0u;
     int nabove = 0;
     const int nb0 = nb;
-    int4 wb[2];
-    int wz[2];
+    uint4 wb[2];
     uint32_t wm[2] = {0u, 0u};
 #pragma unroll
     for (int r = 0; r < 3; r++) {
@@ -954,28 +957,14 @@ __device__ __forceinline__ int place1(uint32_t pkey, int pw, int pd, int ph, uin
         for (int hi = nb0 - 32 * r; hi > 0; hi -= 32) {
             const int jj = hi - 1 - lane;
             const bool in = jj >= 0;
-            int4 b = make_int4(0, 0, 0, 0);
-            int bzb = 0, bzt = 0;
-            unsigned short bi = 0;
-            if (in) {
-                b = bx[jj];
-                bzb = bzs[jj];
-                bzt = z2s[jj];
-                bi = bis[jj];
-            }
-            const uint32_t m = F.relate(b, bzb, bzt, dead);
-            const bool up = in && bzt > pz2;
+            const uint4 v = in ? bx[jj] : make_uint4(0, 0, 0, 0);   // the empty box lies before every corner
+            const uint32_t m = F.relate(v, dead);
+            const bool up = in && (int)(v.z >> 16) > pz2;
             nabove += __popc(__ballot_sync(FULL, up));
             __syncwarp();
-            if (up) {
-                bx[jj + 1] = b;
-                bzs[jj + 1] = bzb;
-                z2s[jj + 1] = bzt;
-                bis[jj + 1] = bi;
-            }
+            if (up) bx[jj + 1] = v;
             if (r < 2) {
-                wb[r] = b;
-                wz[r] = bzb;
+                wb[r] = v;
                 wm[r] = m;
                 break;
             }
@@ -986,10 +975,8 @@ __device__ __forceinline__ int place1(uint32_t pkey, int pw, int pd, int ph, uin
         const int ip = nb - nabove;   // after the boxes with equal tops
         __syncwarp();
         if (lane == 0) {
-            bx[ip] = make_int4(px, py, px2, py2);
-            bzs[ip] = pz;
-            z2s[ip] = pz2;
-            bis[ip] = (unsigned short)nb;
+            bx[ip] = make_uint4((uint32_t)px | (uint32_t)px2 << 16, (uint32_t)py | (uint32_t)py2 << 16,
+                                (uint32_t)pz | (uint32_t)pz2 << 16, (uint32_t)nb);
         }
     }
     if (zt) {
@@ -1072,16 +1059,16 @@ __device__ __forceinline__ int place1(uint32_t pkey, int pw, int pd, int ph, uin
         for (int r = 0; r < 2; r++) {
             if (32 * r < nb0) {
                 const uint32_t m = wm[r] >> c;
-                if (m & 1u) ex = min(ex, wb[r].x - x);
-                if (m & 0x100u) ey = min(ey, wb[r].y - y);
-                if (m & 0x10000u) ez = min(ez, wz[r] - z);
+                if (m & 1u) ex = min(ex, (int)(wb[r].x & 0xffffu) - x);
+                if (m & 0x100u) ey = min(ey, (int)(wb[r].y & 0xffffu) - y);
+                if (m & 0x10000u) ez = min(ez, (int)(wb[r].z & 0xffffu) - z);
             }
         }
-        const int j0 = nb0 > 64 ? box_start(zt, z2s, nb, z + 1) : nb;
+        const int j0 = nb0 > 64 ? top_start(zt, bx, nb, z + 1) : nb;
 #pragma unroll 1
         for (int j = j0 + lane; j <= nb0 - 64; j += 32) {
-            const int4 b = bx[j];
-            const int bz = bzs[j];
+            const int4 b = PackedBoxes{bx}.xy(j);
+            const int bz = PackedBoxes{bx}.bottom(j);
             const bool ix = b.x < x + ME.w && x < b.z, iy = b.y < y + ME.d && y < b.w, iz = bz < z + ME.h;
             if (iy && iz && x < b.z) ex = min(ex, b.x - x);
             if (ix && iz && y < b.w) ey = min(ey, b.y - y);
@@ -1094,11 +1081,12 @@ __device__ __forceinline__ int place1(uint32_t pkey, int pw, int pd, int ph, uin
 #pragma unroll
         for (int r = 0; r < 2; r++)
             if (32 * r < nb0)
-                meets = meets || (((wm[r] >> c) & 0x1000000u) && wb[r].x < x + ex && wb[r].y < y + ey && wz[r] < z + ez);
+                meets = meets || (((wm[r] >> c) & 0x1000000u) && (int)(wb[r].x & 0xffffu) < x + ex &&
+                                  (int)(wb[r].y & 0xffffu) < y + ey && (int)(wb[r].z & 0xffffu) < z + ez);
 #pragma unroll 1
         for (int j = j0 + lane; j <= nb0 - 64; j += 32) {
-            const int4 b = bx[j];
-            meets = meets || (b.x < x + ex && x < b.z && b.y < y + ey && y < b.w && bzs[j] < z + ez);
+            const int4 b = PackedBoxes{bx}.xy(j);
+            meets = meets || (b.x < x + ex && x < b.z && b.y < y + ey && y < b.w && PackedBoxes{bx}.bottom(j) < z + ez);
         }
         const uint32_t mark = __any_sync(FULL, meets) ? PT_MARKED : 0u;
         if (lane == c) {
@@ -1287,16 +1275,14 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
     const int lane = threadIdx.x & 31;
     const Dec1Layout lay = dec1_layout(a.P, a.C, a.Hz);
     uint32_t* mt = reinterpret_cast<uint32_t*>(base);
-    int4* bx = reinterpret_cast<int4*>(base + lay.off_bx);
-    int* bzs = reinterpret_cast<int*>(base + lay.off_bz);
-    int* z2s = reinterpret_cast<int*>(base + lay.off_z2);
-    unsigned short* bis = reinterpret_cast<unsigned short*>(base + lay.off_bi);
+    uint4* bx = reinterpret_cast<uint4*>(base + lay.off_box);
     uint32_t* pts = reinterpret_cast<uint32_t*>(base + lay.off_pts);
     uint2* Wl = reinterpret_cast<uint2*>(base + lay.off_w);
     unsigned short* free_slots = reinterpret_cast<unsigned short*>(base + lay.off_free);
     unsigned short* zt = a.Hz ? reinterpret_cast<unsigned short*>(base + lay.off_zt) : nullptr;
 
     constexpr bool SERVE = MODE != 0;
+    constexpr int SPACE = MODE == 2 ? 1 : 0;   // the overflow decoders' tile is in global memory
     const int n_work = SERVE ? 0 : (a.n_work_dev ? *a.n_work_dev : a.n_work);
 #pragma unroll 1
     for (;;) {
@@ -1353,7 +1339,7 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
                 for (int i = lane; i < 156; i += 32) dst[i] = __ldg(src + i);
                 __syncwarp();
             } else {
-                mt_seed_warp(mt, (unsigned long long)(sd < 0 ? -sd : sd), a.mt_init, lane);
+                mt_seed_warp<SPACE>(mt, (unsigned long long)(sd < 0 ? -sd : sd), a.mt_init, lane);
             }
         }
         const long long t0 = global_ns();   // the reference's run() clock starts after seeding
@@ -1446,7 +1432,7 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
                     unsigned cand = e.y & 0x3fu;
                     const int z = (int)(e.x >> xyb);
                     if (z > 0 && cand) {
-                        const int j = box_start(zt, z2s, nb, z), je = box_start(zt, z2s, nb, z + 1);
+                        const int j = top_start(zt, bx, nb, z), je = top_start(zt, bx, nb, z + 1);
                         cand = support_slots(cand, (int)(e.x & xmask), (int)((e.x >> xb) & ymask), j, je, E, bx);
                     }
                     __syncwarp();
@@ -1456,7 +1442,7 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
                         const uint32_t kq = __shfl_sync(FULL, e.x, q);
                         const int zq = (int)(kq >> xyb);
                         const unsigned blk = blocked_slots((int)(kq & xmask), (int)((kq >> xb) & ymask), zq,
-                                                           box_start(zt, z2s, nb, zq + 1), nb, E, bx, bzs, lane);
+                                                           top_start(zt, bx, nb, zq + 1), nb, E, bx, lane);
                         if (lane == q) cand &= ~blk;
                     }
                     const int c = __popc(cand);
@@ -1473,8 +1459,8 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
                 from_key = pick_key;
                 unsigned pick_set = __shfl_sync(FULL, best_set, __ffs(__ballot_sync(FULL, best_key == pick_key)) - 1);
                 // random() only once a feasible pair exists
-                if (randomized && mt_random(mt, mpos, lane) >= 1.0 - I.eps) {
-                    const int idx = mt_randrange(mt, mpos, lane, __reduce_add_sync(FULL, count));
+                if (randomized && mt_random<SPACE>(mt, mpos, lane) >= 1.0 - I.eps) {
+                    const int idx = mt_randrange<SPACE>(mt, mpos, lane, __reduce_add_sync(FULL, count));
                     if (idx < 0) {
                         err = ERR_RNG;
                         break;
@@ -1516,13 +1502,13 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
                     pass_out[nb] = pack_place((int)(pick_key & xmask), (int)((pick_key >> xb) & ymask),
                                               (int)(pick_key >> xyb), __popc(slots & ((1u << slot) - 1u)), t);
                 vol += 1LL * pw * pd * ph;
-                err = place1(pick_key, pw, pd, ph, pts, lay.cap, free_slots, bx, bzs, z2s, bis, zt, a.Hz, nc, nb, a.P,
-                             a.C, xmask, ymask, xb, xyb, ER, lane);
+                err = place1(pick_key, pw, pd, ph, pts, lay.cap, free_slots, bx, zt, a.Hz, nc, nb, a.P, a.C,
+                             xmask, ymask, xb, xyb, ER, lane);
                 if (err != ERR_NONE) break;
             }
             if (err != ERR_NONE) break;
             const double score =
-                fsr_score_warp(bx, bzs, z2s, bis, nb, I.mu, reinterpret_cast<char*>(pts), lane, nullptr, zt);
+                fsr_score_warp<SPACE>(PackedBoxes{bx}, nb, I.mu, reinterpret_cast<char*>(pts), lane, nullptr, zt);
             const bool acc = !I.has_theta || score >= I.theta;
             bool take;
             if (acc) take = !have_acc || vol > best_vol || (vol == best_vol && nb > best_n);
@@ -1706,7 +1692,7 @@ __global__ void fsr_kernel(const int* __restrict__ rows7, const int* __restrict_
         bi[rank] = (unsigned short)i;
     }
     __syncwarp();
-    const double sc = fsr_score_warp(bx, bz, z2, bi, n, mu, scratch, lane,
+    const double sc = fsr_score_warp(WideBoxes{bx, bz, z2, bi}, n, mu, scratch, lane,
                                      out_fsr ? out_fsr + o0 : nullptr);
     if (lane == 0) out_score[pk] = sc;
 }
@@ -1968,17 +1954,24 @@ cudaError_t launch_gather_best(const InstDesc* inst, int n_inst, const int2* bes
 #endif  // PLP_SERVE_TU
 
 #ifdef PLP_SERVE_TU
+// Overflow decoders run out of line: with both bodies in one, the main
+// decoders' build for 18 per SM spilled 400 bytes and its code doubled.
+static __device__ __noinline__ void serve_deep(const DecoderArgs& a, const ServeArgs& s, int gdec) {
+    DecoderArgs ad = a;
+    ad.P = s.deep_P;
+    ad.C = s.deep_C;
+    decoder1_body<2>(ad, s.deep_scratch + (size_t)gdec * s.deep_bytes, gdec, s);
+}
+
 // The serving launch: the single-warp decoder over the host-published ring.
 template <int D, int M>
-__global__ void __launch_bounds__(32 * D, M) serve_kernel(DecoderArgs a, ServeArgs s) {
+__global__ void __launch_bounds__(32 * D, M == 16 ? 18 : M)
+    serve_kernel(const __grid_constant__ DecoderArgs a, const __grid_constant__ ServeArgs s) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int dec = threadIdx.x >> 5;
     const int gdec = blockIdx.x * D + dec;
     if (gdec < s.n_deep) {
-        DecoderArgs ad = a;
-        ad.P = s.deep_P;
-        ad.C = s.deep_C;
-        decoder1_body<2>(ad, s.deep_scratch + (size_t)gdec * s.deep_bytes, gdec, s);
+        serve_deep(a, s, gdec);
     } else {
         const Dec1Layout lay = dec1_layout(a.P, a.C, a.Hz);
         decoder1_body<1>(a, smem_raw + (size_t)dec * lay.bytes, gdec, s);
@@ -1987,7 +1980,7 @@ __global__ void __launch_bounds__(32 * D, M) serve_kernel(DecoderArgs a, ServeAr
 
 // ---- serving launches ------------------------------------------------------
 using ServeFn = void (*)(DecoderArgs, ServeArgs);
-#define PLP_SERVE_CONFIGS(X) X(1, 1) X(1, 12)
+#define PLP_SERVE_CONFIGS(X) X(1, 1) X(1, 12) X(1, 16)
 
 static ServeFn serve_fn(int D, int M) {
 #define PLP_PICK_SERVE(d, m) \

@@ -131,6 +131,11 @@ __device__ __forceinline__ unsigned lanemask_lt() {
 // init_by_array on |seed| (one or two 32-bit key words), starting from the
 // seed-independent init_genrand(19650218) table `init`. The recurrence is
 // serial: lane 0 runs it, the warp then syncs.
+//
+// SPACE keeps callers whose state lies in different address spaces (the
+// serving launch's main and overflow decoders) on instantiations of their own:
+// an out-of-line function that both call would address memory generically.
+template <int SPACE = 0>
 static __device__ __noinline__ void mt_seed_warp(uint32_t* mt, unsigned long long seed_abs,
                                     const uint32_t* __restrict__ init, int lane) {
     for (int i = lane; i < 624; i += 32) mt[i] = init[i];
@@ -208,6 +213,7 @@ static __device__ __noinline__ void mt_seed_warp(uint32_t* mt, unsigned long lon
 // (i + 397) mod 624, which is still old for i < 227 and already new for
 // i >= 227. Chunks of 32 in increasing i therefore only read finished or
 // untouched words; inside a chunk all lanes read before any lane writes.
+template <int SPACE = 0>
 static __device__ __noinline__ void mt_twist_warp(uint32_t* mt, int lane) {
 #pragma unroll 1
     for (int base = 0; base < 623; base += 32) {
@@ -229,9 +235,10 @@ static __device__ __noinline__ void mt_twist_warp(uint32_t* mt, int lane) {
     __syncwarp();
 }
 
+template <int SPACE = 0>
 __device__ __forceinline__ uint32_t mt_next(uint32_t* mt, int& pos, int lane) {
     if (pos >= 624) {
-        mt_twist_warp(mt, lane);
+        mt_twist_warp<SPACE>(mt, lane);
         pos = 0;
     }
     uint32_t y = mt[pos++];
@@ -243,18 +250,20 @@ __device__ __forceinline__ uint32_t mt_next(uint32_t* mt, int& pos, int lane) {
 }
 
 // CPython random(): (a * 2^26 + b) / 2^53 with a = 27 bits, b = 26 bits.
+template <int SPACE = 0>
 __device__ __forceinline__ double mt_random(uint32_t* mt, int& pos, int lane) {
-    const uint32_t a = mt_next(mt, pos, lane) >> 5;
-    const uint32_t b = mt_next(mt, pos, lane) >> 6;
+    const uint32_t a = mt_next<SPACE>(mt, pos, lane) >> 5;
+    const uint32_t b = mt_next<SPACE>(mt, pos, lane) >> 6;
     return ((double)a * 67108864.0 + (double)b) * (1.0 / 9007199254740992.0);
 }
 
 // CPython randrange(n), n >= 1: getrandbits(bit_length(n)) until < n.
 // Returns -1 if the (astronomically unlikely) rejection bound is hit.
+template <int SPACE = 0>
 __device__ __forceinline__ int mt_randrange(uint32_t* mt, int& pos, int lane, int n) {
     const int k = 32 - __clz(n);
     for (int tries = 0; tries < 4096; tries++) {
-        const uint32_t r = mt_next(mt, pos, lane) >> (32 - k);
+        const uint32_t r = mt_next<SPACE>(mt, pos, lane) >> (32 - k);
         if (r < (uint32_t)n) return (int)r;
     }
     return -1;
