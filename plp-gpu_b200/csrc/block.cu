@@ -350,11 +350,16 @@ __device__ __forceinline__ void block_body(const BlockArgs& a, unsigned char* ba
     unsigned char* fsr_base = base + lay.off_key;
 
     const int n_work = a.n_work_dev ? *a.n_work_dev : a.n_work;
+    const int n_dec = gridDim.x * (blockDim.x >> 5);   // decoders of the launch
+    int item = -1;
     for (;;) {
         if (*reinterpret_cast<volatile int*>(a.abort)) return;
-        int item = 0;
-        if (lane == 0) item = atomicAdd(a.work_next, 1);
-        item = __shfl_sync(FULL, item, 0);
+        if (item < 0) {   // the first item is the decoder's own number (see decoder1_body)
+            item = gdec;
+        } else {
+            if (lane == 0) item = n_dec + atomicAdd(a.work_next, 1);
+            item = __shfl_sync(FULL, item, 0);
+        }
         if (item >= n_work) break;
         const int2 wk = a.work[item];
         const InstDesc I = a.inst[wk.x];

@@ -1284,37 +1284,48 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
     constexpr bool SERVE = MODE != 0;
     constexpr int SPACE = MODE == 2 ? 1 : 0;   // the overflow decoders' tile is in global memory
     const int n_work = SERVE ? 0 : (a.n_work_dev ? *a.n_work_dev : a.n_work);
+    const int n_dec = gridDim.x * (blockDim.x >> 5);   // decoders of the launch
+    [[maybe_unused]] int item = -1;
 #pragma unroll 1
     for (;;) {
         if (*reinterpret_cast<volatile int*>(a.abort)) break;
         int2 wk;
         if constexpr (SERVE) {
-            int item = -1, wx = 0, wy = 0;
+            int sitem = -1, wx = 0, wy = 0;
             if (lane == 0) {
                 if constexpr (MODE == 1) {
-                    item = serve_claim(sv);
-                    if (item >= 0) {
-                        const int2 w = ld_relaxed_gpu_int2(sv.ring + (item & sv.ring_mask));
+                    sitem = serve_claim(sv);
+                    if (sitem >= 0) {
+                        const int2 w = ld_relaxed_gpu_int2(sv.ring + (sitem & sv.ring_mask));
                         wx = w.x;
                         wy = w.y;
                     }
                 } else {
-                    item = serve_claim_deep(sv);
+                    sitem = serve_claim_deep(sv);
                     int2 w = make_int2(0, 0);
-                    if (item >= 0 && !serve_deep_item(sv, item, &w)) {
+                    if (sitem >= 0 && !serve_deep_item(sv, sitem, &w)) {
                         atomicOr(a.err_flag, 1 << ERR_SYNC);   // a producer never finished its item
-                        item = -1;
+                        sitem = -1;
                     }
                     wx = w.x;
                     wy = w.y;
                 }
             }
-            if (__shfl_sync(FULL, item, 0) < 0) break;
+            if (__shfl_sync(FULL, sitem, 0) < 0) break;
             wk = make_int2(__shfl_sync(FULL, wx, 0), __shfl_sync(FULL, wy, 0));
         } else {
-            int item = 0;
-            if (lane == 0) item = atomicAdd(a.work_next, 1);
-            item = __shfl_sync(FULL, item, 0);
+            // The first item is the decoder's own number. Blocks of consecutive
+            // numbers lie on different SMs, so the longest items (first in the
+            // list) spread over the chip; the order in which blocks start, and
+            // would claim, fills a few SMs first (48 longest items on 12 to 21 of
+            // them, up to 8 on one). 61 batched instances x 48 restarts: 2.5 ms
+            // with every item claimed, 1.5 ms so.
+            if (item < 0) {
+                item = gdec;
+            } else {
+                if (lane == 0) item = n_dec + atomicAdd(a.work_next, 1);
+                item = __shfl_sync(FULL, item, 0);
+            }
             if (item >= n_work) break;
             wk = a.work[item];
         }
@@ -1954,8 +1965,8 @@ cudaError_t launch_gather_best(const InstDesc* inst, int n_inst, const int2* bes
 #endif  // PLP_SERVE_TU
 
 #ifdef PLP_SERVE_TU
-// Overflow decoders run out of line: with both bodies in one, the main
-// decoders' build for 18 per SM spilled 400 bytes and its code doubled.
+// Overflow decoders run out of line, so that the main decoders keep a body of
+// their own (158 registers instead of 170).
 static __device__ __noinline__ void serve_deep(const DecoderArgs& a, const ServeArgs& s, int gdec) {
     DecoderArgs ad = a;
     ad.P = s.deep_P;
@@ -1965,7 +1976,7 @@ static __device__ __noinline__ void serve_deep(const DecoderArgs& a, const Serve
 
 // The serving launch: the single-warp decoder over the host-published ring.
 template <int D, int M>
-__global__ void __launch_bounds__(32 * D, M == 16 ? 18 : M)
+__global__ void __launch_bounds__(32 * D, M)
     serve_kernel(const __grid_constant__ DecoderArgs a, const __grid_constant__ ServeArgs s) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int dec = threadIdx.x >> 5;
@@ -1980,7 +1991,7 @@ __global__ void __launch_bounds__(32 * D, M == 16 ? 18 : M)
 
 // ---- serving launches ------------------------------------------------------
 using ServeFn = void (*)(DecoderArgs, ServeArgs);
-#define PLP_SERVE_CONFIGS(X) X(1, 1) X(1, 12) X(1, 16)
+#define PLP_SERVE_CONFIGS(X) X(1, 1) X(1, 12)
 
 static ServeFn serve_fn(int D, int M) {
 #define PLP_PICK_SERVE(d, m) \
