@@ -181,7 +181,9 @@ void plp_destroy(plp_handle* h);
  * 160 registers, so three warps fit in each SM partition's register file
  * where 185 allow two. Restarts that outgrow the tile
  * are re-run with a deeper one, so the tile affects speed only, never results.
- * A new handle starts at P = 256, C = 512, G = 1, D = 1, M = 1. */
+ * Until a tile is set or tuned, each batch's tile follows from its sizes; a
+ * first call that leaves values out takes them from P = 256, C = 512, G = 1,
+ * D = 1, M = 1. */
 int plp_set_tile(plp_handle* h, int32_t P, int32_t C, int32_t G, int32_t D, int32_t M);
 
 /* Autotuner (no reference counterpart): times candidate tiles -- one warp per

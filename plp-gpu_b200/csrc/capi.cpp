@@ -94,9 +94,8 @@ void record(plp_handle* h, int status);
 // batch: device tables + one persistent decoder launch (+ retries)
 // ===========================================================================
 struct TileConfig {
-    // default: the tile the autotuner picks on every bench workload (one
-    // decoder per CTA spreads a launch over all SMs; these depths hold the
-    // 400-item instances without capacity retries)
+    // one decoder per CTA spreads a launch over all SMs; a handle whose tile was
+    // neither set nor tuned takes a tile per batch instead (auto_tile)
     int P = 256;       // placed-box tile depth per decoder
     int C = 512;       // live-point tile depth per decoder
     int G = 1;         // warps per decoder
@@ -378,6 +377,7 @@ struct Batch {
     std::vector<int2> work;
     long long n_slots = 0, n_places = 0;
     int max_stride = 1, max_steps = 0, Hz = 0;
+    long long sum_steps = 0, long_steps = 1;   // of all restarts and of the longest, over their passes
     bool multi_pass = false;
     // block-building engine: shape catalogue and per-instance orderings
     int engine = 0, max_types = 0;
@@ -430,6 +430,7 @@ struct Batch {
         engine = op.empty() ? 0 : op[0].engine;
         max_types = 0;
         n_slots = 0; n_places = 0; max_stride = 1; max_steps = 0; multi_pass = false;
+        sum_steps = 0; long_steps = 1;
         int maxH = 0;
         best_only = true;
         // item sequences and orientation tables of a large batch are built on
@@ -525,6 +526,11 @@ struct Batch {
             n_places += (long long)o.restarts * d.place_stride;
             max_stride = std::max(max_stride, d.place_stride);
             max_steps = std::max(max_steps, d.n_steps);
+            {
+                const long long s = (long long)d.n_steps * std::min(d.passes, 1 << 16);
+                sum_steps += s * o.restarts;
+                long_steps = std::max(long_steps, s);
+            }
             multi_pass = multi_pass || d.passes > 1;
             best_only = best_only && o.best_only;
             maxH = std::max(maxH, I.H);
@@ -605,6 +611,68 @@ cudaError_t tile_occupancy(const Batch& b, const TileConfig& t, int* occ) {
     if (b.engine == 1)
         return block_occupancy(t.P, t.C, std::max(1, b.max_steps), std::max(1, b.max_types), b.Hz, t.D, t.M, occ);
     return decoder_occupancy(t.P, t.C, b.Hz, t.G, t.D, t.M, occ);
+}
+
+// Deepest tile that a batch of this handle needed so far, when the tile is
+// chosen per batch: [0] batches of one wave, [1] of several.
+struct TileFloor {
+    int P[2] = {0, 0}, C[2] = {0, 0};
+};
+
+// The tile of a batch on a handle whose tile was neither set nor tuned.
+//  * Bound by its longest restart (the batch's steps spread over the resident
+//    decoders are fewer than the longest restart's): the uncapped build, which
+//    runs one restart fastest, and a tile that no restart outgrows (a pass
+//    places at most one box per step and holds about as many live points).
+//    1024 restarts of one instance: 0.294 ms, 0.314 with the M = 16 build; 61
+//    batched instances x 48: 1.24 ms against 1.43.
+//  * Otherwise M = 16, up to 21 decoders per SM: 2048 restarts of one instance
+//    0.407 ms, 0.522 with the uncapped build (13 per SM). While the batch fits
+//    one wave the deepest tile that keeps it there, since a restart that
+//    outgrows it runs again afterwards; in several waves 256 boxes and up to
+//    192 points, which about every restart fits (the device retry stage takes
+//    the others). 512 batched instances x 128 restarts: 7.15 ms at 160 points,
+//    8.49 at 128 and 8.18 at 96, where the stage runs a few restarts again.
+// The block engine has one build: 128 blocks, 384 points for several waves
+// (9.07 ms against 10.1 at 256, 512 for 512 instances x 64 restarts).
+TileConfig auto_tile(const Batch& b, int sms, const TileFloor& f, int* wave) {
+    const int steps = (std::max(1, b.max_steps) + 15) & ~15;
+    const int points = std::max(128, (steps + 63) & ~31);
+    // decoders the SMs hold at this tile, 0 when it does not run
+    auto resident = [&](const TileConfig& t) -> long long {
+        int occ = 0;
+        if (tile_smem(b, t) > 227 * 1024 || !tile_supported(b, t)) return 0;
+        if (tile_occupancy(b, t, &occ) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        return (long long)sms * occ;
+    };
+    struct Depth { int P, C, M; };
+    const Depth ep[] = {{std::min(steps, 512), std::min(points, 512), 1},
+                        {std::min(steps, 512), std::min(points, 256), 16},
+                        {std::min(steps, 256), std::min(points, 192), 16}};
+    const Depth blk[] = {{std::min(steps, 256), 512, 1}, {std::min(steps, 128), 384, 1}};
+    const Depth* d = b.engine == 1 ? blk : ep;
+    const int n = b.engine == 1 ? 2 : 3;
+    TileConfig t;
+    for (int k = 0; k < n; k++) {
+        t.P = d[k].P;
+        t.C = d[k].C;
+        t.M = d[k].M;
+        TileConfig w = t;
+        w.P = std::max(w.P, f.P[0]);
+        w.C = std::max(w.C, f.C[0]);
+        const long long r = resident(w);
+        if (b.n_slots <= r || (k == 0 && b.sum_steps <= r * b.long_steps)) {
+            *wave = 0;
+            return w;
+        }
+    }
+    t.P = std::max(t.P, f.P[1]);
+    t.C = std::max(t.C, f.C[1]);
+    *wave = 1;
+    return t;
 }
 
 // Fewer decoders per CTA when the tile plus this batch's top-z index (and,
@@ -1340,6 +1408,8 @@ struct plp_handle {
     size_t budget = 0;
     size_t in_use = 0;
     TileConfig tile;
+    bool tile_auto = true;            // no tile set or tuned: one per batch
+    TileFloor tile_floor;
     std::string err;
     std::mutex mu;
     std::condition_variable cv;       // request state changes
@@ -1375,6 +1445,43 @@ void record(plp_handle* h, int status) {
 }
 
 // rough device bytes of one request (tables + results + scratch share)
+// The tile a batch starts with, and what its run leaves for later ones.
+struct TilePick {
+    TileConfig tile;      // in: to use; out of an execution: to start the next one with
+    TileConfig first;
+    int wave = -1;        // -1: the handle's tile, else the floor it raises
+};
+
+TilePick pick_tile(plp_handle* h, const Batch& b) {
+    TilePick p;
+    TileFloor f;
+    bool autot;
+    {
+        std::lock_guard<std::mutex> lk(h->mu);
+        p.tile = h->tile;
+        f = h->tile_floor;
+        autot = h->tile_auto;
+    }
+    if (autot) {
+        const TileConfig keep = p.tile;
+        p.tile = auto_tile(b, h->sms, f, &p.wave);
+        p.tile.sync_limit = keep.sync_limit;
+        p.tile.sync_skip = keep.sync_skip;
+    }
+    p.first = p.tile;
+    return p;
+}
+
+void keep_tile(plp_handle* h, const TilePick& p) {
+    std::lock_guard<std::mutex> lk(h->mu);
+    if (p.wave < 0) {
+        remember_tile(h->tile, p.tile);
+        return;
+    }
+    if (p.tile.P > p.first.P) h->tile_floor.P[p.wave] = std::max(h->tile_floor.P[p.wave], p.tile.P);
+    if (p.tile.C > p.first.C) h->tile_floor.C[p.wave] = std::max(h->tile_floor.C[p.wave], p.tile.C);
+}
+
 size_t request_bytes(const Instance& I, const plp_run_opts& o) {
     const size_t steps = (size_t)std::max(1, I.n_items());
     return 4096 + I.types.size() * sizeof(TypeOrs) + steps * 4 +
@@ -1441,15 +1548,10 @@ void worker_main(plp_handle* h, int wi) {
         }
         const double t0 = now_seconds();
         int s = b.build(in, op);
-        TileConfig tile;
-        {
-            std::lock_guard<std::mutex> lk(h->mu);
-            tile = h->tile;
-        }
-        if (s == PLP_OK) s = run_batch(b, st, pin, h->sms, tile);
         if (s == PLP_OK) {
-            std::lock_guard<std::mutex> lk(h->mu);
-            remember_tile(h->tile, tile);
+            TilePick tile = pick_tile(h, b);
+            s = run_batch(b, st, pin, h->sms, tile.tile);
+            if (s == PLP_OK) keep_tile(h, tile);
         }
         std::vector<plp_result*> res;
         if (s == PLP_OK) res = collect(b, now_seconds() - t0);
@@ -1501,11 +1603,11 @@ void worker_main(plp_handle* h, int wi) {
 // SERVE_IDLE_STOP_S without requests and starts it again for the next one; a
 // decoder that finds no work for about a second exits by itself as well
 // (bounded polling). A request that the running launch's configuration cannot
-// take (a container taller than its top-z index covers, or footprints too
-// large for its 16-bit contact areas) waits until the launch has drained, and
-// the next launch takes the merged configuration. Restarts that overflow the
-// serving tile (P = 256 boxes, C = 768 live points; rare) make their request
-// run again on the wave path's code, which retries with deeper tiles.
+// take (a container taller than its top-z index covers) waits until the launch
+// has drained, and the next launch takes the merged configuration. Restarts
+// that overflow the serving tile (256 boxes, 256 live points, 12 decoders per
+// SM) go to the launch's overflow decoders; one that outgrows even their tile
+// makes its request run again on the wave path's code.
 constexpr int SERVE_RING = 1 << 20;            // work items in flight at most
 constexpr int SERVE_RECORDS = 1 << 16;         // requests in flight at most
 constexpr double SERVE_IDLE_STOP_S = 0.05;
@@ -1598,7 +1700,7 @@ size_t serve_align(size_t x, size_t unit) {    // a multiple of unit and of 128 
 }
 
 struct ServeConfig {
-    int P = 256, C = 512, D = 1, M = 12, Hz = 0;
+    int P = 256, C = 256, D = 1, M = 12, Hz = 0;
     int deep_P = 512, deep_C = 2048;   // the overflow decoders' tile (global memory)
     bool valid = false;
 };
@@ -1706,7 +1808,7 @@ struct ServeEngine {
         if (e == cudaSuccess) e = cudaMemset(dring, 0, sizeof(int4) * SERVE_RING);
         // PLP_SERVE_TILE=P,C,M: the main decoders' tile (M 1 or 12); taken
         // only if it fits one CTA's shared memory with the largest top-z
-        // index and 32-bit contact areas, so no later launch can fail on it
+        // index, so no later launch can fail on it
         if (const char* v = std::getenv("PLP_SERVE_TILE")) {
             int p = 0, c = 0, m = 0;
             if (std::sscanf(v, "%d,%d,%d", &p, &c, &m) == 3 && p >= 16 && p <= P_MAX && c >= 32 && c <= C_MAX &&
@@ -1967,15 +2069,13 @@ struct ServeEngine {
             cudaEventSynchronize(ev_kern);
             running = false;
         }
-        TileConfig tile;
-        {
-            std::lock_guard<std::mutex> lk(h->mu);
-            tile = h->tile;
-        }
         Batch b;
         const double t0 = now_seconds();
         int s = b.build({&j.inst}, {j.opts});
-        if (s == PLP_OK) s = run_batch(b, down, pin, sms, tile, &h->pool);
+        if (s == PLP_OK) {
+            TilePick tile = pick_tile(h, b);
+            s = run_batch(b, down, pin, sms, tile.tile, &h->pool);
+        }
         std::vector<plp_result*> res;
         if (s == PLP_OK) res = collect(b, now_seconds() - t0);
         complete(j, s, s == PLP_OK ? res[0] : nullptr, s == PLP_OK ? "" : g_err);
@@ -2652,6 +2752,7 @@ int plp_set_tile(plp_handle* h, int32_t P, int32_t C, int32_t G, int32_t D, int3
         return s;
     }
     h->tile = t;
+    h->tile_auto = false;
     return PLP_OK;
 }
 
@@ -2693,8 +2794,8 @@ int plp_autotune(plp_handle* h, const plp_instance* const* insts, int32_t n_inst
     std::vector<int> Ps, Cs;
     for (int p : {64, 128, 256})
         if (p <= P_MAX && (p >= std::min(max_steps, 64) || p == 128)) Ps.push_back(p);
-    for (int c : {256, 384, 512, 768}) Cs.push_back(c);
-    const int dm[][2] = {{1, 1}, {1, 12}, {1, 16}, {2, 1}, {4, 1}, {8, 1}, {8, 2}};
+    for (int c : {96, 160, 256, 512}) Cs.push_back(c);
+    const int dm[][2] = {{1, 1}, {1, 16}, {2, 1}, {8, 1}};
     std::vector<TileConfig> cand;
     for (int p : Ps)
         for (int c : Cs)
@@ -2752,6 +2853,7 @@ int plp_autotune(plp_handle* h, const plp_instance* const* insts, int32_t n_inst
     {
         std::lock_guard<std::mutex> lk(h->mu);
         h->tile = best;
+        h->tile_auto = false;
     }
     if (tile_out) {
         tile_out[0] = best.P; tile_out[1] = best.C; tile_out[2] = best.G; tile_out[3] = best.D; tile_out[4] = best.M;
@@ -2783,15 +2885,10 @@ int plp_solve(plp_handle* h, const plp_instance* const* insts, int32_t n_inst,
     const double t0 = now_seconds();
     Batch b;
     int s = b.build(in, op);
-    TileConfig tile;
-    {
-        std::lock_guard<std::mutex> lk(h->mu);
-        tile = h->tile;
-    }
-    if (s == PLP_OK) s = run_batch(b, h->sync_stream, h->sync_pin, h->sms, tile, &h->pool);
     if (s == PLP_OK) {
-        std::lock_guard<std::mutex> lk(h->mu);
-        remember_tile(h->tile, tile);
+        TilePick tile = pick_tile(h, b);
+        s = run_batch(b, h->sync_stream, h->sync_pin, h->sms, tile.tile, &h->pool);
+        if (s == PLP_OK) keep_tile(h, tile);
     }
     if (s != PLP_OK) {
         record(h, s);
@@ -2973,12 +3070,7 @@ int plp_batch_prepare(plp_handle* h, const plp_instance* const* insts, int32_t n
         op.push_back(opts[n_opts == 1 ? 0 : i]);
     }
     int s = pb->b.build(in, op);
-    TileConfig tile;
-    {
-        std::lock_guard<std::mutex> lk(h->mu);
-        tile = h->tile;
-    }
-    if (s == PLP_OK) s = batch_prepare(pb->b, h->sync_stream, h->sync_pin, h->sms, tile, false);
+    if (s == PLP_OK) s = batch_prepare(pb->b, h->sync_stream, h->sync_pin, h->sms, pick_tile(h, pb->b).tile, false);
     if (s != PLP_OK) {
         record(h, s);
         return s;
@@ -2993,21 +3085,14 @@ int plp_batch_run(plp_batch* pb, double* device_ms, double* decoder_ms, int32_t*
     serve_yield(h);
     std::lock_guard<std::mutex> g(h->sync_mu);
     cudaSetDevice(h->device);
-    TileConfig tile;
-    {
-        std::lock_guard<std::mutex> lk(h->mu);
-        tile = h->tile;
-    }
+    TilePick tile = pick_tile(h, pb->b);
     ExecStats x;
-    int s = batch_execute(pb->b, h->sync_stream, h->sms, tile, &x, true);
+    int s = batch_execute(pb->b, h->sync_stream, h->sms, tile.tile, &x, true);
     if (s != PLP_OK) {
         record(h, s);
         return s;
     }
-    {
-        std::lock_guard<std::mutex> lk(h->mu);
-        remember_tile(h->tile, tile);
-    }
+    keep_tile(h, tile);
     pb->executed = true;
     if (device_ms) *device_ms = x.device_ms;
     if (decoder_ms) *decoder_ms = x.decoder_ms;
