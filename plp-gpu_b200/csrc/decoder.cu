@@ -1687,14 +1687,20 @@ __global__ void fsr_kernel(const int* __restrict__ rows7, const int* __restrict_
     char* scratch = reinterpret_cast<char*>(base + ((26 * cap + 15) & ~15));
     const int o0 = offsets[pk];
     const int n = offsets[pk + 1] - o0;
-    // insertion by rank on top z (ties by index) gives the sorted order
+    // insertion by rank on top z (ties by index) gives the sorted order; the
+    // tops are ranked in shared memory (the rows may lie in host memory)
+    int* tops = reinterpret_cast<int*>(scratch);
     for (int i = lane; i < n; i += 32) {
         const int* r = rows7 + 7 * (o0 + i);
-        const int t = r[3] + r[6];
+        tops[i] = r[3] + r[6];
+    }
+    __syncwarp();
+    for (int i = lane; i < n; i += 32) {
+        const int* r = rows7 + 7 * (o0 + i);
+        const int t = tops[i];
         int rank = 0;
         for (int j = 0; j < n; j++) {
-            const int* q = rows7 + 7 * (o0 + j);
-            const int tj = q[3] + q[6];
+            const int tj = tops[j];
             rank += tj < t || (tj == t && j < i);
         }
         bx[rank] = make_int4(r[1], r[2], r[1] + r[4], r[2] + r[5]);

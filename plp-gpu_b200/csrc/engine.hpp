@@ -113,10 +113,8 @@ cudaError_t launch_fsr(const int* rows7, const int* offsets, int n_pack, int cap
 cudaError_t launch_item_order(const long long* vols, const int* qty, const int* type_off,
                               const int* n_types, const long long* step_off, int n_inst, int order,
                               int* out_types, int sort_cap, cudaStream_t st);
-// one-step feasibility (kernel a); first_out (optional) receives the smallest
-// feasible pair index (atomicMin; caller initialises it to INT_MAX)
+// one-step feasibility (kernel a)
 cudaError_t launch_feas(const int* cand, int n_cand, const int* ors, int n_ors, const int* fast6,
-                        int n_fast, int L, int W, int H, unsigned char* bits, int* first_out,
-                        cudaStream_t st);
+                        int n_fast, int L, int W, int H, unsigned char* bits, cudaStream_t st);
 
 }  // namespace plpb
