@@ -143,6 +143,7 @@ struct BlockTables {
     // offsets into tab
     int bo_order = 0, bo_qty = 0, bo_list_off = 0, bo_list = 0, bo_start_off = 0, bo_start = 0,
         bo_shape_of_rank = 0;
+    int xw = 1, xd = 1, xh = 1;   // largest block edges
     size_t bytes() const { return cat.size() * sizeof(BlkShape) + tab.size() * sizeof(int); }
 };
 
@@ -196,6 +197,11 @@ int make_block_tables(const Instance& I, const std::vector<TypeOrs>& ors, int am
         return p.b > q.b;
     });
     for (int r = 0; r < nc; r++) cat[by_rank[r]].rank = r;
+    for (const BlkShape& c : cat) {
+        d.xw = std::max(d.xw, c.bw);
+        d.xd = std::max(d.xd, c.bd);
+        d.xh = std::max(d.xh, c.bh);
+    }
     std::vector<int> tord(nt);
     for (int t = 0; t < nt; t++) tord[t] = t;
     std::sort(tord.begin(), tord.end(), [&](int x, int y) {
@@ -312,6 +318,9 @@ int build_block_tables(const Instance& I, const std::vector<TypeOrs>& ors, const
     d.n_cat = (int)bt->cat.size();
     tab.insert(tab.end(), bt->tab.begin(), bt->tab.end());
     cat_all.insert(cat_all.end(), bt->cat.begin(), bt->cat.end());
+    d.xw = bt->xw;
+    d.xd = bt->xd;
+    d.xh = bt->xh;
     d.blk_topk = std::max(1, o.blk_topk);
     d.blk_pick = o.blk_pick;
     if (tab.size() > (size_t)INT_MAX / 2 || cat_all.size() > (size_t)INT_MAX / 2)
@@ -540,7 +549,7 @@ struct Batch {
         // a table of seeded states pays when at least two restarts share each seed
         seed_lo = 0;
         seed_n = 0;
-        if (engine == 0 && !desc.empty()) {
+        if (!desc.empty()) {
             long long lo = LLONG_MAX, hi = LLONG_MIN;
             for (const auto& d : desc) {
                 lo = std::min(lo, d.seed);
@@ -633,8 +642,8 @@ struct TileFloor {
 //    192 points, which about every restart fits (the device retry stage takes
 //    the others). 512 batched instances x 128 restarts: 7.15 ms at 160 points,
 //    8.49 at 128 and 8.18 at 96, where the stage runs a few restarts again.
-// The block engine has one build: 128 blocks, 384 points for several waves
-// (9.07 ms against 10.1 at 256, 512 for 512 instances x 64 restarts).
+// The block engine has one build: 128 blocks, 192 points for several waves (512
+// instances x 64 restarts: 3.2 ms; about 9 % more at 256, 512).
 TileConfig auto_tile(const Batch& b, int sms, const TileFloor& f, int* wave) {
     const int steps = (std::max(1, b.max_steps) + 15) & ~15;
     const int points = std::max(128, (steps + 63) & ~31);
@@ -652,7 +661,7 @@ TileConfig auto_tile(const Batch& b, int sms, const TileFloor& f, int* wave) {
     const Depth ep[] = {{std::min(steps, 512), std::min(points, 512), 1},
                         {std::min(steps, 512), std::min(points, 256), 16},
                         {std::min(steps, 256), std::min(points, 192), 16}};
-    const Depth blk[] = {{std::min(steps, 256), 512, 1}, {std::min(steps, 128), 384, 1}};
+    const Depth blk[] = {{std::min(steps, 256), 512, 1}, {std::min(steps, 128), 192, 1}};
     const Depth* d = b.engine == 1 ? blk : ep;
     const int n = b.engine == 1 ? 2 : 3;
     TileConfig t;

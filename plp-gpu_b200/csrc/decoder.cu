@@ -46,6 +46,7 @@
 //    full count / idx-th selection runs only on the random branch.
 #include "device_common.cuh"
 #include "engine.hpp"
+#include "ep_state.cuh"
 #include "feas_eval.cuh"
 #include "fsr_warp.cuh"
 
@@ -831,11 +832,6 @@ __device__ __forceinline__ unsigned z_within(const Edges& E, int v) {
     return (E.l <= v ? 0x03u : 0u) | (E.w <= v ? 0x0cu : 0u) | (E.h <= v ? 0x30u : 0u);
 }
 
-// First box with top >= z: from the top-z index, or by search without one.
-__device__ __forceinline__ int top_start(const unsigned short* zt, const uint4* bx, int nb, int z) {
-    return zt ? (int)zt[z] : first_top(PackedBoxes{bx}, nb, z);
-}
-
 // Slots of `cand` whose C3 holds at (x, y, z), z > 0: contact with the boxes
 // [j, je), whose top is z. Areas are at most the container's footprint, below
 // 2^31, so twice an area fits 32 unsigned bits.
@@ -889,214 +885,6 @@ __device__ __forceinline__ unsigned blocked_slots(int x, int y, int z, int j0, i
         }
     }
     return __reduce_or_sync(FULL, blk & 0x3fu);
-}
-
-// Smallest and largest edges over the instance's orientations (InstDesc) and
-// the container.
-struct EdgeRange {
-    int w, d, h;      // smallest along x, y, z
-    int Mw, Md, Mh;   // largest
-    int L, W, H;
-};
-
-constexpr uint32_t PT_MARKED = 1u << 16;   // z extent word: a box meets the extents' cuboid
-
-// A new box's corner coordinates (px .. px2 and so on) and the far ends of the
-// smallest-edge cuboid at them. Sets of corners are eight-bit masks over
-// c = (z2 << 2) | (y2 << 1) | x2.
-struct CornerFrame {
-    int x, y, z, x2, y2, z2;
-    int xm, ym, zm, x2m, y2m, z2m;
-    // How a placed box lies to the corners, a byte each from the low end: the
-    // corners whose x extent it ends, whose y extent, whose z extent, and
-    // those it reaches past on every axis. Corners whose cuboid it meets are
-    // added to dead.
-    __device__ __forceinline__ uint32_t relate(const uint4& v, unsigned& dead) const {
-        const int bx2 = (int)(v.x >> 16), by2 = (int)(v.y >> 16), bt = (int)(v.z >> 16);
-        const int bx = (int)(v.x & 0xffffu), by = (int)(v.y & 0xffffu), bz = (int)(v.z & 0xffffu);
-        const bool ax = x < bx2, ax2 = x2 < bx2, ay = y < by2, ay2 = y2 < by2, az = z < bt, az2 = z2 < bt;
-        const unsigned xa = (ax ? 0x55u : 0u) | (ax2 ? 0xaau : 0u), ya = (ay ? 0x33u : 0u) | (ay2 ? 0xccu : 0u),
-                       za = (az ? 0x0fu : 0u) | (az2 ? 0xf0u : 0u);
-        const unsigned xi = xa & ((bx < xm ? 0x55u : 0u) | (bx < x2m ? 0xaau : 0u)),
-                       yi = ya & ((by < ym ? 0x33u : 0u) | (by < y2m ? 0xccu : 0u)),
-                       zi = za & ((bz < zm ? 0x0fu : 0u) | (bz < z2m ? 0xf0u : 0u));
-        dead |= xi & yi & zi;
-        return (xa & yi & zi) | (xi & ya & zi) << 8 | (xi & yi & za) << 16 | (xa & ya & za) << 24;
-    }
-};
-
-// Warp: places a w x d x h box at the point with key pkey: top-sorted box
-// tables, top-z index, and the points K (arrays of `cap` entries: key,
-// x | y << 16 extents, z extent | mark): the box is applied to every point,
-// dead ones give up their slots, and the box's live corners come in.
-__device__ __forceinline__ int place1(uint32_t pkey, int pw, int pd, int ph, uint32_t* K, int cap,
-                                      unsigned short* free_slots, uint4* bx,
-                                      unsigned short* zt, int Hz, int& nc, int& nb, int P, int C, uint32_t xmask,
-                                      uint32_t ymask, int xb, int xyb, const EdgeRange& ME, int lane) {
-    const int px = (int)(pkey & xmask), py = (int)((pkey >> xb) & ymask), pz = (int)(pkey >> xyb);
-    const int px2 = px + pw, py2 = py + pd, pz2 = pz + ph;
-    if (nb >= P) return ERR_BOX_CAP;
-    // Box tables, one pass from the top: how each placed box lies to the new
-    // box's corners, and the boxes whose top is above the new box's move up
-    // one slot (each round reads before it writes, and writes only slots it or
-    // an earlier round has read). The two top rounds stay in registers for the
-    // corners' extents.
-    const CornerFrame F{px, py, pz, px2, py2, pz2, px + ME.w, py + ME.d, pz + ME.h, px2 + ME.w, py2 + ME.d, pz2 + ME.h};
-    unsigned dead = 1u;   // corner 0 = (px, py, pz): inside the new box
-    if (F.x2m > ME.L) dead |= 0xaau;
-    if (F.y2m > ME.W) dead |= 0xccu;
-    if (F.z2m > ME.H) dead |= 0xf0u;
-    int nabove = 0;
-    const int nb0 = nb;
-    uint4 wb[2];
-    uint32_t wm[2] = {0u, 0u};
-#pragma unroll
-    for (int r = 0; r < 3; r++) {
-        // rounds 0 and 1 keep their box; round 2 stands for all below them
-#pragma unroll 1
-        for (int hi = nb0 - 32 * r; hi > 0; hi -= 32) {
-            const int jj = hi - 1 - lane;
-            const bool in = jj >= 0;
-            const uint4 v = in ? bx[jj] : make_uint4(0, 0, 0, 0);   // the empty box lies before every corner
-            const uint32_t m = F.relate(v, dead);
-            const bool up = in && (int)(v.z >> 16) > pz2;
-            nabove += __popc(__ballot_sync(FULL, up));
-            __syncwarp();
-            if (up) bx[jj + 1] = v;
-            if (r < 2) {
-                wb[r] = v;
-                wm[r] = m;
-                break;
-            }
-        }
-    }
-    unsigned live = ~__reduce_or_sync(FULL, dead) & 0xffu;
-    {
-        const int ip = nb - nabove;   // after the boxes with equal tops
-        __syncwarp();
-        if (lane == 0) {
-            bx[ip] = make_uint4((uint32_t)px | (uint32_t)px2 << 16, (uint32_t)py | (uint32_t)py2 << 16,
-                                (uint32_t)pz | (uint32_t)pz2 << 16, (uint32_t)nb);
-        }
-    }
-    if (zt) {
-        // entries above the new top, two to a word (counts stay below 2^16), four words a lane in flight
-        const int z0 = pz2 + 1;
-        if ((z0 & 1) && lane == 0) zt[z0]++;
-        uint32_t* zw = reinterpret_cast<uint32_t*>(zt);
-#pragma unroll 1
-        for (int w = ((z0 + 1) >> 1) + lane; w < Hz >> 1; w += 128) {
-            uint32_t v[4];
-#pragma unroll
-            for (int u = 0; u < 4; u++) v[u] = w + 32 * u < Hz >> 1 ? zw[w + 32 * u] : 0u;
-#pragma unroll
-            for (int u = 0; u < 4; u++)
-                if (w + 32 * u < Hz >> 1) zw[w + 32 * u] = v[u] + 0x10001u;
-        }
-    }
-    nb++;
-    // Points in place. A corner whose key a point already has is not new.
-    const uint32_t ck = ((uint32_t)((lane & 4) ? pz2 : pz) << xyb) | ((uint32_t)((lane & 2) ? py2 : py) << xb) |
-                        (uint32_t)((lane & 1) ? px2 : px);
-    int nf = 0;            // slots freed
-    unsigned dup = 0;      // corners this lane has met
-#pragma unroll 1
-    for (int cb = 0; cb < nc; cb += 32) {
-        const int i = cb + lane;
-        const bool in = i < nc;
-        const uint32_t key = in ? K[i] : 0u, exy = in ? K[cap + i] : 0u, ezm = in ? K[2 * cap + i] : 0u;
-        int ex = (int)(exy & 0xffffu), ey = (int)(exy >> 16), ez = (int)(ezm & 0xffffu);
-        uint32_t mark = ezm & PT_MARKED;
-        const int x = (int)(key & xmask), y = (int)((key >> xb) & ymask), z = (int)(key >> xyb);
-        const bool ax = x < px2, ay = y < py2, az = z < pz2;
-        const bool ix = ax && px < x + ME.w, iy = ay && py < y + ME.d, iz = az && pz < z + ME.h;
-        if (iy && iz && ax) ex = min(ex, px - x);
-        if (ix && iz && ay) ey = min(ey, py - y);
-        if (ix && iy && az) ez = min(ez, pz - z);
-        if (ax && ay && az && px < x + ex && py < y + ey && pz < z + ez) mark = PT_MARKED;
-        const bool gone = in && (ex < ME.w || ey < ME.d || ez < ME.h);
-        if (in) {
-            K[cap + i] = gone ? 0u : (uint32_t)ex | ((uint32_t)ey << 16);
-            K[2 * cap + i] = (uint32_t)ez | mark;
-        }
-        if ((x == px || x == px2) && (y == py || y == py2) && (z == pz || z == pz2))
-            dup |= 1u << ((x == px2 ? 1 : 0) | (y == py2 ? 2 : 0) | (z == pz2 ? 4 : 0));
-        const unsigned fr = __ballot_sync(FULL, gone);
-        if (fr) {
-            const int q = nf + __popc(fr & lanemask_lt());
-            if (gone && q < 32) free_slots[q] = (unsigned short)i;
-            nf += __popc(fr);
-        }
-    }
-    // (Lanes past the end read key 0, the container's corner: never a live corner.)
-    live &= ~__reduce_or_sync(FULL, dup);
-    __syncwarp();   // box tables, top-z index, points and freed slots are final
-    // The n-th live corner takes the n-th freed slot, or one past the end; the
-    // last point fills a slot left over. Slots past the 32nd freed in one
-    // placement keep their dead point, which the next placement frees again.
-    nf = min(nf, 32);
-    const int nl = __popc(live);
-    const int nth = __popc(live & ((1u << (lane & 7)) - 1u));
-    const int slot = nth < nf ? (int)free_slots[nth] : nc + nth - nf;
-#pragma unroll 1
-    for (int q = nf - 1; q >= nl; q--) {   // from the highest slot: the last point is alive or in it
-        const int h = free_slots[q];
-        nc--;
-        if (h != nc && lane < 3) K[lane * cap + h] = K[lane * cap + nc];
-        __syncwarp();
-    }
-    nc += max(nl - nf, 0);
-    if (nc > C) return ERR_CAND_CAP;
-    // Extents of the new corners: the boxes in registers, then any below them
-    // from the tables (their old slots [0, nb0 - 64) now lie within
-    // [0, nb0 - 64]; a box met twice, or the new one, changes nothing).
-#pragma unroll 1
-    for (unsigned mc = live; mc; mc &= mc - 1) {
-        const int c = __ffs(mc) - 1;
-        const int x = (c & 1) ? px2 : px, y = (c & 2) ? py2 : py, z = (c & 4) ? pz2 : pz;
-        int ex = min(ME.L - x, ME.Mw), ey = min(ME.W - y, ME.Md), ez = min(ME.H - z, ME.Mh);
-#pragma unroll
-        for (int r = 0; r < 2; r++) {
-            if (32 * r < nb0) {
-                const uint32_t m = wm[r] >> c;
-                if (m & 1u) ex = min(ex, (int)(wb[r].x & 0xffffu) - x);
-                if (m & 0x100u) ey = min(ey, (int)(wb[r].y & 0xffffu) - y);
-                if (m & 0x10000u) ez = min(ez, (int)(wb[r].z & 0xffffu) - z);
-            }
-        }
-        const int j0 = nb0 > 64 ? top_start(zt, bx, nb, z + 1) : nb;
-#pragma unroll 1
-        for (int j = j0 + lane; j <= nb0 - 64; j += 32) {
-            const int4 b = PackedBoxes{bx}.xy(j);
-            const int bz = PackedBoxes{bx}.bottom(j);
-            const bool ix = b.x < x + ME.w && x < b.z, iy = b.y < y + ME.d && y < b.w, iz = bz < z + ME.h;
-            if (iy && iz && x < b.z) ex = min(ex, b.x - x);
-            if (ix && iz && y < b.w) ey = min(ey, b.y - y);
-            if (ix && iy) ez = min(ez, bz - z);
-        }
-        ex = __reduce_min_sync(FULL, ex);
-        ey = __reduce_min_sync(FULL, ey);
-        ez = __reduce_min_sync(FULL, ez);
-        bool meets = false;
-#pragma unroll
-        for (int r = 0; r < 2; r++)
-            if (32 * r < nb0)
-                meets = meets || (((wm[r] >> c) & 0x1000000u) && (int)(wb[r].x & 0xffffu) < x + ex &&
-                                  (int)(wb[r].y & 0xffffu) < y + ey && (int)(wb[r].z & 0xffffu) < z + ez);
-#pragma unroll 1
-        for (int j = j0 + lane; j <= nb0 - 64; j += 32) {
-            const int4 b = PackedBoxes{bx}.xy(j);
-            meets = meets || (b.x < x + ex && x < b.z && b.y < y + ey && y < b.w && PackedBoxes{bx}.bottom(j) < z + ez);
-        }
-        const uint32_t mark = __any_sync(FULL, meets) ? PT_MARKED : 0u;
-        if (lane == c) {
-            K[slot] = ck;
-            K[cap + slot] = (uint32_t)ex | ((uint32_t)ey << 16);
-            K[2 * cap + slot] = (uint32_t)ez | mark;
-        }
-    }
-    __syncwarp();
-    return ERR_NONE;
 }
 
 // ---------------------------------------------------------------------------
