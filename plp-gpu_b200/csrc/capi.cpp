@@ -297,34 +297,49 @@ std::shared_ptr<const BlockTables> block_tables(const Instance& I, const std::ve
     return bt;
 }
 
-// Appends one instance's block tables to the batch's catalogue and table,
-// with its descriptor's offsets.
-int build_block_tables(const Instance& I, const std::vector<TypeOrs>& ors, const plp_run_opts& o,
-                       std::vector<BlkShape>& cat_all, std::vector<int>& tab, InstDesc& d) {
-    int status = PLP_OK;
-    const auto bt = block_tables(I, ors, std::max(1, o.blk_amax), std::max(1, o.blk_bmax),
-                                 std::max(1, o.blk_kmax), &status);
-    if (!bt) return status;
-    const int base = (int)tab.size();
+// Runs fn(k) for k in [0, n) on up to 16 threads, `grain` at a time.
+template <class F>
+void parallel_for(size_t n, size_t grain, const F& fn) {
+    const unsigned hw = std::thread::hardware_concurrency();
+    const size_t nt = std::min<size_t>(std::max(1u, std::min(16u, hw ? hw : 1u)), (n + grain - 1) / grain);
+    std::atomic<size_t> next{0};
+    auto job = [&] {
+        for (size_t i0; (i0 = next.fetch_add(grain)) < n;)
+            for (size_t k = i0; k < std::min(n, i0 + grain); k++) fn(k);
+    };
+    std::vector<std::thread> pool;
+    for (size_t t = 1; t < nt; t++) pool.emplace_back(job);
+    job();
+    for (auto& th : pool) th.join();
+}
+
+std::shared_ptr<const BlockTables> block_tables(const Instance& I, const std::vector<TypeOrs>& ors,
+                                                const plp_run_opts& o, int* status) {
+    return block_tables(I, ors, std::max(1, o.blk_amax), std::max(1, o.blk_bmax), std::max(1, o.blk_kmax), status);
+}
+
+// One instance's descriptor entries for block tables that start at `cat` and
+// `tab` of the batch's.
+int place_block_tables(const BlockTables& bt, const Instance& I, const plp_run_opts& o, size_t cat, size_t tab,
+                       InstDesc& d) {
+    if (tab + bt.tab.size() > (size_t)INT_MAX / 2 || cat + bt.cat.size() > (size_t)INT_MAX / 2)
+        return set_error(PLP_E_CAPACITY, "block tables too large for one batch");
+    const int base = (int)tab;
     d.n_types = (int)I.types.size();
-    d.bo_order = base + bt->bo_order;
-    d.bo_qty = base + bt->bo_qty;
-    d.bo_list_off = base + bt->bo_list_off;
-    d.bo_list = base + bt->bo_list;
-    d.bo_start_off = base + bt->bo_start_off;
-    d.bo_start = base + bt->bo_start;
-    d.bo_shape_of_rank = base + bt->bo_shape_of_rank;
-    d.cat_off = (int)cat_all.size();
-    d.n_cat = (int)bt->cat.size();
-    tab.insert(tab.end(), bt->tab.begin(), bt->tab.end());
-    cat_all.insert(cat_all.end(), bt->cat.begin(), bt->cat.end());
-    d.xw = bt->xw;
-    d.xd = bt->xd;
-    d.xh = bt->xh;
+    d.bo_order = base + bt.bo_order;
+    d.bo_qty = base + bt.bo_qty;
+    d.bo_list_off = base + bt.bo_list_off;
+    d.bo_list = base + bt.bo_list;
+    d.bo_start_off = base + bt.bo_start_off;
+    d.bo_start = base + bt.bo_start;
+    d.bo_shape_of_rank = base + bt.bo_shape_of_rank;
+    d.cat_off = (int)cat;
+    d.n_cat = (int)bt.cat.size();
+    d.xw = bt.xw;
+    d.xd = bt.xd;
+    d.xh = bt.xh;
     d.blk_topk = std::max(1, o.blk_topk);
     d.blk_pick = o.blk_pick;
-    if (tab.size() > (size_t)INT_MAX / 2 || cat_all.size() > (size_t)INT_MAX / 2)
-        return set_error(PLP_E_CAPACITY, "block tables too large for one batch");
     return PLP_OK;
 }
 
@@ -395,8 +410,9 @@ struct Batch {
     // seeds seed_lo .. seed_lo + seed_n - 1, or seed_n = 0 to seed in place
     long long seed_lo = 0;
     int seed_n = 0;
-    std::vector<BlkShape> bcat;
-    std::vector<int> btab;
+    // the instances' block tables, one behind the other in the upload
+    std::vector<std::shared_ptr<const BlockTables>> blk;
+    size_t n_bcat = 0, n_btab = 0;
     // device
     char* d_mem = nullptr;
     size_t bytes = 0;
@@ -435,7 +451,8 @@ struct Batch {
         insts = in;
         opts = op;
         desc.clear(); steps.clear(); types.clear(); work.clear(); inst_ors.clear();
-        bcat.clear(); btab.clear();
+        blk.clear();
+        n_bcat = n_btab = 0;
         engine = op.empty() ? 0 : op[0].engine;
         max_types = 0;
         n_slots = 0; n_places = 0; max_stride = 1; max_steps = 0; multi_pass = false;
@@ -446,23 +463,19 @@ struct Batch {
         // several threads; the rest of the build is appends in instance order
         std::vector<std::vector<int>> seqs;
         std::vector<std::vector<TypeOrs>> ors;
-        if (in.size() >= 256) {
+        // (an instance's first block tables take about 0.35 ms, so those are
+        // spread from a few instances on)
+        if (engine == 1) blk.resize(in.size());
+        if (in.size() >= (engine == 1 ? 8u : 256u)) {
             seqs.resize(in.size());
             ors.resize(in.size());
-            const unsigned hw = std::thread::hardware_concurrency();
-            const int nt = (int)std::max(1u, std::min(16u, hw ? hw : 1u));
-            std::atomic<size_t> next{0};
-            auto job = [&] {
-                for (size_t i0; (i0 = next.fetch_add(64)) < in.size();)
-                    for (size_t k = i0; k < std::min(in.size(), i0 + 64); k++) {
-                        if (op[k].order == 0 || op[k].order == 1) seqs[k] = item_sequence(*in[k], op[k].order);
-                        ors[k] = type_orientations(*in[k]);
-                    }
-            };
-            std::vector<std::thread> pool;
-            for (int t = 1; t < nt; t++) pool.emplace_back(job);
-            job();
-            for (auto& th : pool) th.join();
+            parallel_for(in.size(), engine == 1 ? 4 : 64, [&](size_t k) {
+                if (op[k].order == 0 || op[k].order == 1) seqs[k] = item_sequence(*in[k], op[k].order);
+                ors[k] = type_orientations(*in[k]);
+                int status = PLP_OK;
+                if (engine == 1 && op[k].engine == 1 && in[k]->types.size() <= 2048)
+                    blk[k] = block_tables(*in[k], ors[k], op[k], &status);   // a failure is met again below
+            });
         }
         {
             size_t n_types = 0, n_steps = 0;
@@ -527,8 +540,13 @@ struct Batch {
             desc.back().n_types = (int)I.types.size();
             max_types = std::max(max_types, (int)I.types.size());
             if (o.engine == 1) {
-                const int sb = build_block_tables(I, ot, o, bcat, btab, desc.back());
+                int sb = PLP_OK;
+                if (!blk[i]) blk[i] = block_tables(I, ot, o, &sb);
                 if (sb != PLP_OK) return sb;
+                sb = place_block_tables(*blk[i], I, o, n_bcat, n_btab, desc.back());
+                if (sb != PLP_OK) return sb;
+                n_bcat += blk[i]->cat.size();
+                n_btab += blk[i]->tab.size();
             }
             inst_ors.push_back(std::move(ot));
             n_slots += o.restarts;
@@ -588,8 +606,8 @@ struct Batch {
         o_desc = o;    o = al(o + desc.size() * sizeof(InstDesc));
         o_steps = o;   o = al(o + std::max<size_t>(1, steps.size()) * sizeof(int));
         o_types = o;   o = al(o + std::max<size_t>(1, types.size()) * sizeof(TypeOrs));
-        o_bcat = o;    o = al(o + std::max<size_t>(1, bcat.size()) * sizeof(BlkShape));
-        o_btab = o;    o = al(o + std::max<size_t>(1, btab.size()) * sizeof(int));
+        o_bcat = o;    o = al(o + std::max<size_t>(1, n_bcat) * sizeof(BlkShape));
+        o_btab = o;    o = al(o + std::max<size_t>(1, n_btab) * sizeof(int));
         o_work = o;    o = al(o + work.size() * sizeof(int2));
         // counters and flags: [0] work counter, [4] retry-stage work counter,
         // [8] error flag, [12] abort, [16] retry-stage error flag, [20] retry count
@@ -892,8 +910,15 @@ int batch_prepare(Batch& b, cudaStream_t st, Pinned& pin, int sms, const TileCon
     std::memcpy(pin.p + b.o_desc, b.desc.data(), b.desc.size() * sizeof(InstDesc));
     std::memcpy(pin.p + b.o_steps, b.steps.data(), b.steps.size() * sizeof(int));
     std::memcpy(pin.p + b.o_types, b.types.data(), b.types.size() * sizeof(TypeOrs));
-    if (!b.bcat.empty()) std::memcpy(pin.p + b.o_bcat, b.bcat.data(), b.bcat.size() * sizeof(BlkShape));
-    if (!b.btab.empty()) std::memcpy(pin.p + b.o_btab, b.btab.data(), b.btab.size() * sizeof(int));
+    // block tables straight from the kept ones (tens of MB in a large batch)
+    if (!b.blk.empty())
+        parallel_for(b.blk.size(), std::max<size_t>(16, b.blk.size() / 8), [&](size_t k) {
+            const BlockTables& t = *b.blk[k];
+            std::memcpy(pin.p + b.o_bcat + (size_t)b.desc[k].cat_off * sizeof(BlkShape), t.cat.data(),
+                        t.cat.size() * sizeof(BlkShape));
+            std::memcpy(pin.p + b.o_btab + (size_t)(b.desc[k].bo_order - t.bo_order) * sizeof(int), t.tab.data(),
+                        t.tab.size() * sizeof(int));
+        });
     std::memcpy(pin.p + b.o_work, b.work.data(), b.work.size() * sizeof(int2));
     e = cudaMemcpyAsync(b.d_mem, pin.p, up, cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return fail("batch upload", e);
