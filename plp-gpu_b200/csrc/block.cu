@@ -193,7 +193,7 @@ __device__ __forceinline__ void block_body(const BlockArgs& a, unsigned char* ba
         unsigned long long* pass_out =
             I.passes > 1 ? a.scratch + (long long)gdec * a.scratch_stride : best_out;
         int mpos = 624;
-        {
+        if (randomized) {   // else no draw is ever made
             const long long sd = I.seed + restart;
             if (a.seed_tab && sd >= a.seed_lo && sd - a.seed_lo < a.seed_n) {
                 const uint4* src = reinterpret_cast<const uint4*>(a.seed_tab + (sd - a.seed_lo) * 624);

@@ -1124,11 +1124,12 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
         const uint32_t xmask = (1u << I.xb) - 1u, ymask = (1u << I.yb) - 1u;
         const int xb = I.xb, xyb = I.xb + I.yb;
         const bool randomized = !(I.first_fit || I.eps == 0.0);
+        const unsigned long long random_from = mt_threshold(1.0 - I.eps);
         unsigned long long* best_out = a.places + I.place_off + (long long)restart * I.place_stride;
         unsigned long long* pass_out =
             I.passes > 1 ? a.scratch + (long long)gdec * a.scratch_stride : best_out;
         int mpos = 624;
-        {
+        if (randomized) {   // else no draw is ever made
             const long long sd = I.seed + restart;
             if (!SERVE && a.seed_tab && sd >= a.seed_lo && sd - a.seed_lo < a.seed_n) {
                 // the seeded state, computed once for every restart of the batch with this seed
@@ -1220,45 +1221,68 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
                     nW += __popc(bal);
                 }
                 __syncwarp();
-                // feasible set of every item: C3, then C1 of the marked ones. The
-                // first feasible point is the one with the smallest key.
-                uint32_t best_key = 0xffffffffu;   // of this lane's items
-                unsigned best_set = 0;
-                int count = 0;
+                // C3 of every item
 #pragma unroll 1
-                for (int w0 = 0; w0 < nW; w0 += 32) {
-                    const uint2 e = w0 + lane < nW ? Wl[w0 + lane] : make_uint2(0, 0);
+                for (int w = lane; w < nW; w += 32) {
+                    const uint2 e = Wl[w];
                     unsigned cand = e.y & 0x3fu;
                     const int z = (int)(e.x >> xyb);
-                    if (z > 0 && cand) {
+                    if (z > 0) {
                         const int j = top_start(zt, bx, nb, z), je = top_start(zt, bx, nb, z + 1);
                         cand = support_slots(cand, (int)(e.x & xmask), (int)((e.x >> xb) & ymask), j, je, E, bx);
                     }
-                    __syncwarp();
-#pragma unroll 1
-                    for (unsigned bal = __ballot_sync(FULL, cand && (e.y & 0x80u)); bal; bal &= bal - 1) {
-                        const int q = __ffs(bal) - 1;
-                        const uint32_t kq = __shfl_sync(FULL, e.x, q);
-                        const int zq = (int)(kq >> xyb);
-                        const unsigned blk = blocked_slots((int)(kq & xmask), (int)((kq >> xb) & ymask), zq,
-                                                           top_start(zt, bx, nb, zq + 1), nb, E, bx, lane);
-                        if (lane == q) cand &= ~blk;
-                    }
-                    const int c = __popc(cand);
-                    count += c;
-                    if (cand && e.x < best_key) {
-                        best_key = e.x;
-                        best_set = cand;
-                    }
-                    if (w0 + lane < nW) Wl[w0 + lane].y = cand | (unsigned)c << 8;
+                    Wl[w].y = cand ? cand | (e.y & 0x80u) : 0u;
                 }
-                uint32_t pick_key = __reduce_min_sync(FULL, best_key);
+                __syncwarp();
+                // The first feasible point is the one with the smallest key, once C1
+                // holds there if it is marked. On the random branch every feasible
+                // pair counts, so C1 of the marked items left follows.
+                uint32_t pick_key = 0xffffffffu;
+                unsigned pick_set = 0;
+                bool full = false;
+#pragma unroll 1
+                for (;;) {
+                    uint32_t key = 0xffffffffu;
+                    unsigned set = 0;
+                    int at = 0;
+#pragma unroll 1
+                    for (int w = lane; w < nW; w += 32) {
+                        const uint2 e = Wl[w];
+                        if ((full ? e.y & 0x80u : e.y) && e.x < key) {
+                            key = e.x;
+                            set = e.y;
+                            at = w;
+                        }
+                    }
+                    const uint32_t k = __reduce_min_sync(FULL, key);
+                    if (k == 0xffffffffu) break;
+                    const bool mine = key == k;
+                    set = __shfl_sync(FULL, set, __ffs(__ballot_sync(FULL, mine)) - 1);
+                    if (!(set & 0x80u)) {
+                        pick_key = k;
+                        pick_set = set;
+                        // random() only once a feasible pair exists
+                        full = randomized && mt_random53<SPACE>(mt, mpos, lane) >= random_from;
+                        if (!full) break;
+                    } else {
+                        const int z = (int)(k >> xyb);
+                        set &= 0x3fu & ~blocked_slots((int)(k & xmask), (int)((k >> xb) & ymask), z,
+                                                      top_start(zt, bx, nb, z + 1), nb, E, bx, lane);
+                        if (mine) Wl[at].y = set;
+                        __syncwarp();
+                    }
+                }
                 stuck = pick_key == 0xffffffffu;
                 if (stuck) continue;                     // no feasible pair: no draw
                 from_key = pick_key;
-                unsigned pick_set = __shfl_sync(FULL, best_set, __ffs(__ballot_sync(FULL, best_key == pick_key)) - 1);
-                // random() only once a feasible pair exists
-                if (randomized && mt_random<SPACE>(mt, mpos, lane) >= 1.0 - I.eps) {
+                if (full) {
+                    int count = 0;   // each item's pairs, beside its slots
+#pragma unroll 1
+                    for (int w = lane; w < nW; w += 32) {
+                        const unsigned m = Wl[w].y;
+                        count += __popc(m);
+                        Wl[w].y = m | (unsigned)__popc(m) << 8;
+                    }
                     const int idx = mt_randrange<SPACE>(mt, mpos, lane, __reduce_add_sync(FULL, count));
                     if (idx < 0) {
                         err = ERR_RNG;
@@ -1396,7 +1420,8 @@ __global__ void __launch_bounds__(32 * D, M == 16 ? 18 : M) decoder1_kernel(Deco
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int dec = threadIdx.x >> 5;
     const Dec1Layout lay = dec1_layout(a.P, a.C, a.Hz);
-    decoder1_body<0>(a, smem_raw + (size_t)dec * lay.bytes, blockIdx.x * D + dec, ServeArgs{});
+    unsigned char* base = smem_raw + (size_t)dec * lay.bytes;
+    decoder1_body<0>(a, base, blockIdx.x * D + dec, ServeArgs{});
 }
 
 
@@ -1775,12 +1800,10 @@ __global__ void __launch_bounds__(32 * D, M)
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int dec = threadIdx.x >> 5;
     const int gdec = blockIdx.x * D + dec;
-    if (gdec < s.n_deep) {
-        serve_deep(a, s, gdec);
-    } else {
-        const Dec1Layout lay = dec1_layout(a.P, a.C, a.Hz);
-        decoder1_body<1>(a, smem_raw + (size_t)dec * lay.bytes, gdec, s);
-    }
+    const Dec1Layout lay = dec1_layout(a.P, a.C, a.Hz);
+    unsigned char* base = smem_raw + (size_t)dec * lay.bytes;
+    if (gdec < s.n_deep) serve_deep(a, s, gdec);
+    else decoder1_body<1>(a, base, gdec, s);
 }
 
 // ---- serving launches ------------------------------------------------------

@@ -257,6 +257,21 @@ __device__ __forceinline__ double mt_random(uint32_t* mt, int& pos, int lane) {
     return ((double)a * 67108864.0 + (double)b) * (1.0 / 9007199254740992.0);
 }
 
+// The same draw as the integer random() * 2^53, and the least such integer that
+// is at or above t * 2^53: random() >= t exactly when the draw reaches it (the
+// scaling by 2^53 and the ceiling are exact). Spares the FP64 pipe a
+// conversion and a product on each draw.
+template <int SPACE = 0>
+__device__ __forceinline__ unsigned long long mt_random53(uint32_t* mt, int& pos, int lane) {
+    const uint32_t a = mt_next<SPACE>(mt, pos, lane) >> 5;
+    const uint32_t b = mt_next<SPACE>(mt, pos, lane) >> 6;
+    return ((unsigned long long)a << 26) | b;
+}
+__device__ __forceinline__ unsigned long long mt_threshold(double t) {
+    if (!(t <= 1.0)) return ~0ull;   // above every draw; NaN compares false
+    return t <= 0.0 ? 0ull : (unsigned long long)ceil(t * 9007199254740992.0);
+}
+
 // CPython randrange(n), n >= 1: getrandbits(bit_length(n)) until < n.
 // Returns -1 if the (astronomically unlikely) rejection bound is hit.
 template <int SPACE = 0>

@@ -38,12 +38,13 @@ struct CornerFrame {
     __device__ __forceinline__ uint32_t relate(const uint4& v, unsigned& dead) const {
         const int bx2 = (int)(v.x >> 16), by2 = (int)(v.y >> 16), bt = (int)(v.z >> 16);
         const int bx = (int)(v.x & 0xffffu), by = (int)(v.y & 0xffffu), bz = (int)(v.z & 0xffffu);
-        const bool ax = x < bx2, ax2 = x2 < bx2, ay = y < by2, ay2 = y2 < by2, az = z < bt, az2 = z2 < bt;
-        const unsigned xa = (ax ? 0x55u : 0u) | (ax2 ? 0xaau : 0u), ya = (ay ? 0x33u : 0u) | (ay2 ? 0xccu : 0u),
-                       za = (az ? 0x0fu : 0u) | (az2 ? 0xf0u : 0u);
-        const unsigned xi = xa & ((bx < xm ? 0x55u : 0u) | (bx < x2m ? 0xaau : 0u)),
-                       yi = ya & ((by < ym ? 0x33u : 0u) | (by < y2m ? 0xccu : 0u)),
-                       zi = za & ((bz < zm ? 0x0fu : 0u) | (bz < z2m ? 0xf0u : 0u));
+        // (reaching past the far corner implies reaching past the near one, and
+        // beginning before the near end implies before the far one)
+        const unsigned xa = x2 < bx2 ? 0xffu : x < bx2 ? 0x55u : 0u, ya = y2 < by2 ? 0xffu : y < by2 ? 0x33u : 0u,
+                       za = z2 < bt ? 0xffu : z < bt ? 0x0fu : 0u;
+        const unsigned xi = xa & (bx < xm ? 0xffu : bx < x2m ? 0xaau : 0u),
+                       yi = ya & (by < ym ? 0xffu : by < y2m ? 0xccu : 0u),
+                       zi = za & (bz < zm ? 0xffu : bz < z2m ? 0xf0u : 0u);
         dead |= xi & yi & zi;
         return (xa & yi & zi) | (xi & ya & zi) << 8 | (xi & yi & za) << 16 | (xa & ya & za) << 24;
     }
@@ -72,26 +73,24 @@ __device__ __forceinline__ int place1(uint32_t pkey, int pw, int pd, int ph, uin
     if (F.z2m > ME.H) dead |= 0xf0u;
     int nabove = 0;
     const int nb0 = nb;
-    uint4 wb[2];
-    uint32_t wm[2] = {0u, 0u};
-#pragma unroll
-    for (int r = 0; r < 3; r++) {
-        // rounds 0 and 1 keep their box; round 2 stands for all below them
+    uint4 wb0 = make_uint4(0, 0, 0, 0), wb1 = wb0;
+    uint32_t wm0 = 0, wm1 = 0;
 #pragma unroll 1
-        for (int hi = nb0 - 32 * r; hi > 0; hi -= 32) {
-            const int jj = hi - 1 - lane;
-            const bool in = jj >= 0;
-            const uint4 v = in ? bx[jj] : make_uint4(0, 0, 0, 0);   // the empty box lies before every corner
-            const uint32_t m = F.relate(v, dead);
-            const bool up = in && (int)(v.z >> 16) > pz2;
-            nabove += __popc(__ballot_sync(FULL, up));
-            __syncwarp();
-            if (up) bx[jj + 1] = v;
-            if (r < 2) {
-                wb[r] = v;
-                wm[r] = m;
-                break;
-            }
+    for (int r = 0; 32 * r < nb0; r++) {
+        const int jj = nb0 - 32 * r - 1 - lane;
+        const bool in = jj >= 0;
+        const uint4 v = in ? bx[jj] : make_uint4(0, 0, 0, 0);   // the empty box lies before every corner
+        const uint32_t m = F.relate(v, dead);
+        const bool up = in && (int)(v.z >> 16) > pz2;
+        nabove += __popc(__ballot_sync(FULL, up));
+        __syncwarp();
+        if (up) bx[jj + 1] = v;
+        if (r == 0) {
+            wb0 = v;
+            wm0 = m;
+        } else if (r == 1) {
+            wb1 = v;
+            wm1 = m;
         }
     }
     unsigned live = ~__reduce_or_sync(FULL, dead) & 0xffu;
@@ -133,7 +132,7 @@ __device__ __forceinline__ int place1(uint32_t pkey, int pw, int pd, int ph, uin
         uint32_t mark = ezm & PT_MARKED;
         const int x = (int)(key & xmask), y = (int)((key >> xb) & ymask), z = (int)(key >> xyb);
         const bool ax = x < px2, ay = y < py2, az = z < pz2;
-        const bool ix = ax && px < x + ME.w, iy = ay && py < y + ME.d, iz = az && pz < z + ME.h;
+        const bool ix = ax && x > px - ME.w, iy = ay && y > py - ME.d, iz = az && z > pz - ME.h;
         if (iy && iz && ax) ex = min(ex, px - x);
         if (ix && iz && ay) ey = min(ey, py - y);
         if (ix && iy && az) ez = min(ez, pz - z);
@@ -181,12 +180,11 @@ __device__ __forceinline__ int place1(uint32_t pkey, int pw, int pd, int ph, uin
         int ex = min(ME.L - x, ME.Mw), ey = min(ME.W - y, ME.Md), ez = min(ME.H - z, ME.Mh);
 #pragma unroll
         for (int r = 0; r < 2; r++) {
-            if (32 * r < nb0) {
-                const uint32_t m = wm[r] >> c;
-                if (m & 1u) ex = min(ex, (int)(wb[r].x & 0xffffu) - x);
-                if (m & 0x100u) ey = min(ey, (int)(wb[r].y & 0xffffu) - y);
-                if (m & 0x10000u) ez = min(ez, (int)(wb[r].z & 0xffffu) - z);
-            }
+            const uint4 v = r ? wb1 : wb0;
+            const uint32_t m = (r ? wm1 : wm0) >> c;
+            if (m & 1u) ex = min(ex, (int)(v.x & 0xffffu) - x);
+            if (m & 0x100u) ey = min(ey, (int)(v.y & 0xffffu) - y);
+            if (m & 0x10000u) ez = min(ez, (int)(v.z & 0xffffu) - z);
         }
         const int j0 = nb0 > 64 ? top_start(zt, bx, nb, z + 1) : nb;
 #pragma unroll 1
@@ -203,10 +201,11 @@ __device__ __forceinline__ int place1(uint32_t pkey, int pw, int pd, int ph, uin
         ez = __reduce_min_sync(FULL, ez);
         bool meets = false;
 #pragma unroll
-        for (int r = 0; r < 2; r++)
-            if (32 * r < nb0)
-                meets = meets || (((wm[r] >> c) & 0x1000000u) && (int)(wb[r].x & 0xffffu) < x + ex &&
-                                  (int)(wb[r].y & 0xffffu) < y + ey && (int)(wb[r].z & 0xffffu) < z + ez);
+        for (int r = 0; r < 2; r++) {
+            const uint4 v = r ? wb1 : wb0;
+            meets = meets || ((((r ? wm1 : wm0) >> c) & 0x1000000u) && (int)(v.x & 0xffffu) < x + ex &&
+                              (int)(v.y & 0xffffu) < y + ey && (int)(v.z & 0xffffu) < z + ez);
+        }
 #pragma unroll 1
         for (int j = j0 + lane; j <= nb0 - 64; j += 32) {
             const int4 b = PackedBoxes{bx}.xy(j);
