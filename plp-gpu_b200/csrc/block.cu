@@ -553,10 +553,12 @@ cudaError_t configure_block(const DecodeLaunch& L) {
 cudaError_t enqueue_block(const DecodeLaunch& L, cudaStream_t st) {
     BlockFn fn = block_fn(L.decoders_per_cta, L.min_blocks);
     if (!fn) return cudaErrorInvalidConfiguration;
-    cudaError_t e = cudaMemsetAsync(L.work_next, 0, sizeof(int), st);
-    if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(L.abort, 0, sizeof(int), st);
-    if (e != cudaSuccess) return e;
+    if (!L.zeroed) {
+        cudaError_t e = cudaMemsetAsync(L.work_next, 0, sizeof(int), st);
+        if (e != cudaSuccess) return e;
+        e = cudaMemsetAsync(L.abort, 0, sizeof(int), st);
+        if (e != cudaSuccess) return e;
+    }
     BlockArgs a;
     a.inst = L.inst;
     a.types = L.types;

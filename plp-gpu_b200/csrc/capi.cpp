@@ -426,6 +426,7 @@ struct Batch {
     int2* h_redo_stage(size_t n) { redo_host.resize(n); return redo_host.data(); }
     size_t scratch_bytes = 0;
     int ctas = 0;
+    bool counters_zero = false;            // uploaded as zeros and not used yet
     TileConfig tile;
     // one-graph replay of a clean execution (flag reset, decoder, flag copy,
     // select, gather), kept for later executions with the same tile
@@ -593,6 +594,7 @@ struct Batch {
         return PLP_OK;
     }
 
+    static constexpr size_t COUNTER_BYTES = 32;
     static size_t al(size_t v) { return (v + 255) & ~size_t(255); }
 
     void plan(int sms, const TileConfig& t) {
@@ -610,11 +612,12 @@ struct Batch {
         o_btab = o;    o = al(o + std::max<size_t>(1, n_btab) * sizeof(int));
         o_work = o;    o = al(o + work.size() * sizeof(int2));
         // counters and flags: [0] work counter, [4] retry-stage work counter,
-        // [8] error flag, [12] abort, [16] retry-stage error flag, [20] retry count
-        o_next = o;    o = al(o + 32);
+        // [8] error flag, [12] abort, [16] retry-stage error flag, [20] retry count.
+        // Results follow them, so one copy brings flags and results back.
+        o_next = o;    o = al(o + COUNTER_BYTES);
         o_heads = o;   o = al(o + n_slots * sizeof(SlotHead));
-        o_places = o;  o = al(o + std::max<long long>(1, n_places) * 8);
         o_best = o;    o = al(o + desc.size() * sizeof(int2));
+        o_places = o;  o = al(o + std::max<long long>(1, n_places) * 8);
         o_gather = o;  o = al(o + desc.size() * (size_t)max_stride * 8);
         o_scratch = o; o = al(o + std::max<size_t>(8, scratch_bytes));
         o_redo = o;    o = al(o + work.size() * sizeof(int2));
@@ -622,7 +625,7 @@ struct Batch {
         bytes = o;
     }
 
-    size_t upload_bytes() const { return o_next; }   // desc .. work are contiguous at the front
+    size_t upload_bytes() const { return o_next; }   // desc .. work are contiguous at the front, then the counters
 };
 
 int tile_smem(const Batch& b, const TileConfig& t) {
@@ -846,7 +849,8 @@ struct ExecStats {
     long long redo_wave = 0;      // resident decoders of the retry stage's tile
 };
 
-int batch_release(Batch& b, cudaStream_t st) {
+// drained: the stream has been synchronised after the batch's last operation.
+int batch_release(Batch& b, cudaStream_t st, bool drained = false) {
     if (b.gexec) {
         cudaGraphExecDestroy(b.gexec);
         b.gexec = nullptr;
@@ -858,7 +862,7 @@ int batch_release(Batch& b, cudaStream_t st) {
     cudaError_t e = cudaSuccess;
     if (b.d_mem) e = cudaFreeAsync(b.d_mem, st);
     b.d_mem = nullptr;
-    cudaError_t e2 = cudaStreamSynchronize(st);
+    cudaError_t e2 = drained ? cudaSuccess : cudaStreamSynchronize(st);
     if (b.own_ctx) {
         for (auto& ev : b.ev)
             if (ev) cudaEventDestroy(ev);
@@ -904,8 +908,8 @@ int batch_prepare(Batch& b, cudaStream_t st, Pinned& pin, int sms, const TileCon
     }
     e = cudaMallocAsync(&b.d_mem, b.bytes, st);
     if (e != cudaSuccess) return fail("batch allocation", e);
-    const size_t up = b.upload_bytes();
-    e = pin.ensure(std::max(up, (size_t)1));
+    const size_t up = b.upload_bytes() + Batch::COUNTER_BYTES;   // the counters go in as zeros
+    e = pin.ensure(up);
     if (e != cudaSuccess) return fail("pinned staging", e);
     std::memcpy(pin.p + b.o_desc, b.desc.data(), b.desc.size() * sizeof(InstDesc));
     std::memcpy(pin.p + b.o_steps, b.steps.data(), b.steps.size() * sizeof(int));
@@ -920,8 +924,10 @@ int batch_prepare(Batch& b, cudaStream_t st, Pinned& pin, int sms, const TileCon
                         t.tab.size() * sizeof(int));
         });
     std::memcpy(pin.p + b.o_work, b.work.data(), b.work.size() * sizeof(int2));
+    std::memset(pin.p + b.o_next, 0, Batch::COUNTER_BYTES);
     e = cudaMemcpyAsync(b.d_mem, pin.p, up, cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return fail("batch upload", e);
+    b.counters_zero = true;
     e = launch_seed_table(b.seed_lo, b.seed_n, b.mt_init, reinterpret_cast<uint32_t*>(b.d_mem + b.o_seedtab), st);
     if (e != cudaSuccess) return fail("seed table", e);
     // the staging buffer is reused by the next batch of this thread
@@ -1140,23 +1146,25 @@ void batch_capture(Batch& b, cudaStream_t st, int sms, const TileConfig& t) {
     cudaGetLastError();
 }
 
-// Host destination of a batch's results: [slot heads | best per instance |
-// packed placements (all slots, or the gathered best per instance)]. With a
-// pool, a pooled pinned block that the results keep; else a pageable block,
-// staged through the thread's pinned buffer when it is large enough (that
-// buffer is reused by the thread's next batch, so it is copied out).
+// Host destination of a batch's results: the device's bytes from the counters
+// to the end of [slot heads | best per instance | packed placements], or of a
+// best-only batch [slot heads | best per instance] and the gathered best
+// placements behind them. With a pool, a pooled pinned block that the results
+// keep; else a pageable block, staged through the thread's pinned buffer when
+// it is large enough (that buffer is reused by the thread's next batch, so it
+// is copied out).
 struct ResultCopy {
     std::shared_ptr<char> blk;
     char* dst = nullptr;
     char* stage = nullptr;
-    size_t hb = 0, bb = 0, pb = 0;
+    size_t front = 0;     // bytes from the counters on
+    size_t gather = 0;    // best-only: bytes of the gathered placements, behind them
 };
 
 int result_dst(const Batch& b, Pinned* pin, const std::shared_ptr<HostPool>* pool, ResultCopy& rc) {
-    rc.hb = b.n_slots * sizeof(SlotHead);
-    rc.bb = b.desc.size() * sizeof(int2);
-    rc.pb = b.best_only ? b.desc.size() * (size_t)b.max_stride * 8 : (size_t)b.n_places * 8;
-    const size_t total = rc.hb + rc.bb + rc.pb;
+    rc.front = (b.best_only ? b.o_best + b.desc.size() * sizeof(int2) : b.o_places + (size_t)b.n_places * 8) - b.o_next;
+    rc.gather = b.best_only ? b.desc.size() * (size_t)b.max_stride * 8 : 0;
+    const size_t total = Batch::al(rc.front) + rc.gather;
     if (pool && *pool) rc.blk = pool_take(*pool, total);
     if (!rc.blk) {
         if (pin && pin->p && total <= pin->cap) rc.stage = pin->p;
@@ -1168,21 +1176,21 @@ int result_dst(const Batch& b, Pinned* pin, const std::shared_ptr<HostPool>* poo
 }
 
 cudaError_t result_enqueue(const Batch& b, const ResultCopy& rc, cudaStream_t st) {
-    cudaError_t e = cudaMemcpyAsync(rc.dst, b.d_mem + b.o_heads, rc.hb, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(rc.dst + rc.hb, b.d_mem + b.o_best, rc.bb, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess && rc.pb)
-        e = cudaMemcpyAsync(rc.dst + rc.hb + rc.bb, b.d_mem + (b.best_only ? b.o_gather : b.o_places), rc.pb,
-                            cudaMemcpyDeviceToHost, st);
+    cudaError_t e = cudaMemcpyAsync(rc.dst, b.d_mem + b.o_next, rc.front, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess && rc.gather)
+        e = cudaMemcpyAsync(rc.dst + Batch::al(rc.front), b.d_mem + b.o_gather, rc.gather, cudaMemcpyDeviceToHost, st);
     return e;
 }
 
 // after the copies completed: the batch's results view the block
 void result_take(Batch& b, ResultCopy& rc) {
-    if (rc.stage) std::memcpy(rc.blk.get(), rc.stage, rc.hb + rc.bb + rc.pb);
+    if (rc.stage) std::memcpy(rc.blk.get(), rc.stage, Batch::al(rc.front) + rc.gather);
     b.host = std::move(rc.blk);
-    b.heads_ptr = reinterpret_cast<const SlotHead*>(b.host.get());
-    b.best_ptr = reinterpret_cast<const int2*>(b.host.get() + rc.hb);
-    b.places_ptr = reinterpret_cast<const unsigned long long*>(b.host.get() + rc.hb + rc.bb);
+    const char* p = b.host.get();
+    b.heads_ptr = reinterpret_cast<const SlotHead*>(p + (b.o_heads - b.o_next));
+    b.best_ptr = reinterpret_cast<const int2*>(p + (b.o_best - b.o_next));
+    b.places_ptr = reinterpret_cast<const unsigned long long*>(
+        p + (b.best_only ? Batch::al(rc.front) : b.o_places - b.o_next));
 }
 
 // tile: in = tile to use, out = tile to start the next execution with (deeper
@@ -1237,33 +1245,44 @@ int batch_execute(Batch& b, cudaStream_t st, int sms, TileConfig& tile, ExecStat
     // restarts below and select again
     TileConfig deep;
     const bool staged = redo_stage(b, t, sms, &deep, &x.redo_wave);
-    cudaError_t e = cudaMemsetAsync(d_flag, 0, 16, st);
+    // freshly uploaded counters are zero; the events only serve the caller's statistics
+    const bool zeroed = b.counters_zero;
+    b.counters_zero = false;
+    cudaError_t e = zeroed ? cudaSuccess : cudaMemsetAsync(d_flag, 0, 16, st);
     if (e != cudaSuccess) return fail("flag reset", e);
-    e = cudaEventRecord(b.ev[0], st);
-    if (e == cudaSuccess) e = launch_decoder(make_launch(b, t, d_work, (int)b.work.size(), sms), st);
-    if (e == cudaSuccess) e = cudaEventRecord(b.ev[1], st);
+    if (xs) e = cudaEventRecord(b.ev[0], st);
+    if (e == cudaSuccess) {
+        DecodeLaunch L = make_launch(b, t, d_work, (int)b.work.size(), sms);
+        L.zeroed = zeroed;
+        e = launch_decoder(L, st);
+    }
+    if (e == cudaSuccess && xs) e = cudaEventRecord(b.ev[1], st);
     if (e != cudaSuccess) return fail("decoder launch", e);
     x.launches++;
     if (staged) {
-        const DecodeLaunch L2 = redo_launch(b, deep, sms);
+        DecodeLaunch L2 = redo_launch(b, deep, sms);
+        L2.zeroed = zeroed;
         e = configure_decoder(L2);
         if (e == cudaSuccess) e = enqueue_redo(b, L2, sms, st, &x.launches);
         if (e != cudaSuccess) return fail("retry stage launch", e);
     }
-    e = cudaMemcpyAsync(b.h_flag, d_flag, 16, cudaMemcpyDeviceToHost, st);
-    if (e != cudaSuccess) return fail("flag copy", e);
+    if (!rc) {   // else the flags come with the results
+        e = cudaMemcpyAsync(b.h_flag, d_flag, 16, cudaMemcpyDeviceToHost, st);
+        if (e != cudaSuccess) return fail("flag copy", e);
+    }
     {
         int n = 0;
         e = enqueue_select(b, st, &n);
         x.launches += n;
         if (e != cudaSuccess) return fail("select launch", e);
     }
-    e = cudaEventRecord(b.ev[2], st);
+    if (xs) e = cudaEventRecord(b.ev[2], st);
     if (e == cudaSuccess && rc) e = result_enqueue(b, *rc, st);   // valid unless host retries follow
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return fail("decoder", e);
+    if (rc) std::memcpy(b.h_flag, rc->dst + 8, 16);
     float ms = 0;
-    cudaEventElapsedTime(&ms, b.ev[0], b.ev[1]);
+    if (xs) cudaEventElapsedTime(&ms, b.ev[0], b.ev[1]);
     x.decoder_ms = ms;
     const int staged_count = staged ? fl[3] : 0;
     x.redo = staged_count;
@@ -1322,12 +1341,12 @@ int batch_execute(Batch& b, cudaStream_t st, int sms, TileConfig& tile, ExecStat
         e = enqueue_select(b, st, &n);
         x.launches += n;
         if (e != cudaSuccess) return fail("select launch", e);
-        e = cudaEventRecord(b.ev[2], st);
+        if (xs) e = cudaEventRecord(b.ev[2], st);
         if (e == cudaSuccess && rc) e = result_enqueue(b, *rc, st);   // again, after the retries
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) return fail("select", e);
     }
-    cudaEventElapsedTime(&ms, b.ev[0], b.ev[2]);
+    if (xs) cudaEventElapsedTime(&ms, b.ev[0], b.ev[2]);
     x.device_ms = ms;
     if (graph && !retried) batch_capture(b, st, sms, t);
     if (staged) {
@@ -1386,7 +1405,7 @@ int run_batch(Batch& b, cudaStream_t st, Pinned& pin, int sms, TileConfig& tile,
     s = batch_execute(b, st, sms, tile, nullptr, false, &rc);   // results copied in the same pass
     if (s != PLP_OK) return s;
     result_take(b, rc);
-    return batch_release(b, st);
+    return batch_release(b, st, true);
 }
 
 // Builds the per-instance result objects of a finished batch; they view the
@@ -3198,9 +3217,8 @@ int plp_decode_noalloc(const plp_instance* inst, const plp_run_opts* opts, void*
     t.C = std::min(C_MAX, ((1 + 7 * steps) + 31) & ~31);
     t.G = 1;
     t.M = 1;
-    t.D = 8;
-    while (t.D > 1 && decoder_smem_bytes(t.P, t.C, b.Hz, t.G) * t.D > 200 * 1024) t.D >>= 1;
-    if (t.P > P_MAX || decoder_smem_bytes(t.P, t.C, b.Hz, t.G) * t.D > 227 * 1024 || 1 + 7 * steps > C_MAX)
+    t.D = 1;   // spread over the SMs
+    if (t.P > P_MAX || decoder_smem_bytes(t.P, t.C, b.Hz, t.G) > 227 * 1024 || 1 + 7 * steps > C_MAX)
         return set_error(PLP_E_CAPACITY, "plp_decode_noalloc: instance too large for the shared-memory tile");
     // scratch: the address is set up on the first call on each device
     void* scr = nullptr;
@@ -3211,6 +3229,10 @@ int plp_decode_noalloc(const plp_instance* inst, const plp_run_opts* opts, void*
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     e = decoder_occupancy(t.P, t.C, b.Hz, t.G, t.D, t.M, &occ);
+    if (e == cudaSuccess && b.n_slots > (long long)sms * std::max(occ, 1)) {   // several waves: more decoders per SM
+        t.M = 16;
+        e = decoder_occupancy(t.P, t.C, b.Hz, t.G, t.D, t.M, &occ);
+    }
     if (e != cudaSuccess) return set_cuda_error("plp_decode_noalloc: occupancy", e);
     occ = std::max(occ, 1);
     long long ctas = std::max<long long>(1, std::min<long long>((b.n_slots + t.D - 1) / t.D, (long long)sms * occ));
@@ -3245,6 +3267,7 @@ int plp_decode_noalloc(const plp_instance* inst, const plp_run_opts* opts, void*
     L.work = reinterpret_cast<const int2*>(d + o_work);
     L.n_work = (int)b.work.size();
     L.work_next = reinterpret_cast<int*>(d + o_flags);
+    L.zeroed = true;
     L.err_flag = reinterpret_cast<int*>(d + o_flags + 8);
     L.abort = reinterpret_cast<int*>(d + o_flags + 12);
     L.heads = static_cast<SlotHead*>(d_heads);

@@ -1683,10 +1683,12 @@ cudaError_t enqueue_decoder(const DecodeLaunch& L, cudaStream_t st) {
     if (L.engine == 1) return enqueue_block(L, st);
     DecoderFn fn = decoder_fn(L.warps_per_decoder, L.decoders_per_cta, L.min_blocks);
     if (!fn) return cudaErrorInvalidConfiguration;
-    cudaError_t e = cudaMemsetAsync(L.work_next, 0, sizeof(int), st);
-    if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(L.abort, 0, sizeof(int), st);
-    if (e != cudaSuccess) return e;
+    if (!L.zeroed) {
+        cudaError_t e = cudaMemsetAsync(L.work_next, 0, sizeof(int), st);
+        if (e != cudaSuccess) return e;
+        e = cudaMemsetAsync(L.abort, 0, sizeof(int), st);
+        if (e != cudaSuccess) return e;
+    }
     fn<<<L.ctas, 32 * L.warps_per_decoder * L.decoders_per_cta, decoder_launch_smem(L), st>>>(decoder_args(L));
     return cudaGetLastError();
 }

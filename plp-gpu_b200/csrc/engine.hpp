@@ -15,6 +15,7 @@ struct DecodeLaunch {
     int n_work;
     const int* n_work_dev;    // set: the work count is read here at kernel start (n_work bounds it)
     int* work_next;
+    bool zeroed;              // work_next and abort are already zero
     int* err_flag;            // OR of (1 << err) over restarts that failed
     int* abort;               // set when a bounded barrier wait gives up
     SlotHead* heads;
