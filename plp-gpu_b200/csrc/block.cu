@@ -152,6 +152,22 @@ static __device__ __noinline__ void blk_contact(int x0, int y0, int z0, int bw, 
     side = si;
 }
 
+// The engine draws at five places of its loop; out of line, its code stays short.
+struct MtDraw {
+    unsigned long long v;
+    MtPos p;
+};
+static __device__ __noinline__ MtDraw blk_random53(uint32_t* mt, MtPos p, int lane) {
+    MtDraw d{0, p};
+    d.v = mt_random53(mt, d.p, lane);
+    return d;
+}
+static __device__ __noinline__ MtDraw blk_randrange(uint32_t* mt, MtPos p, int lane, int n) {
+    MtDraw d{0, p};
+    d.v = (unsigned long long)(long long)mt_randrange(mt, d.p, lane, n);
+    return d;
+}
+
 __device__ __forceinline__ void block_body(const BlockArgs& a, unsigned char* base, int gdec) {
     const int lane = threadIdx.x & 31;
     const BlkLayout lay = blk_layout(a.P, a.C, a.N, a.T, a.Hz);
@@ -192,7 +208,18 @@ __device__ __forceinline__ void block_body(const BlockArgs& a, unsigned char* ba
         unsigned long long* best_out = a.places + I.place_off + (long long)restart * I.place_stride;
         unsigned long long* pass_out =
             I.passes > 1 ? a.scratch + (long long)gdec * a.scratch_stride : best_out;
-        int mpos = 624;
+        MtPos mpos{MT_WORDS, 0u};
+        const unsigned long long random_from = mt_threshold(1.0 - I.eps);
+        auto draw53 = [&] {
+            const MtDraw d = blk_random53(mt, mpos, lane);
+            mpos = d.p;
+            return d.v;
+        };
+        auto draw_below = [&](int n) {
+            const MtDraw d = blk_randrange(mt, mpos, lane, n);
+            mpos = d.p;
+            return (int)d.v;
+        };
         if (randomized) {   // else no draw is ever made
             const long long sd = I.seed + restart;
             if (a.seed_tab && sd >= a.seed_lo && sd - a.seed_lo < a.seed_n) {
@@ -247,10 +274,10 @@ __device__ __forceinline__ void block_body(const BlockArgs& a, unsigned char* ba
                 }
                 __syncwarp();
                 if (nty == 0) break;
-                if (randomized && mt_random(mt, mpos, lane) >= 1.0 - I.eps) {   // shuffle the type order
+                if (randomized && draw53() >= random_from) {   // shuffle the type order
 #pragma unroll 1
                     for (int i = nty - 1; i > 0; i--) {
-                        const int j = mt_randrange(mt, mpos, lane, i + 1);
+                        const int j = draw_below(i + 1);
                         if (j < 0) { err = ERR_RNG; break; }
                         if (lane == 0) {
                             const int tmp = tys[i];
@@ -276,8 +303,8 @@ __device__ __forceinline__ void block_body(const BlockArgs& a, unsigned char* ba
                         if (start >= ns) break;
                         const int tk = min(I.blk_topk, ns - start);
                         int pick = 0;
-                        if (randomized && mt_random(mt, mpos, lane) >= 1.0 - I.eps) {
-                            pick = mt_randrange(mt, mpos, lane, tk);
+                        if (randomized && draw53() >= random_from) {
+                            pick = draw_below(tk);
                             if (pick < 0) { err = ERR_RNG; break; }
                         }
                         const BlkShape S = cat[tab[I.bo_list + l0 + start + pick]];
@@ -362,8 +389,8 @@ __device__ __forceinline__ void block_body(const BlockArgs& a, unsigned char* ba
                     if (stuck) continue;   // this block stays out (for now): no draw
                     from_key = pkey;
                     __syncwarp();
-                    if (randomized && mt_random(mt, mpos, lane) >= 1.0 - I.eps) {
-                        const int idx = mt_randrange(mt, mpos, lane, __reduce_add_sync(FULL, count));
+                    if (randomized && draw53() >= random_from) {
+                        const int idx = draw_below(__reduce_add_sync(FULL, count));
                         if (idx < 0) { err = ERR_RNG; break; }
                         // the feasible item with idx feasible ones at smaller keys
 #pragma unroll 1

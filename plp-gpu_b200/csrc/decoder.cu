@@ -384,7 +384,7 @@ __device__ __forceinline__ uint2 filter_point(uint32_t key, const StepOrs& S, in
 // Warp 0 of a decoder: pick the pair, place the box, update the live points,
 // the top-sorted box tables and the top-z index. Returns a DecodeErr.
 __device__ __forceinline__ int place_step(DecShared* sh, const StepOrs& S, int t, int best, bool full,
-                                          uint32_t* mt, int& mpos, uint32_t* candA, uint32_t* candB,
+                                          uint32_t* mt, MtPos& mpos, uint32_t* candA, uint32_t* candB,
                                           const uint2* W,
                                           const unsigned char* cmask, int4* bx, int* bzs, int* z2s,
                                           unsigned short* bis, unsigned short* zt, int Hz, int& nc,
@@ -579,7 +579,7 @@ __device__ __forceinline__ void decoder_body(const DecoderArgs& a, unsigned char
         unsigned long long* best_out = a.places + I.place_off + (long long)restart * I.place_stride;
         unsigned long long* pass_out =
             I.passes > 1 ? a.scratch + (long long)gdec * a.scratch_stride : best_out;
-        int mpos = 624;   // RNG position (warp 0)
+        MtPos mpos{MT_WORDS, 0u};   // RNG position (warp 0)
         if (g == 0) {
             const long long sd = I.seed + restart;
             mt_seed_warp(mt, (unsigned long long)(sd < 0 ? -sd : sd), a.mt_init, lane);
@@ -1128,7 +1128,7 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
         unsigned long long* best_out = a.places + I.place_off + (long long)restart * I.place_stride;
         unsigned long long* pass_out =
             I.passes > 1 ? a.scratch + (long long)gdec * a.scratch_stride : best_out;
-        int mpos = 624;
+        MtPos mpos{MT_WORDS, 0u};
         if (randomized) {   // else no draw is ever made
             const long long sd = I.seed + restart;
             if (!SERVE && a.seed_tab && sd >= a.seed_lo && sd - a.seed_lo < a.seed_n) {
@@ -1408,15 +1408,15 @@ static DecoderArgs decoder_args(const DecodeLaunch& L) {
 }
 
 #ifndef PLP_SERVE_TU
-// The M = 16 configuration is built for 18 resident decoders: the compiler
-// settles at 90 registers (112 for a bound of 16), and 18 decoders of 112
-// registers or fewer fit the register file as well as 16 do. 512 batched
-// instances x 128 restarts: 7.9 ms built for 16, 7.25 for 18, 8.3 for 20 (4 KB
-// more code, see below). Straight-line code is kept short throughout
-// (unroll 1): with the twist and the FSR unrolled, 68 KB instead of 44, the
-// same build took 8.0 ms and one 4 KB larger 12 ms, waiting for instructions.
+// The M = 16 configuration is built for 17 resident decoders: the compiler
+// settles at 88 registers (106 for a bound of 15 or 16), which leaves 21 of them
+// room in the register file. 512 batched instances x 128 restarts at 256 boxes
+// and 160 points: 6.98 ms built for 15 or 16, 6.40 for 17, 6.44 for 18, 6.62 for
+// 19, 7.0 for 20 (fewer registers, more code). Straight-line code is kept short
+// throughout (unroll 1): at an earlier stage 68 KB instead of 44 cost 10 % and a
+// build 4 KB larger half of the rate, waiting for instructions.
 template <int D, int M>
-__global__ void __launch_bounds__(32 * D, M == 16 ? 18 : M) decoder1_kernel(DecoderArgs a) {
+__global__ void __launch_bounds__(32 * D, M == 16 ? 17 : M) decoder1_kernel(DecoderArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int dec = threadIdx.x >> 5;
     const Dec1Layout lay = dec1_layout(a.P, a.C, a.Hz);
@@ -1468,7 +1468,7 @@ __global__ void rng_dump_kernel(const long long* __restrict__ seeds, int n_seeds
     uint32_t* mt = mts[wid];
     const long long sv = seeds[s];
     mt_seed_warp(mt, (unsigned long long)(sv < 0 ? -sv : sv), mt_init, lane);
-    int pos = 624;
+    MtPos pos{MT_WORDS, 0u};
     for (int i = 0; i < n_random; i++) {
         const double r = mt_random(mt, pos, lane);
         if (lane == 0) out_r[(long long)s * n_random + i] = r;

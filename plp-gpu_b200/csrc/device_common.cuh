@@ -235,23 +235,35 @@ static __device__ __noinline__ void mt_twist_warp(uint32_t* mt, int lane) {
     __syncwarp();
 }
 
+// Read position: the next word, and this lane's word of its block of 32,
+// tempered. The warp tempers 32 words at once and a draw is one shuffle (the
+// dependent shifts of a word at a time cost a step of the decoder some 20
+// instructions).
+struct MtPos {
+    int pos;
+    uint32_t word;
+};
+constexpr int MT_WORDS = 624;
+
 template <int SPACE = 0>
-__device__ __forceinline__ uint32_t mt_next(uint32_t* mt, int& pos, int lane) {
-    if (pos >= 624) {
-        mt_twist_warp<SPACE>(mt, lane);
-        pos = 0;
+__device__ __forceinline__ uint32_t mt_next(uint32_t* mt, MtPos& p, int lane) {
+    if ((p.pos & 31) == 0 || p.pos >= MT_WORDS) {
+        if (p.pos >= MT_WORDS) {
+            mt_twist_warp<SPACE>(mt, lane);
+            p.pos = 0;
+        }
+        uint32_t y = mt[min(p.pos + lane, MT_WORDS - 1)];   // 624 is 19 blocks and a half
+        y ^= y >> 11;
+        y ^= (y << 7) & 0x9d2c5680u;
+        y ^= (y << 15) & 0xefc60000u;
+        p.word = y ^ (y >> 18);
     }
-    uint32_t y = mt[pos++];
-    y ^= y >> 11;
-    y ^= (y << 7) & 0x9d2c5680u;
-    y ^= (y << 15) & 0xefc60000u;
-    y ^= y >> 18;
-    return y;
+    return __shfl_sync(FULL, p.word, p.pos++ & 31);
 }
 
 // CPython random(): (a * 2^26 + b) / 2^53 with a = 27 bits, b = 26 bits.
 template <int SPACE = 0>
-__device__ __forceinline__ double mt_random(uint32_t* mt, int& pos, int lane) {
+__device__ __forceinline__ double mt_random(uint32_t* mt, MtPos& pos, int lane) {
     const uint32_t a = mt_next<SPACE>(mt, pos, lane) >> 5;
     const uint32_t b = mt_next<SPACE>(mt, pos, lane) >> 6;
     return ((double)a * 67108864.0 + (double)b) * (1.0 / 9007199254740992.0);
@@ -262,7 +274,7 @@ __device__ __forceinline__ double mt_random(uint32_t* mt, int& pos, int lane) {
 // scaling by 2^53 and the ceiling are exact). Spares the FP64 pipe a
 // conversion and a product on each draw.
 template <int SPACE = 0>
-__device__ __forceinline__ unsigned long long mt_random53(uint32_t* mt, int& pos, int lane) {
+__device__ __forceinline__ unsigned long long mt_random53(uint32_t* mt, MtPos& pos, int lane) {
     const uint32_t a = mt_next<SPACE>(mt, pos, lane) >> 5;
     const uint32_t b = mt_next<SPACE>(mt, pos, lane) >> 6;
     return ((unsigned long long)a << 26) | b;
@@ -275,7 +287,7 @@ __device__ __forceinline__ unsigned long long mt_threshold(double t) {
 // CPython randrange(n), n >= 1: getrandbits(bit_length(n)) until < n.
 // Returns -1 if the (astronomically unlikely) rejection bound is hit.
 template <int SPACE = 0>
-__device__ __forceinline__ int mt_randrange(uint32_t* mt, int& pos, int lane, int n) {
+__device__ __forceinline__ int mt_randrange(uint32_t* mt, MtPos& pos, int lane, int n) {
     const int k = 32 - __clz(n);
     for (int tries = 0; tries < 4096; tries++) {
         const uint32_t r = mt_next<SPACE>(mt, pos, lane) >> (32 - k);
