@@ -261,7 +261,7 @@ int plp_request_times(plp_handle* h, int64_t request_id, double* queued_s, doubl
  * the same launch, by one of its overflow decoders (a deeper tile in global
  * memory). While the serving launch runs it holds the SMs: plp_solve,
  * plp_batch_run and plp_autotune on this handle ask an idle launch to stop at
- * once; other work on the GPU runs once it has stopped (50 ms after the last
+ * once; other work on the GPU runs once it has stopped (5 ms after the last
  * request finished). This call reports the handle's serving launches,
  * requests served by them, requests re-run on the wave path's code after a
  * restart outgrew even the overflow tile, and eligible requests sent to the
