@@ -838,7 +838,6 @@ __device__ __forceinline__ unsigned z_within(const Edges& E, int v) {
 __device__ __forceinline__ unsigned support_slots(unsigned cand, int x, int y, int j, int je, const Edges& E,
                                                   const uint4* bx) {
     unsigned a0 = 0, a1 = 0, a2 = 0, a3 = 0, a4 = 0, a5 = 0;
-    const int xl = x + E.l, xw = x + E.w, xh = x + E.h, yl = y + E.l, yw = y + E.w, yh = y + E.h;
     // two boxes at a time; past the end an empty box, which adds nothing
 #pragma unroll 1
     for (; j < je; j += 2) {
@@ -847,13 +846,14 @@ __device__ __forceinline__ unsigned support_slots(unsigned cand, int x, int y, i
 #pragma unroll
         for (int u = 0; u < 2; u++) {
             const uint2 b = u ? b1 : b0;
-            const int nx = -max(x, (int)(b.x & 0xffffu)), ny = -max(y, (int)(b.y & 0xffffu));
-            const int tx = (int)(b.x >> 16) + nx, ty = (int)(b.y >> 16) + ny;
-            // overlap along an axis: max(0, min(x + e, b.x2) - max(x, b.x))
-            const unsigned ol = __viaddmin_s32_relu(xl, nx, tx), ow = __viaddmin_s32_relu(xw, nx, tx),
-                           oh = __viaddmin_s32_relu(xh, nx, tx);
-            const unsigned pl = __viaddmin_s32_relu(yl, ny, ty), pw = __viaddmin_s32_relu(yw, ny, ty),
-                           ph = __viaddmin_s32_relu(yh, ny, ty);
+            // from the point: the box spans [-nx, tx - nx) along x; overlap with an
+            // edge e: max(0, min(e, tx - nx) + nx)
+            const int nx = min(x - (int)(b.x & 0xffffu), 0), ny = min(y - (int)(b.y & 0xffffu), 0);
+            const int tx = (int)(b.x >> 16) - x + nx, ty = (int)(b.y >> 16) - y + ny;
+            const unsigned ol = __viaddmin_s32_relu(E.l, nx, tx), ow = __viaddmin_s32_relu(E.w, nx, tx),
+                           oh = __viaddmin_s32_relu(E.h, nx, tx);
+            const unsigned pl = __viaddmin_s32_relu(E.l, ny, ty), pw = __viaddmin_s32_relu(E.w, ny, ty),
+                           ph = __viaddmin_s32_relu(E.h, ny, ty);
             a0 += ow * ph;
             a1 += oh * pw;
             a2 += ol * ph;

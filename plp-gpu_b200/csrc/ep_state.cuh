@@ -108,17 +108,17 @@ __device__ __forceinline__ int place1(uint32_t pkey, int pw, int pd, int ph, uin
         const int i = cb + lane;
         const bool in = i < nc;
         const uint32_t key = in ? K[i] : 0u, exy = in ? K[cap + i] : 0u, ezm = in ? K[2 * cap + i] : 0u;
-        int ex = (int)(exy & 0xffffu), ey = (int)(exy >> 16), ez = (int)(ezm & 0xffffu);
-        uint32_t mark = ezm & PT_MARKED;
         const int x = (int)(key & xmask), y = (int)((key >> xb) & ymask), z = (int)(key >> xyb);
-        const bool ax = x < px2, ay = y < py2, az = z < pz2;
-        const bool ix = ax && x > px - ME.w, iy = ay && y > py - ME.d, iz = az && z > pz - ME.h;
-        if (iy && iz && ax) ex = min(ex, px - x);
-        if (ix && iz && ay) ey = min(ey, py - y);
-        if (ix && iy && az) ez = min(ez, pz - z);
-        if (ax && ay && az && px < x + ex && py < y + ey && pz < z + ez) mark = PT_MARKED;
-        const bool gone = in && (ex < ME.w || ey < ME.d || ez < ME.h);
-        if (in) {
+        bool gone = false;
+        if (in && x < px2 && y < py2 && z < pz2) {   // else the box lies before the point
+            int ex = (int)(exy & 0xffffu), ey = (int)(exy >> 16), ez = (int)(ezm & 0xffffu);
+            const int dx = px - x, dy = py - y, dz = pz - z;
+            const bool ix = dx < ME.w, iy = dy < ME.d, iz = dz < ME.h;
+            if (iy && iz) ex = min(ex, dx);
+            if (ix && iz) ey = min(ey, dy);
+            if (ix && iy) ez = min(ez, dz);
+            gone = ex < ME.w || ey < ME.d || ez < ME.h;
+            const uint32_t mark = dx < ex && dy < ey && dz < ez ? PT_MARKED : ezm & PT_MARKED;
             K[cap + i] = gone ? 0u : (uint32_t)ex | ((uint32_t)ey << 16);
             K[2 * cap + i] = (uint32_t)ez | mark;
         }
