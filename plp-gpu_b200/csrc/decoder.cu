@@ -1164,6 +1164,7 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
             }
             __syncwarp();
             int state_type = -1;
+            unsigned long long placed = 0;   // this lane's placement of the current 32
             uint32_t from_key = 0;  // points at smaller keys hold no feasible pair of state_type
             bool stuck = false;     // the last step of state_type found no feasible pair
             const EdgeRange ER{I.mw, I.md, I.mh, I.xw, I.xd, I.xh, L, W, H};
@@ -1321,15 +1322,19 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
                 const int pw = (0x14 >> slot) & 1 ? E.l : (0x21 >> slot) & 1 ? E.w : E.h;
                 const int pd = (0x28 >> slot) & 1 ? E.l : (0x12 >> slot) & 1 ? E.w : E.h;
                 const int ph = slot < 2 ? E.l : slot < 4 ? E.w : E.h;
-                if (lane == 0 && nb < a.P)
-                    pass_out[nb] = pack_place((int)(pick_key & xmask), (int)((pick_key >> xb) & ymask),
-                                              (int)(pick_key >> xyb), __popc(slots & ((1u << slot) - 1u)), t);
+                // placements go out 32 at a time, one whole piece of the row (which
+                // may lie in host memory) per store
+                if (lane == (nb & 31))
+                    placed = pack_place((int)(pick_key & xmask), (int)((pick_key >> xb) & ymask),
+                                        (int)(pick_key >> xyb), __popc(slots & ((1u << slot) - 1u)), t);
+                if ((nb & 31) == 31 && nb < a.P) pass_out[nb - 31 + lane] = placed;
                 vol += 1LL * pw * pd * ph;
                 err = place1(pick_key, pw, pd, ph, pts, lay.cap, free_slots, bx, zt, a.Hz, nc, nb, a.P, a.C,
                              xmask, ymask, xb, xyb, ER, lane);
                 if (err != ERR_NONE) break;
             }
             if (err != ERR_NONE) break;
+            if (lane < (nb & 31)) pass_out[(nb & ~31) + lane] = placed;
             const double score =
                 fsr_score_warp<SPACE>(PackedBoxes{bx}, nb, I.mu, reinterpret_cast<char*>(pts), lane, nullptr, zt);
             const bool acc = !I.has_theta || score >= I.theta;
