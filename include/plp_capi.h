@@ -175,12 +175,14 @@ void plp_destroy(plp_handle* h);
  * live-point depth C (per decoder, in shared memory; C a multiple of 32),
  * warps per decoder G, decoders per CTA D and minimum resident CTAs per SM M
  * (which caps registers per thread at 65536 / (32 G D M)). (G, D, M) must be
- * one of (1,1,1) (1,1,12) (1,2,1) (1,4,1) (1,4,4) (1,8,1) (1,8,2) (2,1,1) (2,2,1) (2,2,5)
- * (2,4,1) (2,4,3) (4,1,1) (4,1,5) (4,1,6) (4,2,1) (4,2,3) (4,4,1) (8,1,1)
- * (8,1,3) (8,2,1); 0 keeps the current value. (1,1,12) holds the decoder to
- * 160 registers, so three warps fit in each SM partition's register file
- * where 185 allow two. Restarts that outgrow the tile
- * are re-run with a deeper one, so the tile affects speed only, never results.
+ * one of (1,1,1) (1,1,12) (1,1,16) (1,2,1) (1,4,1) (1,4,4) (1,8,1) (1,8,2)
+ * (2,1,1) (2,2,1) (2,2,5) (2,4,1) (2,4,3) (4,1,1) (4,1,5) (4,1,6) (4,2,1)
+ * (4,2,3) (4,4,1) (8,1,1) (8,1,3) (8,2,1); 0 keeps the current value. (1,1,1)
+ * is the fastest build for one restart; (1,1,16) holds the decoder to fewer
+ * registers, so that five warps fit in each SM partition's register file where
+ * (1,1,1) allows four, and is the faster one for batches of several waves.
+ * Restarts that outgrow the tile are re-run with a deeper one, so the tile
+ * affects speed only, never results.
  * Until a tile is set or tuned, each batch's tile follows from its sizes; a
  * first call that leaves values out takes them from P = 256, C = 512, G = 1,
  * D = 1, M = 1. */

@@ -343,8 +343,7 @@ int place_block_tables(const BlockTables& bt, const Instance& I, const plp_run_o
     return PLP_OK;
 }
 
-// Orientation table of every box type of an instance; clears *small when an
-// orientation's footprint area reaches 65536 (its contact areas need 32 bits).
+// Orientation table of every box type of an instance.
 std::vector<TypeOrs> type_orientations(const Instance& I) {
     std::vector<TypeOrs> ot;
     ot.reserve(I.types.size());

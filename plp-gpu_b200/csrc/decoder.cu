@@ -13,17 +13,18 @@
 //   rows               gpu/plp_gpu.cu:350 (restart k = PyRng(seed + k))
 //
 // Two persistent decoders share the work list and result layout:
-//   decoder1_kernel<D, M>    one warp per restart, incremental per-point
-//                            evaluation (the default; see its section)
+//   decoder1_kernel<D, M>    one warp per restart, free extents kept at every
+//                            live point (the default; see its section)
 //   decoder_kernel<G, D, M>  G warps per restart, lockstep scan of the
 //                            filtered points every step (multi-warp variant)
 //
-// Layout of one decoder in shared memory (both kernels):
+// Layout of one decoder in shared memory:
 //   MT19937 state       624 x u32
-//   placed boxes        sorted by top z (ascending): {x, y, x2, y2} int4,
-//                       bottom z, top z, placement index
-//   live points         sorted unique keys (z, y, x) (+ per-point state and
-//                       contact areas in decoder1_kernel)
+//   placed boxes        sorted by top z (ascending); decoder1_kernel packs a
+//                       box into 16 bytes, decoder_kernel keeps {x, y, x2, y2}
+//                       int4, bottom z, top z and placement index
+//   live points         decoder1_kernel: {key, extents} in no order;
+//                       decoder_kernel: sorted unique keys (z, y, x)
 //   item list           the points to evaluate this step
 // FSR reuses the point buffers as scratch once the pass is done.
 //
@@ -804,11 +805,12 @@ __global__ void __launch_bounds__(32 * G * D, M) decoder_kernel(DecoderArgs a) {
 // and their dependent chains bound it; extents replace per-type masks and six
 // contact areas per point that had to be evaluated against every box at each
 // change of type, kept up to date, and moved with the points. Measured, decoder
-// alone at 128 boxes, 160 points, M = 16: 512 batched instances x 128 restarts
-// 7.0 ms, 64 stress instances x 512 3.7 ms, 1024 restarts of one instance 0.306
-// ms, one greedy decode 0.148 ms (16.3, 11.3, 0.409 and 0.192 ms with masks and
-// areas; 24.5, 21.5, 0.554 and 0.226 ms with those and without the dead-point
-// rule; 7.25, 4.0, 0.325 and 0.169 ms with extents on points kept in order).
+// alone at 256 boxes, 160 points, M = 16: 512 batched instances x 128 restarts
+// 6.3 ms, 64 stress instances x 512 3.5 ms; uncapped, 1024 restarts of one
+// instance 0.28 ms, one greedy decode 0.12 ms (16.3, 11.3, 0.409 and 0.192 ms
+// with masks and areas; 24.5, 21.5, 0.554 and 0.226 ms with those and without
+// the dead-point rule; 7.25, 4.0, 0.325 and 0.169 ms with extents on points kept
+// in order).
 //
 // The C3 test is the integer form of the reference's FP64 ratio:
 // (double)s / (double)(w*d) < 0.5  <=>  2 s < w d. Both s and w d are
