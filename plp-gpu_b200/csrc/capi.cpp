@@ -1817,7 +1817,7 @@ struct ServeEngine {
     char* arena = nullptr;
     size_t cap = 0;
     // ctl: [0] head, [1] tail, [2] stop, [3] error flag, [4] abort, [5] overflow
-    // head, [6] overflow reservations, [7] main decoders alive
+    // head, [6] overflow reservations, [7] main decoders alive, [8] claims
     int* ctl = nullptr;
     int2* ring = nullptr;
     int4* dring = nullptr;
@@ -1917,6 +1917,7 @@ struct ServeEngine {
         args.done_best = static_cast<int2*>(p);
         if (e != cudaSuccess) return set_cuda_error("serving engine set-up", e);
         args.head = ctl;
+        args.claims = ctl + 8;
         args.tail = ctl + 1;
         args.stop = ctl + 2;
         args.ring = ring;
@@ -2375,6 +2376,7 @@ struct ServeEngine {
         if (!running) yield_req = false;
         if (!running && idle && (tail > (1 << 30) || h_word[4] > (1 << 30)) && !work_left()) {
             cudaMemsetAsync(ctl, 0, 2 * sizeof(int), up);        // head, tail
+            cudaMemsetAsync(ctl + 8, 0, sizeof(int), up);        // claims
             cudaMemsetAsync(ctl + 5, 0, 2 * sizeof(int), up);    // overflow head, reservations
             cudaStreamSynchronize(up);
             tail = 0;

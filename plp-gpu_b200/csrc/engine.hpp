@@ -79,6 +79,7 @@ struct ServeTail {
 };
 struct ServeArgs {
     int* head;                      // device: work items claimed
+    int* claims;                    // device: those and the claims about to be taken back
     const int* tail;                // device: work items published (written by stream-ordered copies)
     const int* stop;                // device: nonzero = exit once no work is left
     const int2* ring;               // device: work items (descriptor index, restart)
