@@ -1049,7 +1049,7 @@ __device__ __forceinline__ void serve_finish(const DecoderArgs& a, const ServeAr
     ServeTail* tl = reinterpret_cast<ServeTail*>(const_cast<InstDesc*>(a.inst) + di + 1);
     int last = 0;
     if (lane == 0) {
-        __threadfence();
+        __threadfence_system();   // placements may go to host memory
         last = atomicAdd(&tl->done_count, 1) == I.restarts - 1;
     }
     last = __shfl_sync(FULL, last, 0);
