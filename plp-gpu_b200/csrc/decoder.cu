@@ -1827,7 +1827,7 @@ __global__ void __launch_bounds__(32 * D, M)
 
 // ---- serving launches ------------------------------------------------------
 using ServeFn = void (*)(DecoderArgs, ServeArgs);
-#define PLP_SERVE_CONFIGS(X) X(1, 1) X(1, 12)
+#define PLP_SERVE_CONFIGS(X) X(1, 1) X(1, 12) X(1, 16)
 
 static ServeFn serve_fn(int D, int M) {
 #define PLP_PICK_SERVE(d, m) \
