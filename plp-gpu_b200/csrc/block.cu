@@ -532,9 +532,9 @@ __device__ __forceinline__ void block_body(const BlockArgs& a, unsigned char* ba
 
 // One decoder per CTA is built for 14 resident ones (121 registers instead of
 // 154). 512 batched instances x 64 restarts, campaign configuration, 128 blocks,
-// 192 points: 3.2 ms (3.40 before the divisions by a, b and k went; then 3.68
-// uncapped, 3.48 for 16, 3.59 for 18; 9.07 ms with
-// every point evaluated against every box for every block).
+// 192 points: 2.9 ms (when the bound was chosen 3.40, with 3.68 uncapped, 3.48 for
+// 16 and 3.59 for 18; 9.07 ms with every point evaluated against every box for
+// every block).
 template <int D, int M>
 __global__ void __launch_bounds__(32 * D, D == 1 ? 14 : M) block_kernel(BlockArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];

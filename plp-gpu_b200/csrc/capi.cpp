@@ -651,20 +651,22 @@ struct TileFloor {
 
 // The tile of a batch on a handle whose tile was neither set nor tuned.
 //  * Bound by its longest restart (the batch's steps spread over the resident
-//    decoders are fewer than the longest restart's): the uncapped build, which
-//    runs one restart fastest, and a tile that no restart outgrows (a pass
-//    places at most one box per step and holds about as many live points).
-//    1024 restarts of one instance: 0.294 ms, 0.314 with the M = 16 build; 61
-//    batched instances x 48: 1.24 ms against 1.43.
-//  * Otherwise M = 16, up to 21 decoders per SM: 2048 restarts of one instance
-//    0.407 ms, 0.522 with the uncapped build (13 per SM). While the batch fits
-//    one wave the deepest tile that keeps it there, since a restart that
-//    outgrows it runs again afterwards; in several waves 256 boxes and up to
-//    192 points, which about every restart fits (the device retry stage takes
-//    the others). 512 batched instances x 128 restarts: 7.15 ms at 160 points,
-//    8.49 at 128 and 8.18 at 96, where the stage runs a few restarts again.
+//    decoders are fewer than the longest restart's): the uncapped build and a
+//    tile that no restart outgrows (a pass places at most one box per step and
+//    holds about as many live points). 61 batched instances x 48: decoder 0.525
+//    ms, 0.537 with the M = 16 build; 1024 restarts of one instance 0.279 with
+//    either.
+//  * Otherwise M = 16, up to 20 decoders per SM: 5000 restarts of one instance
+//    0.72 ms, 0.80 with the uncapped build (13 to 16 per SM). While the batch fits
+//    one wave the deepest tile that keeps it there (2048 restarts: 0.36 ms; 0.51 at
+//    256, 512, which takes two), since a restart that outgrows it runs again
+//    afterwards; in several waves 256 boxes and up to 192 points, which about
+//    every restart fits (the device retry stage takes the others). 512 batched
+//    instances x 128 restarts with the retry stage: 6.34 ms at 160 and 192 points,
+//    7.45 at 128 and 7.33 at 96, where the stage runs a few restarts again; 6.83
+//    uncapped.
 // The block engine has one build: 128 blocks, 192 points for several waves (512
-// instances x 64 restarts: 3.2 ms; about 9 % more at 256, 512).
+// instances x 64 restarts: 2.9 ms; about 9 % more at 256, 512).
 TileConfig auto_tile(const Batch& b, int sms, const TileFloor& f, int* wave) {
     const int steps = (std::max(1, b.max_steps) + 15) & ~15;
     const int points = std::max(128, (steps + 63) & ~31);

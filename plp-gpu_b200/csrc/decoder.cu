@@ -1804,7 +1804,7 @@ cudaError_t launch_gather_best(const InstDesc* inst, int n_inst, const int2* bes
 
 #ifdef PLP_SERVE_TU
 // Overflow decoders run out of line, so that the main decoders keep a body of
-// their own (158 registers instead of 170).
+// their own (in one body the M = 16 build spills 400 bytes).
 static __device__ __noinline__ void serve_deep(const DecoderArgs& a, const ServeArgs& s, int gdec) {
     DecoderArgs ad = a;
     ad.P = s.deep_P;
