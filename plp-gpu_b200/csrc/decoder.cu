@@ -50,6 +50,7 @@
 #include "ep_state.cuh"
 #include "feas_eval.cuh"
 #include "fsr_warp.cuh"
+#include "serve_claim.hpp"
 
 #include <algorithm>
 #include <climits>
@@ -959,38 +960,21 @@ __device__ __forceinline__ void serve_push_deep(const ServeArgs& s, int2 wk, int
     __syncwarp();
 }
 
-// Lane 0: claims the next published work item, or returns -1 once the host
-// has asked the launch to stop (and nothing is left) or after idle_polls
-// empty polls. The host publishes by stream-ordered copies into device
-// memory (items first, then the tail), so the polls stay on this GPU's L2.
-// The loop is bounded by idle_polls.
-//
-// A decoder first counts itself among the claims; if the count before it is
-// below the tail, an item is left for it and the head's next value is that
-// item, else it takes its count back. The count is the claims that succeeded
-// and those about to be taken back, so no more succeed than are published. Two
-// additions, which the L2 serves one after the other, in place of a
-// compare-and-swap of the head, which one decoder wins per round trip: that
-// held the launch to 3 restarts per us whatever their size (119872 restarts in
-// 256 requests: 40.3 ms, 20.6 so where the result copies keep up).
-__device__ __forceinline__ int serve_claim(const ServeArgs& s) {
-    unsigned ns = 32;
-    for (int k = 0; k < s.idle_polls; k++) {
-        const int t = ld_acquire_gpu(s.tail);
-        if (*reinterpret_cast<volatile int*>(s.head) < t) {
-            if (atomicAdd(s.claims, 1) < t) {
-                const int i = atomicAdd(s.head, 1);
-                if (i >= t) (void)ld_acquire_gpu(s.tail);   // published since: its words were written before
-                return i;
-            }
-            atomicSub(s.claims, 1);
-        }
-        if (ld_acquire_gpu(s.stop)) return -1;
-        __nanosleep(ns);
-        if (ns < 4096) ns <<= 1;
-    }
-    return -1;
-}
+// The words of serve_claim in device memory. The host publishes by
+// stream-ordered copies into it (items first, then the tail), so the polls stay
+// on this GPU's L2. 119872 restarts in 256 requests: 40.3 ms with one counter
+// and a compare-and-swap, 20.6 with two additions where the result copies keep up.
+struct ServeWords {
+    const ServeArgs& s;
+    __device__ __forceinline__ int tail() const { return ld_acquire_gpu(s.tail); }
+    __device__ __forceinline__ int claims() const { return *reinterpret_cast<volatile int*>(s.claims); }
+    __device__ __forceinline__ int head() const { return *reinterpret_cast<volatile int*>(s.head); }
+    __device__ __forceinline__ int claim() const { return atomicAdd(s.claims, 1); }
+    __device__ __forceinline__ void unclaim() const { atomicSub(s.claims, 1); }
+    __device__ __forceinline__ int take() const { return atomicAdd(s.head, 1); }
+    __device__ __forceinline__ bool stopped() const { return ld_acquire_gpu(s.stop) != 0; }
+    __device__ __forceinline__ void pause(unsigned ns) const { __nanosleep(ns); }
+};
 
 // A request descriptor read through L2 (serving arenas reuse addresses while
 // the launch runs, so no table may come from a stale L1 line).
@@ -1094,7 +1078,8 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
             int sitem = -1, wx = 0, wy = 0;
             if (lane == 0) {
                 if constexpr (MODE == 1) {
-                    sitem = serve_claim(sv);
+                    ServeWords words{sv};
+                    sitem = serve_claim(words, sv.idle_polls);
                     if (sitem >= 0) {
                         const int2 w = ld_relaxed_gpu_int2(sv.ring + (sitem & sv.ring_mask));
                         wx = w.x;

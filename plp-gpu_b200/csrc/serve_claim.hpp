@@ -1,0 +1,55 @@
+// serve_claim.hpp -- how a serving decoder takes the next published work item.
+// Written over the words it reads and changes (Words), so that the same code
+// runs in the decoders (decoder.cu: words in device memory) and in a test's
+// model of many decoders under a chosen order of their accesses.
+#pragma once
+
+#ifdef __CUDACC__
+#define PLP_HD __host__ __device__ __forceinline__
+#else
+#define PLP_HD inline
+#endif
+
+namespace plpb {
+
+// The next item's number, or -1 once the host has asked the launch to stop and
+// every published item is taken, or after `polls` empty polls.
+//
+// Two counters, so that a claim is two additions, which the L2 serves one after
+// the other (a compare-and-swap of one counter, which one decoder wins per round
+// trip, held a launch to 3 restarts per us whatever their size). A decoder first
+// counts itself among the claims; if the count before it is below the tail, an
+// item is left for it and the head's next value is that item, else it takes its
+// count back. The count is the claims that succeeded and those about to be taken
+// back, so no more succeed than are published.
+//
+// A claim is tried only where the count was read below the tail. Claims about
+// to be taken back can then keep nobody from a free item: after the count was
+// read below the tail, the next addition is one that succeeds, so there is no
+// round of failures without a claim between. (Tried whenever the head is below
+// the tail, failures alone hold the count up, and idle decoders, of which there
+// are some 2000, keep all of each other from a request of a few restarts.)
+//
+// The stop word is read before the head and the tail that it is obeyed by, so a
+// decoder leaves no item that was published before the stop.
+template <class Words>
+PLP_HD int serve_claim(Words& w, int polls) {
+    unsigned ns = 32;
+    for (int k = 0; k < polls; k++) {
+        const int t = w.tail();
+        if (w.claims() < t) {
+            if (w.claim() < t) {
+                const int i = w.take();
+                if (i >= t) (void)w.tail();   // published since: its words were written before
+                return i;
+            }
+            w.unclaim();
+        }
+        if (w.stopped() && w.head() >= w.tail()) return -1;
+        w.pause(ns);
+        if (ns < 4096) ns <<= 1;
+    }
+    return -1;
+}
+
+}  // namespace plpb

@@ -1,0 +1,123 @@
+// Many serving decoders on one set of claim words, one access at a time in the
+// order a scheduler picks: it likes to leave decoders between a failed claim and
+// taking it back, but lets every decoder go on after a bounded wait.
+//   serve_claim_model progress   16 items while failed claims are pending
+//   serve_claim_model stop       the same, with the stop word set
+// Prints "<items taken> <items published> <accesses granted>".
+#include <condition_variable>
+#include <cstdio>
+#include <cstring>
+#include <mutex>
+#include <thread>
+#include <vector>
+
+#include "serve_claim.hpp"
+
+namespace {
+
+constexpr int DECODERS = 64, PENDING = 20, WAIT = 8 * DECODERS, LIMIT = 8000;
+
+struct Model {
+    std::mutex mu;
+    std::condition_variable cv;        // the scheduler's
+    int head = 0, tail = 0, claims = 0;
+    bool stop = false, over = false;
+    int turn = -1;                     // the decoder that may make one access
+    struct Decoder {
+        std::condition_variable cv;
+        bool waiting = false, unclaims = false, done = false;
+        int since = 0, got = -1;
+    };
+    std::vector<Decoder> d = std::vector<Decoder>(DECODERS);
+
+    // blocks until the scheduler grants this decoder one access
+    template <class F>
+    auto access(int i, bool unclaims, const F& f) {
+        std::unique_lock<std::mutex> lk(mu);
+        d[i].waiting = true;
+        d[i].unclaims = unclaims;
+        cv.notify_one();
+        d[i].cv.wait(lk, [&] { return turn == i || over; });
+        d[i].waiting = false;
+        if (turn == i) turn = -1;
+        return f();
+    }
+};
+
+struct Words {
+    Model& m;
+    int i;
+    int tail() { return m.access(i, false, [&] { return m.tail; }); }
+    int claims() { return m.access(i, false, [&] { return m.claims; }); }
+    int head() { return m.access(i, false, [&] { return m.head; }); }
+    int claim() { return m.access(i, false, [&] { return m.claims++; }); }
+    void unclaim() { m.access(i, true, [&] { m.claims--; }); }
+    int take() { return m.access(i, false, [&] { return m.head++; }); }
+    bool stopped() { return m.access(i, false, [&] { return m.stop || m.over; }); }
+    void pause(unsigned) {}
+};
+
+}  // namespace
+
+int main(int argc, char** argv) {
+    const bool stop = argc > 1 && !std::strcmp(argv[1], "stop");
+    Model m;
+    // a decoder that ends (with an item, or without) takes part no further, as
+    // one that decodes for long does
+    std::vector<std::thread> ts;
+    for (int i = 0; i < DECODERS; i++)
+        ts.emplace_back([&m, i] {
+            Words w{m, i};
+            const int got = plpb::serve_claim(w, LIMIT);
+            std::lock_guard<std::mutex> lk(m.mu);
+            m.d[i].got = got;
+            m.d[i].done = true;
+            m.cv.notify_one();
+        });
+    // four items, whose claims race with the other decoders' until some of those are pending
+    m.tail = 4;
+    int published = 4, granted = 0, next = 0, taken = 0;
+    for (;;) {
+        std::unique_lock<std::mutex> lk(m.mu);
+        m.cv.wait(lk, [&] {
+            if (m.turn >= 0) return false;
+            for (const auto& x : m.d)
+                if (!x.waiting && !x.done) return false;
+            return true;
+        });
+        int pending = 0, live = 0, oldest = -1;
+        taken = 0;
+        for (int i = 0; i < DECODERS; i++) {
+            auto& x = m.d[i];
+            taken += x.done && x.got >= 0;
+            if (x.done) continue;
+            live++;
+            if (x.unclaims) {
+                pending++;
+                if (oldest < 0 || x.since < m.d[oldest].since) oldest = i;
+            }
+        }
+        if (!live || granted == LIMIT || (taken == 20 && !stop)) {
+            m.over = true;
+            for (auto& x : m.d) x.cv.notify_one();
+            break;
+        }
+        // later items, once failed claims are pending (or nobody is in between)
+        if (published == 4 && (pending >= PENDING || granted > 4 * WAIT)) {
+            published = m.tail = 20;
+            m.stop = stop;
+        }
+        int pick = -1;
+        if (pending > PENDING || (oldest >= 0 && granted - m.d[oldest].since > WAIT)) pick = oldest;
+        for (int k = 0; pick < 0 && k < DECODERS; k++, next = (next + 1) % DECODERS)
+            if (!m.d[next].done && !m.d[next].unclaims) pick = next;
+        if (pick < 0) pick = oldest;
+        m.d[pick].unclaims = false;
+        m.d[pick].since = granted++;
+        m.turn = pick;
+        m.d[pick].cv.notify_one();
+    }
+    for (auto& t : ts) t.join();
+    std::printf("%d %d %d\n", taken, published, granted);
+    return 0;
+}
