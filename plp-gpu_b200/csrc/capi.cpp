@@ -9,6 +9,7 @@
 #include <atomic>
 #include <chrono>
 #include <climits>
+#include <cmath>
 #include <condition_variable>
 #include <cstdio>
 #include <cstdlib>
@@ -372,21 +373,53 @@ std::vector<TypeOrs> type_orientations(const Instance& I) {
     return ot;
 }
 
-// Smallest and largest edge per axis over the types' orientations (1 where
-// there is none).
-void edge_range(const std::vector<TypeOrs>& ors, InstDesc& d) {
+// Smallest and largest edge per axis over an instance's orientations (1 where
+// there is none), and the depths that its passes are likely to need.
+struct Sizes {
+    int mw = 1, md = 1, mh = 1, xw = 1, xd = 1, xh = 1;
+    int boxes = 1, points = 1;
+};
+
+// Boxes: as many as there are, or fill four fifths of the container. Live points
+// per box: a point dies with the free room around it, when the smallest edges no
+// longer fit, so the smallest edges against the mean one say how many stay. In a
+// container that the items fill, the others lie on the packing's front, a surface;
+// one that the items leave open keeps points at all its open faces. The constants
+// are fitted to the peaks of 756 instances, four decodes each, from full
+// containers to ones 15 % full, with smallest edges of 3 to 100 % of the mean: the
+// result is below the peak in 7 % of them (by a tenth in 2 %), 1.35 times the peak
+// at the median and above twice the peak in 8 %. Too few points make restarts run
+// again, too many cost residency in a batch of several waves.
+Sizes instance_sizes(const Instance& I, const std::vector<TypeOrs>& ors) {
+    Sizes z;
     bool any = false;
-    d.mw = d.md = d.mh = d.xw = d.xd = d.xh = 1;
-    for (const TypeOrs& t : ors)
+    double n = 0, vol = 0;
+    for (size_t i = 0; i < ors.size(); i++) {
+        const TypeOrs& t = ors[i];
         for (int k = 0; k < t.n; k++) {
-            d.mw = any ? std::min(d.mw, t.w[k]) : t.w[k];
-            d.md = any ? std::min(d.md, t.d[k]) : t.d[k];
-            d.mh = any ? std::min(d.mh, t.h[k]) : t.h[k];
-            d.xw = std::max(d.xw, t.w[k]);
-            d.xd = std::max(d.xd, t.d[k]);
-            d.xh = std::max(d.xh, t.h[k]);
+            z.mw = any ? std::min(z.mw, t.w[k]) : t.w[k];
+            z.md = any ? std::min(z.md, t.d[k]) : t.d[k];
+            z.mh = any ? std::min(z.mh, t.h[k]) : t.h[k];
+            z.xw = std::max(z.xw, t.w[k]);
+            z.xd = std::max(z.xd, t.d[k]);
+            z.xh = std::max(z.xh, t.h[k]);
             any = true;
         }
+        if (t.n) {
+            n += I.types[i].qty;
+            vol += (double)I.types[i].qty * I.types[i].volume();
+        }
+    }
+    if (n == 0) return z;
+    const double mean = vol / n, room = (double)I.L * I.W * I.H;
+    const double edge = (z.mw + z.md + z.mh) / (3 * std::cbrt(mean));
+    const double boxes = std::min(n, 0.8 * room / mean);
+    const double full = 0.8 * std::cbrt(80 / boxes) + 3.5 * std::exp(-edge / 0.11);
+    const double open = std::max(full, 3.7 - 1.9 * edge);
+    const double share = std::pow(std::min(1.0, std::max(0.0, (1 - vol / room) / 0.8)), 1 + 2 * edge);
+    z.boxes = (int)std::min(1e6, boxes) + 1;
+    z.points = (int)std::min(1e6, 1.1 * boxes * (full + share * (open - full))) + 8;
+    return z;
 }
 
 struct Batch {
@@ -401,6 +434,11 @@ struct Batch {
     long long n_slots = 0, n_places = 0;
     int max_stride = 1, max_steps = 0, Hz = 0;
     long long sum_steps = 0, long_steps = 1;   // of all restarts and of the longest, over their passes
+    int max_points = 1;                        // live points expected of the instance that needs most
+    // the batch's steps in instances that are expected to hold more live points
+    // than POINTS[k], and in those to place more than BOXES[k] boxes
+    static constexpr int POINTS[] = {192, 256, 384, 512}, BOXES[] = {128, 256};
+    long long over_points[4] = {}, over_boxes[2] = {};
     bool multi_pass = false;
     // block-building engine: shape catalogue and per-instance orderings
     int engine = 0, max_types = 0;
@@ -458,21 +496,27 @@ struct Batch {
         max_types = 0;
         n_slots = 0; n_places = 0; max_stride = 1; max_steps = 0; multi_pass = false;
         sum_steps = 0; long_steps = 1;
+        max_points = 1;
+        std::fill(std::begin(over_points), std::end(over_points), 0);
+        std::fill(std::begin(over_boxes), std::end(over_boxes), 0);
         int maxH = 0;
         best_only = true;
         // item sequences and orientation tables of a large batch are built on
         // several threads; the rest of the build is appends in instance order
         std::vector<std::vector<int>> seqs;
         std::vector<std::vector<TypeOrs>> ors;
+        std::vector<Sizes> sizes;
         // (an instance's first block tables take about 0.35 ms, so those are
         // spread from a few instances on)
         if (engine == 1) blk.resize(in.size());
         if (in.size() >= (engine == 1 ? 8u : 256u)) {
             seqs.resize(in.size());
             ors.resize(in.size());
+            sizes.resize(in.size());
             parallel_for(in.size(), engine == 1 ? 4 : 64, [&](size_t k) {
                 if (op[k].order == 0 || op[k].order == 1) seqs[k] = item_sequence(*in[k], op[k].order);
                 ors[k] = type_orientations(*in[k]);
+                sizes[k] = instance_sizes(*in[k], ors[k]);
                 int status = PLP_OK;
                 if (engine == 1 && op[k].engine == 1 && in[k]->types.size() <= 2048)
                     blk[k] = block_tables(*in[k], ors[k], op[k], &status);   // a failure is met again below
@@ -536,7 +580,9 @@ struct Batch {
             steps.insert(steps.end(), seq.begin(), seq.end());
             std::vector<TypeOrs> ot = ors.empty() ? type_orientations(I) : std::move(ors[i]);
             types.insert(types.end(), ot.begin(), ot.end());
-            edge_range(ot, desc.back());
+            const Sizes need = sizes.empty() ? instance_sizes(I, ot) : sizes[i];
+            desc.back().mw = need.mw; desc.back().md = need.md; desc.back().mh = need.mh;
+            desc.back().xw = need.xw; desc.back().xd = need.xd; desc.back().xh = need.xh;
             desc.back().engine = o.engine;
             desc.back().n_types = (int)I.types.size();
             max_types = std::max(max_types, (int)I.types.size());
@@ -558,6 +604,9 @@ struct Batch {
                 const long long s = (long long)d.n_steps * std::min(d.passes, 1 << 16);
                 sum_steps += s * o.restarts;
                 long_steps = std::max(long_steps, s);
+                max_points = std::max(max_points, need.points);
+                for (int k = 0; k < 4; k++) over_points[k] += need.points > POINTS[k] ? s * o.restarts : 0;
+                for (int k = 0; k < 2; k++) over_boxes[k] += need.boxes > BOXES[k] ? s * o.restarts : 0;
             }
             multi_pass = multi_pass || d.passes > 1;
             best_only = best_only && o.best_only;
@@ -650,10 +699,11 @@ struct TileFloor {
 };
 
 // The tile of a batch on a handle whose tile was neither set nor tuned.
+//  * One wave with room to spare: 512 points (or what the batch needs most, if
+//    more), the uncapped build.
 //  * Bound by its longest restart (the batch's steps spread over the resident
 //    decoders are fewer than the longest restart's): the uncapped build and a
-//    tile that no restart outgrows (a pass places at most one box per step and
-//    holds about as many live points). 61 batched instances x 48: decoder 0.525
+//    tile that hardly a restart outgrows. 61 batched instances x 48: decoder 0.525
 //    ms, 0.537 with the M = 16 build; 1024 restarts of one instance 0.279 with
 //    either.
 //  * Otherwise M = 16, up to 20 decoders per SM: 5000 restarts of one instance
@@ -661,15 +711,25 @@ struct TileFloor {
 //    one wave the deepest tile that keeps it there (2048 restarts: 0.36 ms; 0.51 at
 //    256, 512, which takes two), since a restart that outgrows it runs again
 //    afterwards; in several waves 256 boxes and up to 192 points, which about
-//    every restart fits (the device retry stage takes the others). 512 batched
-//    instances x 128 restarts with the retry stage: 6.34 ms at 160 and 192 points,
-//    7.45 at 128 and 7.33 at 96, where the stage runs a few restarts again; 6.83
-//    uncapped.
+//    every restart of the batched instances fits (the device retry stage takes the
+//    others). 512 batched instances x 128 restarts with the retry stage: 6.34 ms
+//    at 160 and 192 points, 7.45 at 128 and 7.33 at 96, where the stage runs a few
+//    restarts again; 6.83 uncapped. More points, up to 768, where more than an
+//    eighth of the batch is expected to hold more (small items among large ones,
+//    open containers): at 192 such restarts ran twice or three times. 32
+//    instances of 120 cartons of 30 to 80 cm and one of 4 cm x 256: 6.0 ms, 4.8 so;
+//    one decode of such an instance on a new handle 1.54 ms, 0.86 so.
 // The block engine has one build: 128 blocks, 192 points for several waves (512
-// instances x 64 restarts: 2.9 ms; about 9 % more at 256, 512).
+// instances x 64 restarts: 2.9 ms; about 9 % more at 256, 512), deeper by the same
+// rule.
 TileConfig auto_tile(const Batch& b, int sms, const TileFloor& f, int* wave) {
     const int steps = (std::max(1, b.max_steps) + 15) & ~15;
     const int points = std::max(128, (steps + 63) & ~31);
+    const int most = std::min(1024, (b.max_points + 31) & ~31);   // of any instance
+    // of seven eighths of the batch
+    int common = 768, boxes = 512;
+    for (int k = 3; k >= 0 && b.over_points[k] * 8 <= b.sum_steps; k--) common = Batch::POINTS[k];
+    for (int k = 1; k >= 0 && b.over_boxes[k] * 8 <= b.sum_steps; k--) boxes = Batch::BOXES[k];
     // decoders the SMs hold at this tile, 0 when it does not run
     auto resident = [&](const TileConfig& t) -> long long {
         int occ = 0;
@@ -680,13 +740,17 @@ TileConfig auto_tile(const Batch& b, int sms, const TileFloor& f, int* wave) {
         }
         return (long long)sms * occ;
     };
-    struct Depth { int P, C, M; };
-    const Depth ep[] = {{std::min(steps, 512), std::min(points, 512), 1},
-                        {std::min(steps, 512), std::min(points, 256), 16},
-                        {std::min(steps, 256), std::min(points, 192), 16}};
-    const Depth blk[] = {{std::min(steps, 256), 512, 1}, {std::min(steps, 128), 192, 1}};
+    struct Depth { int P, C, M; bool longest; };   // longest: also where the longest restart bounds the batch
+    const Depth ep[] = {{std::min(steps, 512), std::max(512, most), 1, false},
+                        {std::min(steps, 512), std::max(std::min(points, 512), most), 1, true},
+                        {std::min(steps, 512), std::max(std::min(points, 256), most), 16, false},
+                        {std::min(steps, 256), std::max(std::min(points, 192), most), 16, false},
+                        {std::min(steps, std::max(256, boxes)), common > 192 ? common : std::min(points, 192), 16, false}};
+    const Depth blk[] = {{std::min(steps, 256), 512, 1, true},
+                         {std::min(steps, b.over_boxes[0] ? 256 : 128), std::max(192, std::min(512, most)), 1, false},
+                         {std::min(steps, boxes), common, 1, false}};
     const Depth* d = b.engine == 1 ? blk : ep;
-    const int n = b.engine == 1 ? 2 : 3;
+    const int n = b.engine == 1 ? 3 : 5;
     TileConfig t;
     for (int k = 0; k < n; k++) {
         t.P = d[k].P;
@@ -696,7 +760,7 @@ TileConfig auto_tile(const Batch& b, int sms, const TileFloor& f, int* wave) {
         w.P = std::max(w.P, f.P[0]);
         w.C = std::max(w.C, f.C[0]);
         const long long r = resident(w);
-        if (b.n_slots <= r || (k == 0 && b.sum_steps <= r * b.long_steps)) {
+        if (b.n_slots <= r || (d[k].longest && b.sum_steps <= r * b.long_steps)) {
             *wave = 0;
             return w;
         }
@@ -1669,7 +1733,8 @@ void worker_main(plp_handle* h, int wi) {
 // SERVE_IDLE_STOP_S without requests and starts it again for the next one; a
 // decoder that finds no work for about a second exits by itself as well
 // (bounded polling). A request that the running launch's configuration cannot
-// take (a container taller than its top-z index covers) waits until the launch
+// take (a container taller than its top-z index covers, or more live points
+// expected than its tile holds) waits until the launch
 // has drained, and the next launch takes the merged configuration. Restarts
 // that overflow the serving tile (256 boxes, 256 live points, 12 decoders per
 // SM) go to the launch's overflow decoders; one that outgrows even their tile
@@ -1822,6 +1887,10 @@ size_t serve_align(size_t x, size_t unit) {    // a multiple of unit and of 128 
 // fit an SM (12 with M = 12 or uncapped, 146 registers): a burst of 256 requests,
 // 119872 restarts, 17.1 ms instead of 20.6. More (18 per SM, 96 registers, spills)
 // gains 3 % with heavy load and nothing without.
+// 256 points; 512 (12 per SM) once a request comes that is expected to hold more,
+// until the launch next stops idle: its restarts would all run a second time, on
+// the overflow decoders. 32 requests x 256 restarts of 120 cartons of 30 to 80 cm
+// and one of 4 cm: 423 ms, 5.3 so; of 250 cartons of 20 to 60 cm 1307 and 15.4.
 struct ServeConfig {
     int P = 256, C = 256, D = 1, M = 16, Hz = 0;
     int deep_P = 512, deep_C = 2048;   // the overflow decoders' tile (global memory)
@@ -1894,6 +1963,7 @@ struct ServeEngine {
     int n_deep = 0;                       // overflow decoders per launch
     std::atomic<bool> yield_req{false};   // a synchronous call on the handle wants the SMs
     ServeConfig cfg;
+    bool fixed_tile = false;              // PLP_SERVE_TILE
     const uint32_t* mt_init = nullptr;
     RegionRing arena_ring;             // request regions of the arena
     std::deque<ServeJob*> pending;     // submitted, not yet taken by the engine (h->mu)
@@ -1943,6 +2013,7 @@ struct ServeEngine {
                 cfg.P = p;
                 cfg.C = c;
                 cfg.M = m;
+                fixed_tile = true;
             }
         }
         n_deep = SERVE_DEEP;
@@ -2060,8 +2131,14 @@ struct ServeEngine {
         return true;
     }
 
+    static constexpr int POINTS = 256, POINTS_DEEP = 512;
+    int points_of(const Batch& b) const {
+        return fixed_tile ? cfg.C : b.max_points > POINTS ? POINTS_DEEP : POINTS;
+    }
+
     bool compatible(const Batch& b) const {
         if (!cfg.valid) return true;
+        if (points_of(b) > cfg.C) return false;
         if (cfg.Hz == 0) return true;
         return b.Hz != 0 && b.Hz <= cfg.Hz;
     }
@@ -2069,6 +2146,7 @@ struct ServeEngine {
     void merge_config(const Batch& b) {
         if (!cfg.valid) {
             cfg.Hz = b.Hz;
+            cfg.C = points_of(b);
             cfg.valid = true;
             return;
         }
@@ -2382,6 +2460,7 @@ struct ServeEngine {
         if (running && cudaEventQuery(ev_kern) == cudaSuccess) {
             running = false;
             progress = true;
+            if (!fixed_tile && active.empty() && fresh.empty()) cfg.C = POINTS;
             if (serve_trace())
                 std::fprintf(stderr, "[serve %.6f] launch ended head=%d overflow=%d/%d tail=%d\n", now_seconds(),
                              h_word[0], h_word[3], h_word[4], tail);
@@ -2939,6 +3018,7 @@ int plp_autotune(plp_handle* h, const plp_instance* const* insts, int32_t n_inst
     for (int p : {64, 128, 256})
         if (p <= P_MAX && (p >= std::min(max_steps, 64) || p == 128)) Ps.push_back(p);
     for (int c : {96, 160, 256, 512}) Cs.push_back(c);
+    if (full.max_points > 512) Cs.push_back(768);
     const int dm[][2] = {{1, 1}, {1, 16}, {2, 1}, {8, 1}};
     std::vector<TileConfig> cand;
     for (int p : Ps)
