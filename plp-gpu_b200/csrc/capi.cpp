@@ -1730,9 +1730,9 @@ void worker_main(plp_handle* h, int wi) {
 //   4. has its slot heads and placements copied out once the record shows its
 //      sequence number, and completes; its arena region is then free.
 // The launch keeps running while requests arrive. The host stops it after
-// SERVE_IDLE_STOP_S without requests and starts it again for the next one; a
-// decoder that finds no work for about a second exits by itself as well
-// (bounded polling). A request that the running launch's configuration cannot
+// SERVE_IDLE_STOP_S without requests and starts it again for the next one; the
+// decoders of a launch in which none finds work for about a second exit by
+// themselves as well (bounded polling). A request that the running launch's configuration cannot
 // take (a container taller than its top-z index covers, or more live points
 // expected than its tile holds) waits until the launch
 // has drained, and the next launch takes the merged configuration. Restarts
@@ -1746,7 +1746,7 @@ constexpr int SERVE_RECORDS = 1 << 16;         // requests in flight at most
 // ms with 96 launches for 151 requests (1.1 and 2.1 ms at the decoders' earlier
 // speed with a 50 ms stop and 2 launches).
 constexpr double SERVE_IDLE_STOP_S = 0.005;
-constexpr int SERVE_IDLE_POLLS = 250000;       // about 1 s of empty polls per decoder
+constexpr int SERVE_IDLE_POLLS = 250000;       // about 1 s of empty polls with no claim in the launch
 constexpr int SERVE_DEEP_IDLE_POLLS = 8000000; // about a minute for an overflow decoder
 constexpr int SERVE_DEEP = 32;                 // overflow decoders per launch (PLP_SERVE_DEEP overrides)
 constexpr size_t SERVE_UP_STAGE = (size_t)32 << 20;     // pinned staging of uploads

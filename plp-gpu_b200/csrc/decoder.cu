@@ -913,28 +913,6 @@ __device__ __forceinline__ void st_release_gpu(int* p, int v) {
     asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// Lane 0 of an overflow decoder: the next overflow item (ticket), or -1 once
-// the host asked the launch to stop and every main decoder has exited with
-// nothing left, or after deep_idle_polls empty polls.
-__device__ __forceinline__ int serve_claim_deep(const ServeArgs& s) {
-    unsigned ns = 64;
-    for (int k = 0; k < s.deep_idle_polls; k++) {
-        const int t = ld_acquire_gpu(s.dtail);
-        int h = *reinterpret_cast<volatile int*>(s.dhead);
-        while (h < t) {
-            const int prev = atomicCAS(s.dhead, h, h + 1);
-            if (prev == h) return h;
-            h = prev;
-        }
-        // main decoders push before they leave, so once none is left the
-        // reservation count seen after that is final
-        if (ld_acquire_gpu(s.stop) && ld_acquire_gpu(s.alive) == 0 && ld_acquire_gpu(s.dtail) <= h) return -1;
-        __nanosleep(ns);
-        if (ns < 8192) ns <<= 1;
-    }
-    return -1;
-}
-
 // Lane 0: waits (bounded) until the producer of ticket t has written it.
 __device__ __forceinline__ bool serve_deep_item(const ServeArgs& s, int t, int2* w) {
     int4* e = s.dring + (t & s.ring_mask);
@@ -960,7 +938,7 @@ __device__ __forceinline__ void serve_push_deep(const ServeArgs& s, int2 wk, int
     __syncwarp();
 }
 
-// The words of serve_claim in device memory. The host publishes by
+// The words of the claims (serve_claim.hpp) in device memory. The host publishes by
 // stream-ordered copies into it (items first, then the tail), so the polls stay
 // on this GPU's L2. 119872 restarts in 256 requests: 40.3 ms with one counter
 // and a compare-and-swap, 20.6 with two additions where the result copies keep up.
@@ -973,6 +951,10 @@ struct ServeWords {
     __device__ __forceinline__ void unclaim() const { atomicSub(s.claims, 1); }
     __device__ __forceinline__ int take() const { return atomicAdd(s.head, 1); }
     __device__ __forceinline__ bool stopped() const { return ld_acquire_gpu(s.stop) != 0; }
+    __device__ __forceinline__ int deep_tail() const { return ld_acquire_gpu(s.dtail); }
+    __device__ __forceinline__ int deep_head() const { return *reinterpret_cast<volatile int*>(s.dhead); }
+    __device__ __forceinline__ int deep_take(int h) const { return atomicCAS(s.dhead, h, h + 1); }
+    __device__ __forceinline__ int alive() const { return ld_acquire_gpu(s.alive); }
     __device__ __forceinline__ void pause(unsigned ns) const { __nanosleep(ns); }
 };
 
@@ -1077,8 +1059,8 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
         if constexpr (SERVE) {
             int sitem = -1, wx = 0, wy = 0;
             if (lane == 0) {
+                ServeWords words{sv};
                 if constexpr (MODE == 1) {
-                    ServeWords words{sv};
                     sitem = serve_claim(words, sv.idle_polls);
                     if (sitem >= 0) {
                         const int2 w = ld_relaxed_gpu_int2(sv.ring + (sitem & sv.ring_mask));
@@ -1086,7 +1068,7 @@ __device__ __forceinline__ void decoder1_body(const DecoderArgs& a, unsigned cha
                         wy = w.y;
                     }
                 } else {
-                    sitem = serve_claim_deep(sv);
+                    sitem = serve_claim_deep(words, sv.deep_idle_polls);
                     int2 w = make_int2(0, 0);
                     if (sitem >= 0 && !serve_deep_item(sv, sitem, &w)) {
                         atomicOr(a.err_flag, 1 << ERR_SYNC);   // a producer never finished its item

@@ -86,7 +86,7 @@ struct ServeArgs {
     int ring_mask;                  // ring entries - 1 (a power of two)
     volatile long long* done_seq;   // host-mapped: per completion record, the finished request's seq
     int2* done_best;                // host-mapped: per completion record, (best restart, fallback)
-    int idle_polls;                 // empty polls before a decoder exits (about 4 us each)
+    int idle_polls;                 // empty polls, with no claim in the launch, before a decoder exits (about 4 us each)
     // Restarts that outgrow the launch's tile are pushed by their decoder onto
     // the overflow ring and decoded again by the launch's first n_deep
     // decoders, whose deeper tile (deep_P, deep_C) lives in global memory.
@@ -96,7 +96,7 @@ struct ServeArgs {
     int* alive;                     // device: main decoders of the launch not yet exited
     int n_deep, deep_P, deep_C, deep_bytes;
     unsigned char* deep_scratch;    // device: n_deep x deep_bytes
-    int deep_idle_polls;            // empty polls before an overflow decoder exits
+    int deep_idle_polls;            // the same for an overflow decoder
 };
 bool serve_config_supported(int D, int M);
 cudaError_t serve_occupancy(int P, int C, int Hz, int D, int M, int* ctas_per_sm);

@@ -3,7 +3,8 @@
 // taking it back, but lets every decoder go on after a bounded wait.
 //   serve_claim_model progress   16 items while failed claims are pending
 //   serve_claim_model stop       the same, with the stop word set
-// Prints "<items taken> <items published> <accesses granted>".
+// Prints "<items taken> <items published> <accesses granted>". Modes with a dash
+// in their name run one decoder on a script (see scripted()).
 #include <condition_variable>
 #include <cstdio>
 #include <cstring>
@@ -54,12 +55,65 @@ struct Words {
     void unclaim() { m.access(i, true, [&] { m.claims--; }); }
     int take() { return m.access(i, false, [&] { return m.head++; }); }
     bool stopped() { return m.access(i, false, [&] { return m.stop || m.over; }); }
+    int deep_head() { return m.access(i, false, [] { return 0; }); }
     void pause(unsigned) {}
 };
+
+// One decoder whose surroundings follow a script over its empty polls.
+struct Script {
+    int polls = 0, n_tail = 0, n_head = 0, n_deep_tail = 0, n_deep_head = 0, n_alive = 1;
+    int others_until = 0, item_at = -1;   // the others take an item every 100 polls until here
+    bool deep = false;                    // this is an overflow decoder (the others are main ones)
+    int tail() { return n_tail; }
+    int claims() { return n_head; }
+    int head() { return n_head; }
+    int claim() { return n_head; }
+    void unclaim() {}
+    int take() { return n_head++; }
+    bool stopped() { return false; }
+    int deep_tail() { return n_deep_tail; }
+    int deep_head() { return n_deep_head; }
+    int deep_take(int) { return n_deep_head++; }
+    int alive() { return n_alive; }
+    void pause(unsigned) {
+        polls++;
+        if (polls <= others_until && polls % 100 == 0) {
+            if (deep) n_tail = ++n_head;
+            else n_deep_tail = ++n_deep_head;
+        }
+        if (polls == item_at) (deep ? n_deep_tail : n_tail)++;
+    }
+};
+
+// "<took an item> <empty polls>"
+int scripted(const char* mode) {
+    Script w;
+    int got = -1;
+    if (!std::strcmp(mode, "main-waits")) {          // overflow decoders at work, an item after a long while
+        w.others_until = w.item_at = 20000;
+        got = plpb::serve_claim(w, 2000);
+    } else if (!std::strcmp(mode, "main-idle")) {    // nobody takes anything any more
+        w.others_until = 5000;
+        got = plpb::serve_claim(w, 2000);
+    } else if (!std::strcmp(mode, "deep-waits")) {   // main decoders at work, the first overflow after a long while
+        w.deep = true;
+        w.others_until = w.item_at = 20000;
+        got = plpb::serve_claim_deep(w, 2000);
+    } else if (!std::strcmp(mode, "deep-left")) {    // the main decoders have left, no stop
+        w.deep = true;
+        w.n_alive = 0;
+        got = plpb::serve_claim_deep(w, 2000);
+    } else {
+        return 2;
+    }
+    std::printf("%d %d\n", got >= 0, w.polls);
+    return 0;
+}
 
 }  // namespace
 
 int main(int argc, char** argv) {
+    if (argc > 1 && std::strchr(argv[1], '-')) return scripted(argv[1]);
     const bool stop = argc > 1 && !std::strcmp(argv[1], "stop");
     Model m;
     // a decoder that ends (with an item, or without) takes part no further, as
