@@ -27,6 +27,7 @@
 
 #include "capi_internal.hpp"
 #include "engine.hpp"
+#include "tile_floor.hpp"
 
 using namespace plpb;
 
@@ -463,6 +464,9 @@ struct Batch {
     int2* h_redo_stage(size_t n) { redo_host.resize(n); return redo_host.data(); }
     size_t scratch_bytes = 0;
     int ctas = 0;
+    // prepared batches: the depths they turned out to need, for as long as they live
+    bool prepared = false;
+    Floor floor[2];
     bool counters_zero = false;            // uploaded as zeros and not used yet
     unsigned long long* direct = nullptr;  // the decoders write placements here (pinned host memory)
     TileConfig tile;
@@ -692,12 +696,6 @@ cudaError_t tile_occupancy(const Batch& b, const TileConfig& t, int* occ) {
     return decoder_occupancy(t.P, t.C, b.Hz, t.G, t.D, t.M, occ);
 }
 
-// Deepest tile that a batch of this handle needed so far, when the tile is
-// chosen per batch: [0] batches of one wave, [1] of several.
-struct TileFloor {
-    int P[2] = {0, 0}, C[2] = {0, 0};
-};
-
 // The tile of a batch on a handle whose tile was neither set nor tuned.
 //  * One wave with room to spare: 512 points (or what the batch needs most, if
 //    more), the uncapped build.
@@ -722,7 +720,8 @@ struct TileFloor {
 // The block engine has one build: 128 blocks, 192 points for several waves (512
 // instances x 64 restarts: 2.9 ms; about 9 % more at 256, 512), deeper by the same
 // rule.
-TileConfig auto_tile(const Batch& b, int sms, const TileFloor& f, int* wave) {
+// f: floors for one wave and for several.
+TileConfig auto_tile(const Batch& b, int sms, const Floor* f, int* wave) {
     const int steps = (std::max(1, b.max_steps) + 15) & ~15;
     const int points = std::max(128, (steps + 63) & ~31);
     const int most = std::min(1024, (b.max_points + 31) & ~31);   // of any instance
@@ -751,24 +750,23 @@ TileConfig auto_tile(const Batch& b, int sms, const TileFloor& f, int* wave) {
                          {std::min(steps, boxes), common, 1, false}};
     const Depth* d = b.engine == 1 ? blk : ep;
     const int n = b.engine == 1 ? 3 : 5;
-    TileConfig t;
+    auto tile = [&](const Depth& e, const Floor& g) {
+        const Floor x = floored({e.P, e.C}, g, std::max(1, b.max_steps));
+        TileConfig t;
+        t.P = x.P;
+        t.C = x.C;
+        t.M = e.M;
+        return t;
+    };
+    *wave = 0;
     for (int k = 0; k < n; k++) {
-        t.P = d[k].P;
-        t.C = d[k].C;
-        t.M = d[k].M;
-        TileConfig w = t;
-        w.P = std::max(w.P, f.P[0]);
-        w.C = std::max(w.C, f.C[0]);
-        const long long r = resident(w);
-        if (b.n_slots <= r || (d[k].longest && b.sum_steps <= r * b.long_steps)) {
-            *wave = 0;
-            return w;
-        }
+        const TileConfig t = tile(d[k], f[0]);
+        const long long r = resident(t);
+        if (b.n_slots <= r || (d[k].longest && b.sum_steps <= r * b.long_steps)) return t;
     }
-    t.P = std::max(t.P, f.P[1]);
-    t.C = std::max(t.C, f.C[1]);
     *wave = 1;
-    return t;
+    const TileConfig t = tile(d[n - 1], f[1]);
+    return resident(t) > 0 ? t : tile(d[n - 1], Floor{});   // a floor that does not fit is left out
 }
 
 // Fewer decoders per CTA when the tile plus this batch's top-z index (and,
@@ -1539,7 +1537,7 @@ struct plp_handle {
     size_t in_use = 0;
     TileConfig tile;
     bool tile_auto = true;            // no tile set or tuned: one per batch
-    TileFloor tile_floor;
+    TileFloors tile_floors;
     std::string err;
     std::mutex mu;
     std::condition_variable cv;       // request state changes
@@ -1584,12 +1582,12 @@ struct TilePick {
 
 TilePick pick_tile(plp_handle* h, const Batch& b) {
     TilePick p;
-    TileFloor f;
+    Floor f[2];
     bool autot;
     {
         std::lock_guard<std::mutex> lk(h->mu);
         p.tile = h->tile;
-        f = h->tile_floor;
+        for (int w = 0; w < 2; w++) f[w] = b.prepared ? b.floor[w] : h->tile_floors.get(b.engine, w);
         autot = h->tile_auto;
     }
     if (autot) {
@@ -1602,14 +1600,15 @@ TilePick pick_tile(plp_handle* h, const Batch& b) {
     return p;
 }
 
-void keep_tile(plp_handle* h, const TilePick& p) {
+void keep_tile(plp_handle* h, const TilePick& p, Batch& b) {
     std::lock_guard<std::mutex> lk(h->mu);
     if (p.wave < 0) {
         remember_tile(h->tile, p.tile);
         return;
     }
-    if (p.tile.P > p.first.P) h->tile_floor.P[p.wave] = std::max(h->tile_floor.P[p.wave], p.tile.P);
-    if (p.tile.C > p.first.C) h->tile_floor.C[p.wave] = std::max(h->tile_floor.C[p.wave], p.tile.C);
+    h->tile_floors.raise(b.engine, p.wave, {p.first.P, p.first.C}, {p.tile.P, p.tile.C});
+    if (p.tile.P > p.first.P) b.floor[p.wave].P = std::max(b.floor[p.wave].P, p.tile.P);
+    if (p.tile.C > p.first.C) b.floor[p.wave].C = std::max(b.floor[p.wave].C, p.tile.C);
 }
 
 size_t request_bytes(const Instance& I, const plp_run_opts& o) {
@@ -1681,7 +1680,7 @@ void worker_main(plp_handle* h, int wi) {
         if (s == PLP_OK) {
             TilePick tile = pick_tile(h, b);
             s = run_batch(b, st, pin, h->sms, tile.tile);
-            if (s == PLP_OK) keep_tile(h, tile);
+            if (s == PLP_OK) keep_tile(h, tile, b);
         }
         std::vector<plp_result*> res;
         if (s == PLP_OK) res = collect(b, now_seconds() - t0);
@@ -3112,7 +3111,7 @@ int plp_solve(plp_handle* h, const plp_instance* const* insts, int32_t n_inst,
     if (s == PLP_OK) {
         TilePick tile = pick_tile(h, b);
         s = run_batch(b, h->sync_stream, h->sync_pin, h->sms, tile.tile, &h->pool);
-        if (s == PLP_OK) keep_tile(h, tile);
+        if (s == PLP_OK) keep_tile(h, tile, b);
     }
     if (s != PLP_OK) {
         record(h, s);
@@ -3294,6 +3293,11 @@ int plp_batch_prepare(plp_handle* h, const plp_instance* const* insts, int32_t n
         op.push_back(opts[n_opts == 1 ? 0 : i]);
     }
     int s = pb->b.build(in, op);
+    {
+        std::lock_guard<std::mutex> lk(h->mu);
+        for (int w = 0; w < 2; w++) pb->b.floor[w] = h->tile_floors.get(pb->b.engine, w);
+        pb->b.prepared = true;
+    }
     if (s == PLP_OK) s = batch_prepare(pb->b, h->sync_stream, h->sync_pin, h->sms, pick_tile(h, pb->b).tile, false);
     if (s != PLP_OK) {
         record(h, s);
@@ -3316,7 +3320,7 @@ int plp_batch_run(plp_batch* pb, double* device_ms, double* decoder_ms, int32_t*
         record(h, s);
         return s;
     }
-    keep_tile(h, tile);
+    keep_tile(h, tile, pb->b);
     pb->executed = true;
     if (device_ms) *device_ms = x.device_ms;
     if (decoder_ms) *decoder_ms = x.decoder_ms;
