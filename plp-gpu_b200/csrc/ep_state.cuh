@@ -109,7 +109,7 @@ __device__ __forceinline__ int place1(uint32_t pkey, int pw, int pd, int ph, uin
         const bool in = i < nc;
         const uint32_t key = in ? K[i] : 0u, exy = in ? K[cap + i] : 0u, ezm = in ? K[2 * cap + i] : 0u;
         const int x = (int)(key & xmask), y = (int)((key >> xb) & ymask), z = (int)(key >> xyb);
-        bool gone = false;
+        bool gone = in && exy == 0u;   // dead since a placement that freed more slots than it noted
         if (in && x < px2 && y < py2 && z < pz2) {   // else the box lies before the point
             int ex = (int)(exy & 0xffffu), ey = (int)(exy >> 16), ez = (int)(ezm & 0xffffu);
             const int dx = px - x, dy = py - y, dz = pz - z;
@@ -135,8 +135,8 @@ __device__ __forceinline__ int place1(uint32_t pkey, int pw, int pd, int ph, uin
     live &= ~__reduce_or_sync(FULL, dup);
     __syncwarp();   // box tables, top-z index, points and freed slots are final
     // New points take freed slots, or come after the end; the last point fills
-    // a slot left over. Slots past the 32nd freed in one
-    // placement keep their dead point, which the next placement frees again.
+    // a slot left over. Slots past the 32nd freed in one placement keep their
+    // dead point (no extents), whose slot the next placement frees.
     nf = min(nf, 32);
     const int nl = __popc(live), nc0 = nc;
 #pragma unroll 1
