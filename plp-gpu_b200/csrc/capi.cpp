@@ -3312,11 +3312,17 @@ int plp_batch_run(plp_batch* pb, double* device_ms, double* decoder_ms, int32_t*
     plp_handle* h = pb->h;
     serve_yield(h);
     std::lock_guard<std::mutex> g(h->sync_mu);
+    if (!pb->b.d_mem) {   // a run that failed gave the batch's tables back
+        int s = set_error(PLP_E_INVALID, "plp_batch_run: an earlier run of this batch failed");
+        record(h, s);
+        return s;
+    }
     cudaSetDevice(h->device);
     TilePick tile = pick_tile(h, pb->b);
     ExecStats x;
     int s = batch_execute(pb->b, h->sync_stream, h->sms, tile.tile, &x, true);
     if (s != PLP_OK) {
+        pb->executed = false;
         record(h, s);
         return s;
     }
@@ -3337,6 +3343,7 @@ int plp_batch_fetch(plp_batch* pb, plp_result** results) {
     const double t0 = now_seconds();
     int s = batch_fetch(pb->b, h->sync_stream, nullptr, &h->pool);
     if (s != PLP_OK) {
+        pb->executed = false;   // its tables went back, as after a failed run
         record(h, s);
         return s;
     }
