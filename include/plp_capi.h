@@ -234,6 +234,8 @@ int plp_batch_io_bytes(const plp_batch* b, int64_t* h2d, int64_t* d2h);
 /* 1 when the batch's next run replays its captured CUDA graph, else 0 (no
  * reference counterpart). */
 int plp_batch_graph(const plp_batch* b);
+/* plp_destroy takes the device memory of the handle's batches back; a batch that
+ * outlives its handle can only be freed. */
 void plp_batch_free(plp_batch* b);
 
 /* Serving: admit a request; it starts as soon as the memory budget allows and

@@ -1530,6 +1530,12 @@ namespace {
 struct ServeEngine;
 }
 
+struct plp_batch {
+    plp_handle* h = nullptr;          // null once the handle is destroyed
+    Batch b;
+    bool executed = false;
+};
+
 struct plp_handle {
     int device = 0;
     int sms = 148;
@@ -1554,6 +1560,7 @@ struct plp_handle {
     // synchronous solves
     cudaStream_t sync_stream = nullptr;
     std::mutex sync_mu;
+    std::vector<plp_batch*> batches;   // prepared and not freed (sync_mu)
     Pinned sync_pin;
     std::shared_ptr<HostPool> pool = std::make_shared<HostPool>();   // result blocks of synchronous solves
     // serving engine (one persistent launch that requests join), made on the
@@ -2919,6 +2926,14 @@ void plp_destroy(plp_handle* h) {
     h->cv_sched.notify_all();
     for (auto& t : h->workers) t.join();
     for (auto& kv : h->reqs) delete kv.second->result;
+    // batches not freed yet give their device memory back on the handle's
+    // stream while there is one; their objects stay the caller's
+    for (plp_batch* pb : h->batches) {
+        cudaSetDevice(h->device);
+        batch_release(pb->b, h->sync_stream);
+        pb->executed = false;
+        pb->h = nullptr;
+    }
     for (auto s : h->streams) cudaStreamDestroy(s);
     if (h->sync_stream) cudaStreamDestroy(h->sync_stream);
     delete h;
@@ -3262,12 +3277,6 @@ int plp_request_times(plp_handle* h, int64_t id, double* queued_s, double* total
 // ---- prepared batches ------------------------------------------------------
 }  // extern "C"
 
-struct plp_batch {
-    plp_handle* h = nullptr;
-    Batch b;
-    bool executed = false;
-};
-
 extern "C" {
 
 int plp_batch_prepare(plp_handle* h, const plp_instance* const* insts, int32_t n_inst,
@@ -3303,12 +3312,14 @@ int plp_batch_prepare(plp_handle* h, const plp_instance* const* insts, int32_t n
         record(h, s);
         return s;
     }
+    h->batches.push_back(pb.get());
     *out = pb.release();
     return PLP_OK;
 }
 
 int plp_batch_run(plp_batch* pb, double* device_ms, double* decoder_ms, int32_t* launches) {
     if (!pb) return set_error(PLP_E_INVALID, "plp_batch_run: null batch");
+    if (!pb->h) return set_error(PLP_E_INVALID, "plp_batch_run: the batch's handle was destroyed");
     plp_handle* h = pb->h;
     serve_yield(h);
     std::lock_guard<std::mutex> g(h->sync_mu);
@@ -3363,9 +3374,11 @@ int plp_batch_graph(const plp_batch* pb) { return pb && pb->b.gexec ? 1 : 0; }
 
 void plp_batch_free(plp_batch* pb) {
     if (!pb) return;
-    {
-        std::lock_guard<std::mutex> g(pb->h->sync_mu);
-        batch_release(pb->b, pb->h->sync_stream);
+    if (plp_handle* h = pb->h) {
+        std::lock_guard<std::mutex> g(h->sync_mu);
+        cudaSetDevice(h->device);
+        batch_release(pb->b, h->sync_stream);
+        h->batches.erase(std::find(h->batches.begin(), h->batches.end(), pb));
     }
     delete pb;
 }

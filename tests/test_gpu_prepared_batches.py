@@ -32,3 +32,26 @@ def test_a_batch_whose_run_failed_refuses_to_run_again():
         for k in range(8):
             assert O.strip_time(r.json(k)) == O.strip_time(O.run(O.OInstance(text), seed=k)[0])
         b.close()
+
+
+def test_a_batch_may_outlive_its_handle():
+    text = synth.multi_restart(2).to_thpack()
+    inst, opts = P.Instance.parse(text), P.make_opts(seed=0, restarts=8)
+    left = []
+    for _ in range(3):
+        with P.Handle() as h:
+            b = h.prepare([inst], opts)
+            b.run()
+            r = b.fetch()[0]
+            left.append(b)
+    for b in left:
+        for call in (b.run, b.fetch):
+            with pytest.raises(P.PlpError) as e:
+                call()
+            assert e.value.status == P.E_INVALID
+        assert not b.graph
+    left.clear()                                          # freed after their handles
+    with P.Handle() as h:
+        again = h.solve([inst], opts)[0]
+    for k in range(8):
+        assert O.strip_time(r.json(k)) == O.strip_time(again.json(k)) == O.strip_time(O.run(O.OInstance(text), seed=k)[0])
