@@ -435,7 +435,7 @@ struct Batch {
     long long n_slots = 0, n_places = 0;
     int max_stride = 1, max_steps = 0, Hz = 0;
     long long sum_steps = 0, long_steps = 1;   // of all restarts and of the longest, over their passes
-    int max_points = 1;                        // live points expected of the instance that needs most
+    int max_points = 1, max_boxes = 1;         // live points and boxes expected of the instance that needs most
     // the batch's steps in instances that are expected to hold more live points
     // than POINTS[k], and in those to place more than BOXES[k] boxes
     static constexpr int POINTS[] = {192, 256, 384, 512}, BOXES[] = {128, 256};
@@ -500,7 +500,7 @@ struct Batch {
         max_types = 0;
         n_slots = 0; n_places = 0; max_stride = 1; max_steps = 0; multi_pass = false;
         sum_steps = 0; long_steps = 1;
-        max_points = 1;
+        max_points = max_boxes = 1;
         std::fill(std::begin(over_points), std::end(over_points), 0);
         std::fill(std::begin(over_boxes), std::end(over_boxes), 0);
         int maxH = 0;
@@ -609,6 +609,7 @@ struct Batch {
                 sum_steps += s * o.restarts;
                 long_steps = std::max(long_steps, s);
                 max_points = std::max(max_points, need.points);
+                max_boxes = std::max(max_boxes, need.boxes);
                 for (int k = 0; k < 4; k++) over_points[k] += need.points > POINTS[k] ? s * o.restarts : 0;
                 for (int k = 0; k < 2; k++) over_boxes[k] += need.boxes > BOXES[k] ? s * o.restarts : 0;
             }
@@ -1739,10 +1740,10 @@ void worker_main(plp_handle* h, int wi) {
 // SERVE_IDLE_STOP_S without requests and starts it again for the next one; the
 // decoders of a launch in which none finds work for about a second exit by
 // themselves as well (bounded polling). A request that the running launch's configuration cannot
-// take (a container taller than its top-z index covers, or more live points
-// expected than its tile holds) waits until the launch
+// take (a container taller than its top-z index covers, or more boxes or
+// live points expected than its tile holds) waits until the launch
 // has drained, and the next launch takes the merged configuration. Restarts
-// that overflow the serving tile (256 boxes, 256 live points, 12 decoders per
+// that overflow the serving tile (256 boxes, 256 live points, 16 decoders per
 // SM) go to the launch's overflow decoders; one that outgrows even their tile
 // makes its request run again on the wave path's code.
 constexpr int SERVE_RING = 1 << 20;            // work items in flight at most
@@ -1893,10 +1894,14 @@ size_t serve_align(size_t x, size_t unit) {    // a multiple of unit and of 128 
 // fit an SM (12 with M = 12 or uncapped, 146 registers): a burst of 256 requests,
 // 119872 restarts, 17.1 ms instead of 20.6. More (18 per SM, 96 registers, spills)
 // gains 3 % with heavy load and nothing without.
-// 256 points; 512 (12 per SM) once a request comes that is expected to hold more,
-// until the launch next stops idle: its restarts would all run a second time, on
-// the overflow decoders. 32 requests x 256 restarts of 120 cartons of 30 to 80 cm
-// and one of 4 cm: 423 ms, 5.3 so; of 250 cartons of 20 to 60 cm 1307 and 15.4.
+// 256 boxes and points, 512 of either (10 to 13 per SM) once more restarts come that
+// are expected to need them than 128 and one in 512 of all, until the launch next stops
+// idle: their restarts would all run a second time, on the overflow decoders, some
+// 10 restarts a ms. 32 requests x 256 restarts of 120 cartons of 30 to 80 cm and
+// one of 4 cm: 423 ms, 5.3 so; of 250 cartons of 20 to 60 cm 1307 and 15.4. Bursts
+// of 256 ordinary requests with one of 300 to 470 boxes and 1024 restarts among
+// them: 142, 119 and 215 ms, 19, 22 and 22 so; with one of 64 restarts, which the
+// overflow decoders take beside the others, 16.2 to 17.3 (3 more after a drain).
 struct ServeConfig {
     int P = 256, C = 256, D = 1, M = 16, Hz = 0;
     int deep_P = 512, deep_C = 2048;   // the overflow decoders' tile (global memory)
@@ -1961,7 +1966,7 @@ struct ServeEngine {
                                    // launch, [2] main decoders, [5] 1 and [6] 0 (stop), [8 ..] tail values
     PinnedRing up_stage, down_stage;
     std::shared_ptr<ResultSlab> slab = std::make_shared<ResultSlab>();
-    std::vector<std::shared_ptr<char>> kept;   // blocks of requests that failed, until the launch has ended
+    std::vector<std::shared_ptr<char>> kept;   // blocks of requests that failed, until the engine goes
     ServeArgs args{};
     cudaStream_t up = nullptr, kern = nullptr, down = nullptr;
     cudaEvent_t ev_kern = nullptr, ev_go = nullptr;
@@ -1970,6 +1975,8 @@ struct ServeEngine {
     std::atomic<bool> yield_req{false};   // a synchronous call on the handle wants the SMs
     ServeConfig cfg;
     bool fixed_tile = false;              // PLP_SERVE_TILE
+    long long deep_restarts = 0;          // of requests taken though the tile is expected not to fit them ...
+    long long deep_since = 0;             // ... after this many published restarts
     const uint32_t* mt_init = nullptr;
     RegionRing arena_ring;             // request regions of the arena
     std::deque<ServeJob*> pending;     // submitted, not yet taken by the engine (h->mu)
@@ -2137,14 +2144,20 @@ struct ServeEngine {
         return true;
     }
 
-    static constexpr int POINTS = 256, POINTS_DEEP = 512;
-    int points_of(const Batch& b) const {
-        return fixed_tile ? cfg.C : b.max_points > POINTS ? POINTS_DEEP : POINTS;
+    // (the boxes expected are more than those placed, by a fifth at the median)
+    static constexpr int DEPTH = 256, DEPTH_MORE = 512, BOXES_LIKELY = 288, DEEP_RESTARTS = 128,
+                         DEEP_SHARE = 512;
+    int boxes_of(const Batch& b) const {
+        return fixed_tile ? cfg.P : b.max_boxes > BOXES_LIKELY ? DEPTH_MORE : DEPTH;
     }
+    int points_of(const Batch& b) const { return fixed_tile ? cfg.C : b.max_points > DEPTH ? DEPTH_MORE : DEPTH; }
+    bool fits(const Batch& b) const { return boxes_of(b) <= cfg.P && points_of(b) <= cfg.C; }
 
     bool compatible(const Batch& b) const {
         if (!cfg.valid) return true;
-        if (points_of(b) > cfg.C) return false;
+        if (!fits(b) && ((!running && active.empty()) ||
+                         deep_restarts + b.n_slots > DEEP_RESTARTS + (published - deep_since) / DEEP_SHARE))
+            return false;
         if (cfg.Hz == 0) return true;
         return b.Hz != 0 && b.Hz <= cfg.Hz;
     }
@@ -2152,10 +2165,14 @@ struct ServeEngine {
     void merge_config(const Batch& b) {
         if (!cfg.valid) {
             cfg.Hz = b.Hz;
-            cfg.C = points_of(b);
+            cfg.P = std::max(cfg.P, boxes_of(b));
+            cfg.C = std::max(cfg.C, points_of(b));
+            deep_restarts = 0;
+            deep_since = published;
             cfg.valid = true;
             return;
         }
+        if (!fits(b)) deep_restarts += b.n_slots;
         cfg.Hz = (cfg.Hz == 0 || b.Hz == 0) ? 0 : std::max(cfg.Hz, b.Hz);
     }
 
@@ -2466,7 +2483,11 @@ struct ServeEngine {
         if (running && cudaEventQuery(ev_kern) == cudaSuccess) {
             running = false;
             progress = true;
-            if (!fixed_tile && active.empty() && fresh.empty()) cfg.C = POINTS;
+            if (active.empty() && fresh.empty()) {
+                deep_restarts = 0;
+                deep_since = published;
+                if (!fixed_tile) cfg.P = cfg.C = DEPTH;
+            }
             if (serve_trace())
                 std::fprintf(stderr, "[serve %.6f] launch ended head=%d overflow=%d/%d tail=%d\n", now_seconds(),
                              h_word[0], h_word[3], h_word[4], tail);

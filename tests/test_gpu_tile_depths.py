@@ -84,24 +84,26 @@ import sys
 sys.path[:0] = {paths!r}
 import test_gpu_tile_depths as T
 import plpb200 as P
-texts = T._texts("cube_2cm")[:2] + T._texts("cartons_and_4cm")[:2] + T._texts("open_250")[:2]
-texts += [T.synth.batched(30010 + i).to_thpack() for i in range(4)]
-texts = texts[6:8] + texts[:6] + texts[8:]
+plain = [T.synth.batched(30010 + i).to_thpack() for i in range(6)]
+deep = T._texts("cube_2cm")[:2] + T._texts("cartons_and_4cm")[:2] + T._texts("open_250")[:2]
+deep += ["1\\n1 9\\n587 233 220\\n1\\n1 20 1 20 1 20 1 300\\n"]
+texts = {order}
 with P.Handle() as h:
-    ids = [h.submit(P.Instance.parse(t), P.make_opts(seed=0, restarts=48)) for t in texts]
+    ids = [h.submit(P.Instance.parse(t), P.make_opts(seed=0, restarts=192)) for t in texts]
     for rid in ids:
         assert h.wait(rid, 60000) == P.OK, P.last_error()
-    T._check(texts, [h.take(rid) for rid in ids], 48)
+    T._check(texts, [h.take(rid) for rid in ids], 192)
     c = h.serve_counters()
 assert c["served"] == len(texts) and c["fallbacks"] == 0, c
 """
 
 
-def test_served_requests_stay_with_the_main_decoders():
+@pytest.mark.parametrize("order", ["deep + plain", "plain + deep + plain"])
+def test_served_requests_stay_with_the_main_decoders(order):
+    """Also after a launch that started with others (it is drained for them)."""
     env = dict(os.environ, PLP_SERVE_TRACE="1")
-    code = SERVED.format(paths=[os.path.join(os.path.dirname(HERE), "plp-gpu_b200"), HERE])
+    code = SERVED.format(paths=[os.path.join(os.path.dirname(HERE), "plp-gpu_b200"), HERE], order=order)
     p = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300, env=env)
     assert p.returncode == 0, p.stderr[-2000:]
     ended = re.findall(r"launch ended head=\d+ overflow=(\d+)/(\d+)", p.stderr)
-    ended += re.findall(r"(?:teardown) overflow=(\d+)/(\d+)", p.stderr)
     assert ended and all(b == "0" for _, b in ended), ended
