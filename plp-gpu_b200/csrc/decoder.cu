@@ -34,16 +34,19 @@
 //    and stays infeasible (boxes are never removed). The reference keeps such
 //    points in its candidate list; they never produce a feasible pair, so the
 //    ordered list of feasible pairs -- the only thing the pick reads -- is the
-//    same when they are dropped. The live list is exactly the reference's
-//    candidate set minus covered points, in the same (z, y, x) order.
+//    same when they are dropped. decoder_kernel's live list is exactly the
+//    reference's candidate set minus covered points, in the same (z, y, x)
+//    order; decoder1_kernel also drops points where no type fits any more, and
+//    keeps the rest in no order (its section says how the pick still is the
+//    reference's).
 //  * C1/C2/C3 are evaluated per point for all orientations at once. C2 is the
 //    same integer test; C3 sums the same integer overlap areas (the ratio
 //    test is the reference's FP64 form in decoder_kernel and its exact
 //    integer equivalent in decoder1_kernel); C1 only visits boxes whose top
 //    lies above z (a box with top <= z cannot overlap a box starting at z),
 //    which does not change the boolean.
-//  * The first feasible pair (greedy branch) is found by scanning points in
-//    order; random() is drawn only after one feasible pair exists, and the
+//  * The first feasible pair (greedy branch) is the one of the first feasible
+//    point in order; random() is drawn only after one feasible pair exists, and the
 //    full count / idx-th selection runs only on the random branch.
 #include "device_common.cuh"
 #include "engine.hpp"
@@ -116,8 +119,9 @@ __host__ __device__ inline DecLayout dec_layout(int P, int C, int Hz) {
 
 // Layout of one single-warp decoder: MT state, top-sorted boxes, the points
 // {key, x extent | y extent << 16, z extent | mark} (SoA, in no order) and
-// the step's items. Eight slots past C take
-// a placement's corners before the capacity check.
+// the step's items. The points' arrays are eight entries longer than C (a
+// multiple of 32), so that a point's three words lie in different banks and it
+// moves in one access.
 struct Dec1Layout {
     int off_box, off_pts, off_w, off_free, off_zt, bytes;
     int cap;   // entries per array of the points
@@ -1393,7 +1397,7 @@ static DecoderArgs decoder_args(const DecodeLaunch& L) {
 
 #ifndef PLP_SERVE_TU
 // The M = 16 configuration is built for 17 resident decoders: the compiler
-// settles at 88 registers (106 for a bound of 15 or 16), which leaves 21 of them
+// settles at 90 registers (106 for a bound of 15 or 16), which leaves 20 of them
 // room in the register file. 512 batched instances x 128 restarts at 256 boxes
 // and 160 points: 6.98 ms built for 15 or 16, 6.40 for 17, 6.44 for 18, 6.62 for
 // 19, 7.0 for 20 (fewer registers, more code). Straight-line code is kept short

@@ -18,7 +18,6 @@
 #include "capi_internal.hpp"
 #include "device_common.cuh"
 #include "engine.hpp"
-#include "feas_eval.cuh"
 
 namespace plpb {
 

@@ -1,6 +1,5 @@
 // feas_eval.cuh -- lookups in a table of placed boxes held sorted by top z, by
-// the top-z index where there is one. Shared by the multi-warp decoder
-// (decoder.cu) and the block engine (block.cu).
+// the top-z index where there is one, for the multi-warp decoder (decoder.cu).
 #pragma once
 
 #include "device_common.cuh"

@@ -7,7 +7,6 @@
 #include <climits>
 
 #include "device_common.cuh"
-#include "feas_eval.cuh"
 
 namespace plpb {
 
