@@ -1749,9 +1749,9 @@ void worker_main(plp_handle* h, int wi) {
 constexpr int SERVE_RING = 1 << 20;            // work items in flight at most
 constexpr int SERVE_RECORDS = 1 << 16;         // requests in flight at most
 // An idle launch keeps the SMs from everything else on the GPU, and starting it
-// again costs a sparse stream little: at 100 requests/s p50 0.61 ms and p99 1.6
-// ms with 96 launches for 151 requests (1.1 and 2.1 ms at the decoders' earlier
-// speed with a 50 ms stop and 2 launches).
+// again costs a sparse stream little: at 100 requests/s p50 0.44 ms and p99
+// 1.1 to 1.5 ms with 82 launches for 151 requests (1.1 and 2.1 ms at the decoders'
+// earlier speed with a 50 ms stop and 2 launches).
 constexpr double SERVE_IDLE_STOP_S = 0.005;
 constexpr int SERVE_IDLE_POLLS = 250000;       // about 1 s of empty polls with no claim in the launch
 constexpr int SERVE_DEEP_IDLE_POLLS = 8000000; // about a minute for an overflow decoder
