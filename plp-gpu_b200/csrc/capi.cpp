@@ -1366,7 +1366,7 @@ int batch_execute(Batch& b, cudaStream_t st, int sms, TileConfig& tile, ExecStat
     // land in place)
     TileConfig tr = staged ? deep : t;
     bool retried = false;
-    for (int attempt = 0, bits = pending_bits(b, staged); bits != 0; attempt++, bits = fl[0]) {
+    for (int bits = pending_bits(b, staged); bits != 0; bits = fl[0]) {
         retried = true;
         if (bits & (1 << ERR_RNG)) {
             batch_release(b, st);
@@ -1388,12 +1388,15 @@ int batch_execute(Batch& b, cudaStream_t st, int sms, TileConfig& tile, ExecStat
             if (h.err == ERR_BOX_CAP) { grow_p = true; redo.push_back(w); }
             else if (h.err == ERR_CAND_CAP) { grow_c = true; redo.push_back(w); }
         }
-        if (redo.empty() || attempt == 6) {
+        // (a retry may meet the boxes' depth or the points', so each grows on its
+        // own, up to its limit: at most 15 retries from the shallowest tile)
+        const TileConfig tried = tr;
+        if (grow_p) tr.P = std::min(P_MAX, std::max(tr.P * 2, 32));
+        if (grow_c) tr.C = std::min(C_MAX, tr.C * 2);
+        if (redo.empty() || (tr.P == tried.P && tr.C == tried.C)) {
             batch_release(b, st);
             return set_error(PLP_E_CAPACITY, "decoder tile capacity exceeded after retries");
         }
-        if (grow_p) tr.P = std::min(P_MAX, std::max(tr.P * 2, 32));
-        if (grow_c) tr.C = std::min(C_MAX, tr.C * 2);
         // deeper tiles: fewer decoders per CTA keeps one CTA within 227 KB
         while (tr.D > 1 && tile_smem(b, tr) * tr.D > 200 * 1024) tr.D >>= 1;
         fit_tile(tr, b);
