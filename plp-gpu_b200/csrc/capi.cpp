@@ -416,10 +416,13 @@ Sizes instance_sizes(const Instance& I, const std::vector<TypeOrs>& ors) {
     const double edge = (z.mw + z.md + z.mh) / (3 * std::cbrt(mean));
     const double boxes = std::min(n, 0.8 * room / mean);
     const double full = 0.8 * std::cbrt(80 / boxes) + 3.5 * std::exp(-edge / 0.11);
-    const double open = std::max(full, 3.7 - 1.9 * edge);
-    const double share = std::pow(std::min(1.0, std::max(0.0, (1 - vol / room) / 0.8)), 1 + 2 * edge);
+    double rate = full;
+    if (vol < room) {
+        const double open = std::max(full, 3.7 - 1.9 * edge);
+        rate += std::pow(std::min(1.0, (1 - vol / room) / 0.8), 1 + 2 * edge) * (open - full);
+    }
     z.boxes = (int)std::min(1e6, boxes) + 1;
-    z.points = (int)std::min(1e6, 1.1 * boxes * (full + share * (open - full))) + 8;
+    z.points = (int)std::min(1e6, 1.1 * boxes * rate) + 8;
     return z;
 }
 
